@@ -12,6 +12,7 @@
 #include <algorithm>
 
 #include "gsr_internal.h"
+#include "ndc.h"
 
 namespace gsr {
 namespace {
@@ -89,8 +90,6 @@ constexpr float kOThin = 0.5f;
 #define GSR_SH_C3_4 (-0.4570457994644658f)
 #define GSR_SH_C3_5 1.445305721320277f
 #define GSR_SH_C3_6 (-0.5900435899266435f)
-
-__device__ __forceinline__ float ndc_to_pix(float v, int S) { return ((v + 1.0) * S - 1.0) * 0.5; }
 
 __device__ __forceinline__ float3 xform43(V3 p, const float* m)
 {
@@ -418,7 +417,7 @@ __global__ __launch_bounds__(kThreads, VIEWS ? 6 : 5) void k_preprocess(const __
             if (2.0f * det * power < kBMinSq * trace && opacity < kOThin) break;
             width = (int)(1.414214f * sqrt_approx(cov.x * power) + 1.0f);
             height = (int)(1.414214f * sqrt_approx(cov.z * power) + 1.0f);
-            point_xy = {ndc_to_pix(p_proj.x, a.W), ndc_to_pix(p_proj.y, a.H)};
+            point_xy = {gsr_ndc::to_pix(p_proj.x, a.W), gsr_ndc::to_pix(p_proj.y, a.H)};
             rect_min = {min(gridx, max(0, (int)((point_xy.x - width) / (float)a.bx))),
                         min(gridy, max(0, (int)((point_xy.y - height) / (float)a.by)))};
             rect_max = {min(gridx, max(0, (int)((point_xy.x + width) / (float)a.bx) + 1)),
