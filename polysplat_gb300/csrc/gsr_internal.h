@@ -167,9 +167,14 @@ constexpr size_t kMassiveQueueBytes = (size_t)kMassiveQueueEntries * sizeof(Mass
 // Small workspace for preprocess-only and render-only calls.
 constexpr size_t kSmallWorkspaceBytes = kHeaderBytes + kMassiveQueueBytes;
 
-constexpr int kSortThreads = 512;
-constexpr int kSortItems = 8;
-constexpr int kSortTile = kSortThreads * kSortItems;  // 4096 keys per tile
+// Digit-pass shape: 3 CTAs of 256 threads per SM, 14 keys per thread.  At
+// 9.2 M 64-bit pairs (5 passes and the first histogram): 349 us; 16 keys per
+// thread 380 (register spills), 13 keys 355, 12 keys at 4 CTAs 367, 512
+// threads x 8 keys at 2 CTAs 420.
+constexpr int kSortThreads = 256;
+constexpr int kSortItems = 14;
+constexpr int kSortCtas = 3;
+constexpr int kSortTile = kSortThreads * kSortItems;  // 3584 keys per tile
 constexpr int kMaxPasses = 8;
 
 size_t sort_workspace_bytes(long long cap);

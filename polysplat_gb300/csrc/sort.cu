@@ -10,14 +10,15 @@
 // Structure (one-sweep radix sort with decoupled look-back):
 //   1. k_upsweep: one read of all keys builds the 256-bin histogram of the
 //      first 8-bit digit, and clears the first look-back array.
-//   2. k_pass (one launch per digit): persistent CTAs take 4096-key tiles in
-//      order from an atomic counter, rank keys stably inside the tile (per-warp
-//      ranking by match.any or by bit ballots), publish per-digit tile counts,
-//      look back over earlier tiles for the running per-digit prefix (bounded
-//      spin, four predecessors per round trip), reorder the tile in shared
-//      memory by digit and write it out with coalesced stores.  While it holds
-//      a tile's keys it also counts their next digit, so the next pass's
-//      histogram is complete when this launch ends.
+//   2. k_pass (one launch per digit): persistent CTAs take 3584-key tiles in
+//      order from an atomic counter, count the tile's digits and publish the
+//      counts at once, rank the keys stably within each warp (match.any, lane
+//      masks in shared memory, or bit ballots) straight to their places in
+//      shared memory, look back over earlier tiles for the running per-digit
+//      prefix (bounded, eight predecessors per round trip), and write the tile
+//      out with coalesced stores.  While it holds a tile's keys it also counts
+//      their next digit, so the next pass's histogram is complete when this
+//      launch ends.
 //
 // Keys are mapped to an "ordering word" before digits are taken (OrderMap):
 // the masked key, or -- for keys the preprocess emitted -- the depth bits
@@ -41,6 +42,7 @@ constexpr uint32_t kFlagPrefix = 2u << 30;
 constexpr uint32_t kValueMask = (1u << 30) - 1u;
 constexpr int kWarpsPerCta = kSortThreads / 32;
 constexpr int kWarpItems = kSortItems * 32;  // consecutive keys per warp
+constexpr int kLook = 8;  // predecessors per look-back round trip
 
 template <typename K>
 struct SortJob {
@@ -192,241 +194,394 @@ template <typename K>
 struct PassSmem {
     K keys[kSortTile];
     uint32_t vals[kSortTile];
-    uint8_t digs[kSortTile];            // each reordered key's digit, so the scatter need not recompute it
-    uint32_t whist[kWarpsPerCta][256];  // per-warp digit counts, then warp-exclusive offsets
-    uint32_t digit_excl[256];           // tile-local start of each digit
+    uint32_t whist[kWarpsPerCta][256];  // per-warp digit counts, then the warp's next position per digit
     int gofs[256];                      // global position of tile position 0 per digit
-    uint32_t gstart[256];               // global start of each digit (scan of histogram)
     uint32_t next_hist[256];            // this CTA's counts of the next pass's digit
+    uint32_t lanes[kWarpsPerCta][256];  // lanes of the warp holding each digit (kRankOr)
     uint32_t warp_sums[kWarpsPerCta];
     int tile;
 };
 
-// Exclusive scan of one value per thread over the whole CTA (kSortThreads);
-// the digit passes hold digit d's value in thread d and zeros above 255.
-__device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* warp_sums)
+// Shifts that give 0 from 32 on, as PTX's do.
+__device__ __forceinline__ uint32_t shl_clamp(uint32_t x, int n)
 {
-    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    uint32_t r;
+    asm("shl.b32 %0, %1, %2;" : "=r"(r) : "r"(x), "r"(n));
+    return r;
+}
+__device__ __forceinline__ uint32_t shr_clamp(uint32_t x, int n)
+{
+    uint32_t r;
+    asm("shr.u32 %0, %1, %2;" : "=r"(r) : "r"(x), "r"(n));
+    return r;
+}
+
+// One digit of the ordering word, in 32-bit operations: the word is lo - floor
+// in its low db bits and hi above them.
+struct Digit {
+    int lo_shift, hi_left, hi_right;
+    uint32_t mask;
+};
+
+__device__ __forceinline__ Digit digit_at(const KeyMap& m, int db, int shift)
+{
+    Digit d;
+    d.lo_shift = shift;
+    d.hi_left = max(db - shift, 0);
+    d.hi_right = max(shift - db, 0);
+    d.mask = (1u << min(8, m.bits - shift)) - 1u;
+    return d;
+}
+
+__device__ __forceinline__ uint32_t digit_of(uint64_t k, const Digit& d, uint32_t floor)
+{
+    const uint32_t lo = (uint32_t)k - floor, hi = (uint32_t)(k >> 32);
+    return (shr_clamp(lo, d.lo_shift) | shr_clamp(shl_clamp(hi, d.hi_left), d.hi_right)) & d.mask;
+}
+
+__device__ __forceinline__ uint32_t digit_of(uint32_t k, const Digit& d, uint32_t floor)
+{
+    return shr_clamp(k - floor, d.lo_shift) & d.mask;
+}
+
+// Exclusive scan over the CTA of one value per thread (thread = digit).  The
+// caller has a barrier before the next call.
+__device__ __forceinline__ uint32_t digit_scan(uint32_t v, uint32_t* warp_sums, unsigned lane, int warp)
+{
     uint32_t incl = v;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
-        uint32_t n = __shfl_up_sync(GSR_FULL_MASK, incl, d);
+        const uint32_t n = __shfl_up_sync(GSR_FULL_MASK, incl, d);
         if (lane >= (unsigned)d) incl += n;
     }
     if (lane == 31) warp_sums[warp] = incl;
     __syncthreads();
-    uint32_t wpre = 0;
+    uint32_t pre = incl - v;
 #pragma unroll
     for (int w = 0; w < kWarpsPerCta; w++)
-        if (w < (int)warp) wpre += warp_sums[w];
-    __syncthreads();
-    return wpre + incl - v;
+        if (w < warp) pre += warp_sums[w];
+    return pre;
 }
 
-// One digit pass.  Keys are ranked within each warp either with match.any
-// (one instruction per key) or with one ballot per digit bit.  RANK 2 picks
-// per pass: match.any for depth digits, ballots for digits holding tile ids
-// (measured at 3 M Gaussians / 1080p: 93 vs 111 us on depth digits, 134 vs
-// 120 us and 125 vs 109 us on the two tile-bit passes); RANK 0 / 1 force
-// ballots / match.any.
-template <typename K, int RANK>
-__global__ __launch_bounds__(kSortThreads, 2) void k_pass(SortJob<K> a, int pass)
+__device__ __forceinline__ unsigned lanemask_gt()
 {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    PassSmem<K>& S = *reinterpret_cast<PassSmem<K>*>(smem_raw);
-    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const KeyMap km = key_map(a.order, a.s.hdr);
-    const int passes = passes_of(km);
-    if (pass >= passes) return;  // nothing left to order in this digit
-    const int n = sort_count(a);
-    const int tiles = (n + kSortTile - 1) / kSortTile;
-    const int shift = 8 * pass;
-    const int bits = min(8, km.bits - shift);
-    const int tile_from = a.order.kind == kOrderDepthCompressed64 ? km.depth_bits : a.order.tile_from_bit;
-    const bool use_match = RANK == 1 || (RANK == 2 && shift + bits <= tile_from);
-    // ping-pong so that the last working pass writes the output buffers
-    const bool to_out = ((passes - 1 - pass) & 1) == 0;
-    K* alt_k = reinterpret_cast<K*>(a.s.alt_keys);
-    const K* kin = a.keys_in;
-    const uint32_t* vin = a.vals_in;
-    if (pass > 0) {
-        const bool prev_out = ((passes - pass) & 1) == 0;
-        kin = prev_out ? a.keys_out : alt_k;
-        vin = prev_out ? a.vals_out : a.s.alt_vals;
-    }
-    K* kout = to_out ? a.keys_out : alt_k;
-    uint32_t* vout = to_out ? a.vals_out : a.s.alt_vals;
-    // selects rather than a dynamic index, so the parameter block stays out of local memory
-    uint32_t* look = (pass & 1) ? a.s.look[1] : a.s.look[0];
-    uint32_t* look_next = (pass & 1) ? a.s.look[0] : a.s.look[1];
-    const bool clear_next = pass + 1 < passes;
-    WorkspaceHeader* hdr = a.s.hdr;
+    unsigned m;
+    asm("mov.u32 %0, %%lanemask_gt;" : "=r"(m));
+    return m;
+}
 
-    const bool digit_thread = threadIdx.x < 256;  // thread d owns digit d in the per-digit steps
-    // the next pass's histogram is counted here, from the keys this pass holds
-    const bool count_next = pass + 1 < passes;
-    if (digit_thread) S.next_hist[threadIdx.x] = 0u;
-    {
-        const uint32_t g = block_excl_scan(digit_thread ? hdr->hist[pass][threadIdx.x] : 0u, S.warp_sums);
-        if (digit_thread) S.gstart[threadIdx.x] = g;
-    }
+// What every tile of a pass shares.
+template <typename K>
+struct PassCtx {
+    const K* kin;
+    const uint32_t* vin;
+    K* kout;
+    uint32_t* vout;
+    uint32_t* look;
+    uint32_t* look_next;
+    WorkspaceHeader* hdr;
+    uint32_t* counter;  // next tile to claim
+    Digit dg, dn;  // this pass's digit and the next one's
+    uint32_t floor;
+    uint32_t spin_limit;
+    int n;
+    bool more;  // a pass follows
+};
 
-    for (;;) {
-        if (threadIdx.x == 0) S.tile = (int)atomicAdd(&hdr->pass_counter[pass], 1u);
-        for (int i = threadIdx.x; i < kWarpsPerCta * 256; i += kSortThreads) (&S.whist[0][0])[i] = 0u;
-        __syncthreads();
-        const int tile = S.tile;
-        if (tile >= tiles) break;
-        const long long tbase = (long long)tile * kSortTile;
-        const int tcount = (int)min((long long)kSortTile, (long long)n - tbase);
-        if (clear_next && digit_thread) look_next[(size_t)tile * 256 + threadIdx.x] = 0u;
+// The digit by where it lies in the key: DLo within the low word, DHi within
+// the high word, DMix across both.
+enum : int { kDLo = 0, kDHi = 1, kDMix = 2 };
 
-        // ---- load (warp-contiguous chunk) + stable per-warp rank ----
-        K key[kSortItems];
-        uint32_t val[kSortItems];
-        uint32_t dig[kSortItems];
-        uint32_t rank[kSortItems];
-        const int wbase = (int)warp * kWarpItems;
+template <int WHERE>
+__device__ __forceinline__ uint32_t digit_in(uint64_t k, const Digit& d, uint32_t floor)
+{
+    if (WHERE == kDLo) return ((uint32_t)k - floor) >> d.lo_shift & d.mask;
+    if (WHERE == kDHi) return (uint32_t)(k >> 32) >> d.hi_right & d.mask;
+    return digit_of(k, d, floor);
+}
+template <int WHERE>
+__device__ __forceinline__ uint32_t digit_in(uint32_t k, const Digit& d, uint32_t floor)
+{
+    return digit_of(k, d, floor);
+}
+
+// How a warp finds the lanes with its digit.
+enum : int { kRankBallot = 0, kRankMatch = 1, kRankOr = 2 };
+
+// Sum of the counts of digit `tid` over the tiles before `tile`: walk back
+// kLook predecessors per round trip; stop at the first inclusive prefix,
+// re-reading any entry that is not published yet.  Whole windows of published
+// counts, the usual case, are summed without looking at single entries.
+template <typename K>
+__device__ __forceinline__ uint32_t look_back(const PassCtx<K>& c, int tile, int tid)
+{
+    uint32_t excl = 0, spins = 0;
+    int j = tile - 1;
+    const uint32_t* at = c.look + (size_t)max(j, 0) * 256 + tid;
+    while (j >= 0) {
+        uint32_t v[kLook];
+        uint32_t sum = 0, any = 0, all = 0xFFFFFFFFu;
+        if (j >= kLook - 1) {
 #pragma unroll
-        for (int i = 0; i < kSortItems; i++) {
-            const int o = wbase + i * 32 + (int)lane;
-            if (o < tcount) {
-                key[i] = kin[tbase + o];
-                val[i] = vin[tbase + o];
-            } else {
-                key[i] = K(0);
-                val[i] = 0u;
-            }
+            for (int k = 0; k < kLook; k++) v[k] = ld_relaxed_u32(at - k * 256);
+        } else {
+#pragma unroll
+            for (int k = 0; k < kLook; k++) v[k] = j - k >= 0 ? ld_relaxed_u32(at - k * 256) : kFlagPrefix;
         }
 #pragma unroll
+        for (int k = 0; k < kLook; k++) {
+            sum += v[k];
+            any |= v[k];
+            all &= v[k];
+        }
+        if ((all & kFlagAgg) && !(any & kFlagPrefix)) {
+            excl += sum;  // the flags wrap past bit 29 and are masked off below
+            j -= kLook;
+            at -= kLook * 256;
+            continue;
+        }
+        bool stuck = false, done = false;
+#pragma unroll
+        for (int k = 0; k < kLook; k++) {
+            const bool live = !done && !stuck;
+            const bool pub = (v[k] & ~kValueMask) != 0u;
+            stuck = stuck || (live && !pub);
+            if (live && pub) {
+                excl += v[k];
+                j--;
+                done = (v[k] & kFlagPrefix) != 0u;
+            }
+        }
+        if (done) break;
+        at = c.look + (size_t)max(j, 0) * 256 + tid;
+        if (stuck && ++spins > c.spin_limit) {
+            record_error(&c.hdr->status, kErrTimeout);
+            break;
+        }
+    }
+    return excl & kValueMask;
+}
+
+template <bool FULL, int RANK, int WHERE, typename K>
+__device__ __forceinline__ void pass_tile(PassSmem<K>& S, const PassCtx<K>& c, int tile, int gstart, unsigned lane,
+                                          int warp, int tid)
+{
+    const long long tbase = (long long)tile * kSortTile;
+    const int tcount = FULL ? kSortTile : (int)((long long)c.n - tbase);
+    const int first = warp * kWarpItems + (int)lane;
+    uint32_t* wh = S.whist[warp];
+
+    // ---- load the warp's chunk, count its digits ----
+    K key[kSortItems];
+    uint32_t val[kSortItems];
+    {
+        const K* kp = c.kin + tbase + first;
+        const uint32_t* vp = c.vin + tbase + first;
+#pragma unroll
+        for (int i = 0; i < kSortItems; i++) key[i] = FULL || first + i * 32 < tcount ? kp[i * 32] : K(0);
+#pragma unroll
+        for (int i = 0; i < kSortItems; i++) val[i] = FULL || first + i * 32 < tcount ? vp[i * 32] : 0u;
+    }
+    if (c.more) c.look_next[(size_t)tile * 256 + tid] = 0u;
+#pragma unroll
+    for (int i = 0; i < kSortItems; i++)
+        if (FULL || first + i * 32 < tcount) atomicAdd(&wh[digit_in<WHERE>(key[i], c.dg, c.floor)], 1u);
+    if (c.more) {
+#pragma unroll
+        for (int i = 0; i < kSortItems; i++)
+            if (FULL || first + i * 32 < tcount) atomicAdd(&S.next_hist[digit_of(key[i], c.dn, c.floor)], 1u);
+    }
+    __syncthreads();
+
+    // ---- thread d: the tile's count of digit d, published before anything
+    //      else so that later tiles can look back over it; then the first
+    //      position of the digit in every warp ----
+    uint32_t dtot = 0, cw[kWarpsPerCta];
+    uint32_t* my = c.look + (size_t)tile * 256 + tid;
+#pragma unroll
+    for (int w = 0; w < kWarpsPerCta; w++) {
+        cw[w] = S.whist[w][tid];
+        dtot += cw[w];
+    }
+    st_relaxed_u32(my, (tile == 0 ? kFlagPrefix : kFlagAgg) | dtot);
+    const uint32_t dstart = digit_scan(dtot, S.warp_sums, lane, warp);
+    {
+        uint32_t run = dstart;
+#pragma unroll
+        for (int w = 0; w < kWarpsPerCta; w++) {
+            S.whist[w][tid] = run;
+            run += cw[w];
+        }
+    }
+    __syncthreads();
+
+    // ---- stable ranks: wh[d] is the warp's next position of digit d in the
+    //      tile's digit order; keys and values go straight to their places ----
+    {
+        const unsigned lt = lanemask_lt(), gt = lanemask_gt();
+#pragma unroll
         for (int i = 0; i < kSortItems; i++) {
-            const int o = wbase + i * 32 + (int)lane;
-            const bool ok = o < tcount;
-            const uint64_t w = order_word(key[i], km);
-            const uint32_t d = (uint32_t)(w >> shift) & ((1u << bits) - 1u);
-            dig[i] = d;
-            if (count_next && ok) atomicAdd(&S.next_hist[(uint32_t)(w >> (shift + 8)) & 0xFFu], 1u);
-            if (use_match) {
-                // out-of-range lanes get a value no real digit has
-                const unsigned peers = __match_any_sync(GSR_FULL_MASK, ok ? d : 0x100u + lane);
-                const int leader = __ffs(peers) - 1;
-                uint32_t base = 0;
-                if (ok && (int)lane == leader) {
-                    base = S.whist[warp][d];
-                    S.whist[warp][d] = base + __popc(peers);
-                }
-                base = __shfl_sync(GSR_FULL_MASK, base, leader);
-                rank[i] = base + __popc(peers & lanemask_lt());
+            const bool ok = FULL || first + i * 32 < tcount;
+            const uint32_t d = digit_in<WHERE>(key[i], c.dg, c.floor);
+            unsigned peers;
+            if (RANK == kRankMatch) {
+                peers = __match_any_sync(GSR_FULL_MASK, ok ? d : 0x100u);
+            } else if (RANK == kRankOr) {
+                uint32_t* m = S.lanes[warp];
+                if (ok) atomicOr(&m[d], 1u << lane);
+                __syncwarp();
+                peers = ok ? m[d] : 0u;
             } else {
-                unsigned peers = __ballot_sync(GSR_FULL_MASK, ok);
-                for (int b = 0; b < bits; b++) {
+                peers = FULL ? GSR_FULL_MASK : __ballot_sync(GSR_FULL_MASK, ok);
+#pragma unroll
+                for (int b = 0; b < 8; b++) {
                     const bool bit = (d >> b) & 1u;
                     const unsigned bb = __ballot_sync(GSR_FULL_MASK, bit);
                     peers &= bit ? bb : ~bb;
                 }
-                uint32_t base = 0;
-                if (ok) base = S.whist[warp][d];
-                __syncwarp();
-                if (ok && (lane == (unsigned)(__ffs(peers) - 1))) S.whist[warp][d] = base + __popc(peers);
-                __syncwarp();
-                rank[i] = base + __popc(peers & lanemask_lt());
+            }
+            uint32_t pos = 0;
+            if (ok) pos = wh[d] + __popc(peers & lt);
+            __syncwarp();
+            if (ok && (peers & gt) == 0u) {
+                wh[d] = pos + 1u;
+                if (RANK == kRankOr) S.lanes[warp][d] = 0u;
+            }
+            __syncwarp();
+            if (ok) {
+                S.keys[pos] = key[i];
+                S.vals[pos] = val[i];
             }
         }
-        __syncthreads();
+    }
 
-        // ---- per-digit offsets across warps; publish the tile's counts;
-        //      offsets across digits ----
-        uint32_t dtot = 0;
-        {
-            const int d = threadIdx.x;
-            if (digit_thread) {
-#pragma unroll
-                for (int w = 0; w < kWarpsPerCta; w++) {
-                    uint32_t c = S.whist[w][d];
-                    S.whist[w][d] = dtot;
-                    dtot += c;
-                }
-                // later tiles' look-back can use the count before this tile's scan is done
-                st_relaxed_u32(look + (size_t)tile * 256 + d, (tile == 0 ? kFlagPrefix : kFlagAgg) | dtot);
-            }
-            const uint32_t ex = block_excl_scan(dtot, S.warp_sums);
-            if (digit_thread) S.digit_excl[d] = ex;
-        }
-        __syncthreads();  // digit_excl complete
+    // ---- decoupled look-back: thread d owns digit d ----
+    {
+        const uint32_t excl = look_back(c, tile, tid);
+        if (tile != 0) st_relaxed_u32(my, kFlagPrefix | ((excl + dtot) & kValueMask));
+        S.gofs[tid] = gstart + (int)excl - (int)dstart;
+    }
+    __syncthreads();
 
-        // ---- reorder in shared memory: the warps without a digit do it while
-        //      the digit warps look back, and the digit warps after ----
-        auto reorder = [&]() {
+    // ---- coalesced scatter of the digit runs; the claim of the next tile
+    //      travels meanwhile ----
+    if (tid == 0) S.tile = (int)atomicAdd(c.counter, 1u);
+    bool oob = false;
 #pragma unroll
-            for (int i = 0; i < kSortItems; i++) {
-                const int o = wbase + i * 32 + (int)lane;
-                if (o < tcount) {
-                    const uint32_t pos = S.digit_excl[dig[i]] + S.whist[warp][dig[i]] + rank[i];
-                    S.keys[pos] = key[i];
-                    S.vals[pos] = val[i];
-                    S.digs[pos] = (uint8_t)dig[i];
-                }
-            }
-        };
-        if (!digit_thread) reorder();
-
-        // ---- decoupled look-back: thread d owns digit d ----
-        if (digit_thread) {
-            const int d = threadIdx.x;
-            uint32_t* my = look + (size_t)tile * 256 + d;
-            // walk back four predecessors per round trip; stop at the first
-            // inclusive prefix, re-reading any entry that is not published yet
-            uint32_t excl = 0;
-            int j = tile - 1;
-            uint32_t spins = 0;
-            bool done = j < 0;
-            while (!done) {
-                // four predecessors per round trip: measured faster than 8
-                // (+6%) or 16 (+25%) at 9.2 M keys
-                uint32_t v[4];
-#pragma unroll
-                for (int k = 0; k < 4; k++)
-                    v[k] = (j - k >= 0) ? ld_relaxed_u32(look + (size_t)(j - k) * 256 + d) : kFlagPrefix;
-#pragma unroll
-                for (int k = 0; k < 4; k++) {
-                    if (done) break;
-                    if ((v[k] & ~kValueMask) == 0u) break;  // not published yet: re-read from j
-                    excl += v[k] & kValueMask;
-                    j--;
-                    if ((v[k] & kFlagPrefix) || j < 0) done = true;
-                }
-                if (!done && (v[0] & ~kValueMask) == 0u) {
-                    if (++spins > a.spin_limit) {
-                        record_error(&hdr->status, kErrTimeout);
-                        break;
-                    }
-                    __nanosleep(32);
-                }
-            }
-            if (tile != 0) st_relaxed_u32(my, kFlagPrefix | ((excl + dtot) & kValueMask));
-            S.gofs[d] = (int)(S.gstart[d] + excl) - (int)S.digit_excl[d];
-            reorder();
-        }
-        __syncthreads();
-
-        // ---- coalesced scatter of the digit runs ----
-        bool oob = false;
-        for (int p = threadIdx.x; p < tcount; p += kSortThreads) {
+    for (int i = 0; i < kSortItems; i++) {
+        const int p = tid + i * kSortThreads;
+        if (FULL || p < tcount) {
             const K k = S.keys[p];
-            const long long g = (long long)S.gofs[S.digs[p]] + p;
-            if (g < 0 || g >= n) {  // only after a look-back timeout: never write outside the buffer
+            const uint32_t v = S.vals[p];
+            const int g = S.gofs[digit_in<WHERE>(k, c.dg, c.floor)] + p;
+            if ((unsigned)g < (unsigned)c.n) {
+                c.kout[g] = k;
+                c.vout[g] = v;
+            } else {  // only after a look-back timeout: never write outside the buffer
                 oob = true;
-                continue;
             }
-            kout[g] = k;
-            vout[g] = S.vals[p];
         }
-        if (oob) record_error(&hdr->status, kErrTimeout);
+    }
+    if (oob) record_error(&c.hdr->status, kErrTimeout);
+}
+
+template <int RANK, int WHERE, typename K>
+__device__ __forceinline__ void pass_tiles(PassSmem<K>& S, const PassCtx<K>& c, int gstart, unsigned lane,
+                                           int warp, int tid)
+{
+    const int tiles = (c.n + kSortTile - 1) / kSortTile;
+    for (;;) {
+        const int tile = S.tile;
+        if (tile >= tiles) break;
+        if ((long long)(tile + 1) * kSortTile <= (long long)c.n)
+            pass_tile<true, RANK, WHERE>(S, c, tile, gstart, lane, warp, tid);
+        else pass_tile<false, RANK, WHERE>(S, c, tile, gstart, lane, warp, tid);
+#pragma unroll
+        for (int k = 0; k < 8; k++) S.whist[warp][k * 32 + lane] = 0u;
         __syncthreads();
     }
+}
+
+// One digit pass.  Per 32 keys it issues about 85 warp instructions and 35 to
+// 50 shared-memory wavefronts (ranking, the reorder and its bank conflicts);
+// the shared-memory pipe (60-70% busy) and the latency of a tile's chain bound
+// it, not DRAM: 60-65 us at 9.2 M 64-bit pairs (3.4-3.7 TB/s of the 24 bytes a
+// pair), where a form with the counts published after the ranking, digits
+// from 64-bit shifts and every access predicated took 78-102 us at 180-250
+// instructions.
+//
+// RANK 2 picks the ranking per pass: match.any for depth digits, which a
+// Gaussian's adjacent keys share (its time grows with the number of distinct
+// digits among the lanes), lane masks in shared memory for digits holding
+// tile ids (all passes of a 13-bit sort of 9.2 M 32-bit pairs: 126 us against
+// 150 with ballots).  RANK 0 / 1 force ballots / match.any.
+template <typename K, int RANK>
+__global__ __launch_bounds__(kSortThreads, kSortCtas) void k_pass(SortJob<K> a, int pass)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    PassSmem<K>& S = *reinterpret_cast<PassSmem<K>*>(smem_raw);
+    static_assert(kSortThreads == 256, "thread d owns digit d");
+    const unsigned lane = threadIdx.x & 31u;
+    const int warp = threadIdx.x >> 5, tid = threadIdx.x;
+    const KeyMap km = key_map(a.order, a.s.hdr);
+    const int passes = passes_of(km);
+    if (pass >= passes) return;  // nothing left to order in this digit
+    const int shift = 8 * pass;
+    const int bits = min(8, km.bits - shift);
+    const int tile_from = a.order.kind == kOrderDepthCompressed64 ? km.depth_bits : a.order.tile_from_bit;
+    const bool depth_digit = shift + bits <= tile_from;
+    const int db = a.order.kind == kOrderDepthCompressed64 ? km.depth_bits : 32;
+    PassCtx<K> c;
+    c.n = sort_count(a);
+    c.floor = a.order.kind == kOrderMasked ? 0u : kDepthBitsFloor;
+    c.dg = digit_at(km, db, shift);
+    // ping-pong so that the last working pass writes the output buffers
+    const bool to_out = ((passes - 1 - pass) & 1) == 0;
+    K* alt_k = reinterpret_cast<K*>(a.s.alt_keys);
+    c.kin = a.keys_in;
+    c.vin = a.vals_in;
+    if (pass > 0) {
+        const bool prev_out = ((passes - pass) & 1) == 0;
+        c.kin = prev_out ? a.keys_out : alt_k;
+        c.vin = prev_out ? a.vals_out : a.s.alt_vals;
+    }
+    c.kout = to_out ? a.keys_out : alt_k;
+    c.vout = to_out ? a.vals_out : a.s.alt_vals;
+    // selects rather than a dynamic index, so the parameter block stays out of local memory
+    c.look = (pass & 1) ? a.s.look[1] : a.s.look[0];
+    c.look_next = (pass & 1) ? a.s.look[0] : a.s.look[1];
+    c.hdr = a.s.hdr;
+    c.spin_limit = a.spin_limit;
+    // the next pass's histogram is counted here, from the keys this pass holds
+    c.more = pass + 1 < passes;
+    c.dn = digit_at(km, db, c.more ? shift + 8 : shift);
+    c.counter = &a.s.hdr->pass_counter[pass];
+
+    S.next_hist[tid] = 0u;
+    if (tid == 0) S.tile = (int)atomicAdd(c.counter, 1u);
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        S.whist[warp][k * 32 + lane] = 0u;
+        S.lanes[warp][k * 32 + lane] = 0u;
+    }
+    // global start of digit tid
+    const int gstart = (int)digit_scan(a.s.hdr->hist[pass][tid], S.warp_sums, lane, warp);
+    __syncthreads();
+
+    const int where = sizeof(K) == 4 || shift + bits <= db ? kDLo : shift >= db ? kDHi : kDMix;
+    if (RANK == 1) {
+        pass_tiles<kRankMatch, kDMix>(S, c, gstart, lane, warp, tid);
+    } else if (RANK == 0) {
+        pass_tiles<kRankBallot, kDMix>(S, c, gstart, lane, warp, tid);
+    } else if (depth_digit) {
+        pass_tiles<kRankMatch, kDLo>(S, c, gstart, lane, warp, tid);
+    } else if (where == kDHi) {
+        pass_tiles<kRankOr, kDHi>(S, c, gstart, lane, warp, tid);
+    } else {
+        pass_tiles<kRankOr, kDMix>(S, c, gstart, lane, warp, tid);
+    }
     // every count of this CTA precedes the barrier that ended its last tile
-    if (count_next && digit_thread && S.next_hist[threadIdx.x])
-        atomicAdd(&hdr->hist[pass + 1][threadIdx.x], S.next_hist[threadIdx.x]);
+    if (c.more && S.next_hist[tid]) atomicAdd(&a.s.hdr->hist[pass + 1][tid], S.next_hist[tid]);
 }
 
 // 2 (choose per sort and pass) unless GSR_SORT_RANK asks for "ballot" (0) or
@@ -460,13 +615,7 @@ cudaError_t run_sort(const SortJob<K>& job, int max_passes, cudaStream_t stream)
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     profile_mark(stream);
 
-    // per-pass choice only where depth and tile digits share the key; the
-    // choice costs a uniform branch per key, so all-depth and all-tile sorts
-    // keep the branch-free match.any kernel
-    const bool mixed = a.order.kind == kOrderDepthCompressed64 ||
-                       (a.order.tile_from_bit > 0 && a.order.tile_from_bit < a.order.end_bit);
-    const int forced = sort_rank_mode();
-    const int mode = forced != 2 ? forced : (mixed ? 2 : 1);
+    const int mode = sort_rank_mode();
     auto kern = mode == 0 ? k_pass<K, 0> : mode == 1 ? k_pass<K, 1> : k_pass<K, 2>;
     // per device and ranking mode: the shared-memory attribute (a property of
     // the kernel on each device), then the occupancy; host threads may race
