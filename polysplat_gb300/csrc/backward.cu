@@ -413,7 +413,7 @@ gsr_status gsr_train_backward_views(int P, const float* means, const float* log_
         return GSR_INVALID_ARG;
     const bool quad = (flags & GSR_QUAD_KEYS) != 0;
     if (quad && (long long)P * n_views > (long long)kQuadGidMask + 1) return GSR_INVALID_ARG;
-    if ((reinterpret_cast<uintptr_t>(grad_feat) & 15u) != 0) return GSR_INVALID_ARG;  // 16-byte atomics
+    if ((reinterpret_cast<uintptr_t>(grad_feat) & 15u) != 0) return GSR_INVALID_ARG;  // read as 16-byte vectors
     const int tiles = div_up(width, 16) * div_up(height, 16);
     if ((long long)P * n_views >= (1LL << 31) || (long long)tiles * n_views >= (1LL << 30)) return GSR_INVALID_ARG;
     if (P == 0) return GSR_OK;

@@ -300,7 +300,7 @@ struct TrainRenderArgs {
     float* grad_rgb;
     // when set, replaces the three arrays above: one 12-float record per
     // feature row, conic/opacity (4), xy (2), colour (3) and 3 unused, added
-    // to with three 16-byte atomics
+    // to by the lanes that hold the totals
     float* grad_rec;
 };
 cudaError_t launch_render_train(const TrainRenderArgs& a, bool backward, cudaStream_t stream);

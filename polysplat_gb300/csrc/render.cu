@@ -4,14 +4,13 @@
 // block of pixels (8 x 4 lanes over the tile, csrc/cuda_rasterizer/
 // render.cu:1736-1737).  Warps take tiles from a per-launch atomic queue in
 // the caller's workspace (no module-global counter, so concurrent launches on
-// different workspaces are safe).  The Gaussians of a tile are consumed in
-// batches of 32: for each batch every lane copies its Gaussian's
-// conic/opacity, colour/depth and centre records into one half of a
-// double-buffered shared-memory ring with per-thread cp.async copies, so the
-// next batch streams in while the current one is blended.  A second staging
-// path issues 1-D TMA bulk copies (cp.async.bulk) completed on an mbarrier
-// (GSR_RENDER_TMA=1); for these 16-byte gathers it measured slower.  Every
-// wait is bounded: on expiry the warp records a timeout in the status word
+// different workspaces are safe); with few tiles a CTA takes one tile.  The
+// Gaussians of a tile are consumed in batches of 32.  k_blend, which renders
+// almost everything, holds the next batch in registers and blends in paired
+// FP32; k_render is the scalar form for the general shader, the
+// distance-thresholded and the split renders, and stages batches with cp.async
+// or (GSR_RENDER_TMA=1) 1-D TMA bulk copies completed on an mbarrier, whose
+// waits are bounded: on expiry the warp records a timeout in the status word
 // and stops.
 //
 // The blend of each Gaussian-pixel pair is the reference's arithmetic
@@ -24,6 +23,7 @@
 #include <cstdlib>
 #include <cstring>
 
+#include "f32x2.cuh"
 #include "gsr_internal.h"
 
 namespace gsr {
@@ -452,6 +452,396 @@ __global__ __launch_bounds__(kRenderWarps * 32) void k_render(const RenderParams
     }
 }
 
+// ---------------------------------------------------------------------------
+// The blend with paired FP32 (shader 0, even tile widths, whole-tile exit).
+//
+// The scalar kernel above is bound by instruction issue: 12.9 thread
+// instructions per pixel and Gaussian at 70% issue.  Here the two columns of a
+// lane go through one fma.rn.f32x2, which gives each pixel the bits of the
+// scalar form (power = fma(b dx, dy, fma(c dy, dy, fma(a dx, dx, w))), C =
+// fma(rgb, alpha T, C), T - alpha T).  A paired instruction holds the FMA pipe
+// for two cycles, so it saves issue slots and not FMA work: a Gaussian costs a
+// warp 72 FMA cycles, 32 MUFU cycles and about 70 issue slots, and the FMA
+// pipe bounds the kernel.  The rows' terms, the same for both columns, are
+// scalar (as pairs they cost 8 FMA cycles more: 2429 against 2192 us per
+// frame of 20 M Gaussians at 7680x4320).  Four CTAs per SM at 120 registers:
+// five at 96 are slower (2623 us), as the Gaussians in flight per warp hide
+// more than another warp does.
+//
+// A batch's records are loaded into registers one batch ahead and its list
+// values one chunk before that, so neither load is waited for.  With DUP a
+// record's scalars are stored twice, so a broadcast read is an operand pair;
+// the kernels that split a tile over warps read every record four times and
+// store them once (5 instead of 9 shared-memory wavefronts per read).
+template <bool DUP>
+struct BlendRing {
+    float4 xyab[kBatch * (DUP ? 2 : 1)];  // x y a b, or x x y y and a a b b
+    float4 cwrg[kBatch * (DUP ? 2 : 1)];  // c w r g
+    float2 bl[kBatch];                    // b b
+    uint32_t gid[kBatch];
+    uint32_t ids[2 * kBatch];  // QUAD: list values of this tile not yet in a batch
+    int at[2 * kBatch];        // QUAD: their list positions
+};
+
+// One Gaussian's record as operand pairs.
+struct PairRecord {
+    f32x2 x, y, a, b, c, w, r, g, bl;
+};
+
+template <bool DUP>
+__device__ __forceinline__ PairRecord read_record(const BlendRing<DUP>& R, int k)
+{
+    PairRecord q;
+    if (DUP) {
+        const ulonglong2 xy = *reinterpret_cast<const ulonglong2*>(&R.xyab[2 * k]);
+        const ulonglong2 ab = *reinterpret_cast<const ulonglong2*>(&R.xyab[2 * k + 1]);
+        const ulonglong2 cw = *reinterpret_cast<const ulonglong2*>(&R.cwrg[2 * k]);
+        const ulonglong2 rg = *reinterpret_cast<const ulonglong2*>(&R.cwrg[2 * k + 1]);
+        q.x = xy.x;
+        q.y = xy.y;
+        q.a = ab.x;
+        q.b = ab.y;
+        q.c = cw.x;
+        q.w = cw.y;
+        q.r = rg.x;
+        q.g = rg.y;
+        q.bl = *reinterpret_cast<const f32x2*>(&R.bl[k]);
+    } else {
+        const float4 u = R.xyab[k], v = R.cwrg[k];
+        const float bl = R.bl[k].x;
+        q.x = pair(u.x, u.x);
+        q.y = pair(u.y, u.y);
+        q.a = pair(u.z, u.z);
+        q.b = pair(u.w, u.w);
+        q.c = pair(v.x, v.x);
+        q.w = pair(v.y, v.y);
+        q.r = pair(v.z, v.z);
+        q.g = pair(v.w, v.w);
+        q.bl = pair(bl, bl);
+    }
+    return q;
+}
+
+struct Features {
+    const float2* xy;
+    const float4* con;
+    const float4* rgbd;
+    const uint32_t* vals;
+    uint32_t P;
+};
+
+// Reads the list positions [start, end) in batches of up to 32 Gaussians, one
+// per lane, from the front or (REV) from the back.  QUAD: the quad's list is
+// compacted to the values with bit `sub_bit` set, in that order, through the
+// ring's ids; otherwise a batch is the next 32 values.
+template <bool QUAD, bool REV, bool DUP>
+struct Feed {
+    int pos, end;     // next list position to take, and where the list stops
+    uint32_t ahead;   // the lane's list value of the next chunk
+    int head, tail;   // QUAD: taken and stored ids
+    uint32_t sub_bit;
+    // the batch in registers
+    int n, where;     // its size; the lane's list position
+    uint32_t gid;     // feature row, ~0 outside the feature arrays
+    float2 xy;
+    float4 con, rgbd;
+
+    __device__ __forceinline__ int left() const { return REV ? pos - end : end - pos; }
+    __device__ __forceinline__ int mine(unsigned lane) const { return REV ? pos - 1 - (int)lane : pos + (int)lane; }
+
+    __device__ __forceinline__ void open(const Features& f, int start, int stop, uint32_t bit, unsigned lane)
+    {
+        pos = REV ? stop : start;
+        end = REV ? start : stop;
+        head = tail = 0;
+        sub_bit = bit;
+        ahead = (int)lane < left() ? __ldg(f.vals + mine(lane)) : 0u;
+    }
+
+    __device__ __forceinline__ void fetch(BlendRing<DUP>& R, const Features& f, unsigned lane, bool& bad)
+    {
+        uint32_t v = 0u;
+        if (QUAD) {
+            while (tail - head < kBatch && left() > 0) {
+                const bool hit = (int)lane < left() && (ahead & sub_bit) != 0u;
+                const unsigned m = __ballot_sync(GSR_FULL_MASK, hit);
+                if (hit) {
+                    const int slot = (tail + __popc(m & lanemask_lt())) & (2 * kBatch - 1);
+                    R.ids[slot] = ahead;
+                    R.at[slot] = mine(lane);
+                }
+                tail += __popc(m);
+                pos += REV ? -kBatch : kBatch;
+                ahead = (int)lane < left() ? __ldg(f.vals + mine(lane)) : 0u;
+            }
+            __syncwarp();
+            n = min(kBatch, tail - head);
+            if ((int)lane < n) {
+                const int slot = (head + (int)lane) & (2 * kBatch - 1);
+                v = R.ids[slot] & kQuadGidMask;
+                where = R.at[slot];
+            }
+            head += n;
+            __syncwarp();
+        } else {
+            n = max(0, min(kBatch, left()));
+            v = ahead;
+            where = mine(lane);
+            pos += REV ? -n : n;
+            ahead = (int)lane < left() ? __ldg(f.vals + mine(lane)) : 0u;
+        }
+        if ((int)lane < n) {
+            if (v < f.P) {
+                gid = v;
+                xy = __ldg(f.xy + v);
+                con = __ldg(f.con + v);
+                rgbd = __ldg(f.rgbd + v);
+            } else {  // index outside the feature arrays: a transparent stand-in
+                bad = true;
+                gid = 0xFFFFFFFFu;
+                xy = make_float2(0.f, 0.f);
+                con = make_float4(0.f, 0.f, 0.f, -1e30f);
+                rgbd = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        }
+    }
+
+    __device__ __forceinline__ void store(BlendRing<DUP>& R, unsigned lane) const
+    {
+        if ((int)lane < n) {
+            if (DUP) {
+                R.xyab[2 * lane] = make_float4(xy.x, xy.x, xy.y, xy.y);
+                R.xyab[2 * lane + 1] = make_float4(con.x, con.x, con.y, con.y);
+                R.cwrg[2 * lane] = make_float4(con.z, con.z, con.w, con.w);
+                R.cwrg[2 * lane + 1] = make_float4(rgbd.x, rgbd.x, rgbd.y, rgbd.y);
+            } else {
+                R.xyab[lane] = make_float4(xy.x, xy.y, con.x, con.y);
+                R.cwrg[lane] = make_float4(con.z, con.w, rgbd.x, rgbd.y);
+            }
+            R.bl[lane] = make_float2(rgbd.z, rgbd.z);
+            if (REV) R.gid[lane] = gid;  // the backward's gradient row
+        }
+    }
+};
+
+// A lane's TY x TX pixels: transmittance and colour, columns in pairs.
+template <int TX, int TY>
+struct Pixels {
+    f32x2 T[TY][TX / 2], C[TY][TX / 2][3];
+    f32x2 ncol[TX / 2];  // minus the pixels' coordinates
+    float nrow[TY];
+
+    __device__ __forceinline__ void reset(int x0, int y0)
+    {
+#pragma unroll
+        for (int j = 0; j < TX / 2; j++) ncol[j] = pair(-(float)(x0 + 2 * j), -(float)(x0 + 2 * j + 1));
+#pragma unroll
+        for (int i = 0; i < TY; i++) {
+            nrow[i] = -(float)(y0 + i);
+#pragma unroll
+            for (int j = 0; j < TX / 2; j++) {
+                T[i][j] = pair(1.0f, 1.0f);
+                C[i][j][0] = C[i][j][1] = C[i][j][2] = pair(0.0f, 0.0f);
+            }
+        }
+    }
+
+    __device__ __forceinline__ void blend(const PairRecord& q)
+    {
+        f32x2 xw[TX / 2], xb[TX / 2];
+#pragma unroll
+        for (int j = 0; j < TX / 2; j++) {
+            const f32x2 dx = add2(q.x, ncol[j]);
+            xw[j] = fma2(mul2(q.a, dx), dx, q.w);
+            xb[j] = mul2(q.b, dx);
+        }
+        const f32x2 minus1 = pair(-1.0f, -1.0f);
+#pragma unroll
+        for (int i = 0; i < TY; i++) {
+            const float y = __fadd_rn(lo_of(q.y), nrow[i]), cy = __fmul_rn(lo_of(q.c), y);
+            const f32x2 dy = pair(y, y), cdy = pair(cy, cy);
+#pragma unroll
+            for (int j = 0; j < TX / 2; j++) {
+                const f32x2 alpha = ex2_2(fma2(xb[j], dy, fma2(cdy, dy, xw[j])));
+                const f32x2 w = mul2(alpha, T[i][j]);
+                C[i][j][0] = fma2(q.r, w, C[i][j][0]);
+                C[i][j][1] = fma2(q.g, w, C[i][j][1]);
+                C[i][j][2] = fma2(q.bl, w, C[i][j][2]);
+                T[i][j] = fma2(w, minus1, T[i][j]);
+            }
+        }
+    }
+
+    // every pixel below the exit transmittance (a NaN is not)
+    __device__ __forceinline__ bool saturated() const
+    {
+        float m = 0.0f;
+#pragma unroll
+        for (int i = 0; i < TY; i++)
+#pragma unroll
+            for (int j = 0; j < TX / 2; j++) m = max_nan(m, max_nan(lo_of(T[i][j]), hi_of(T[i][j])));
+        return m < 0.0001f;
+    }
+};
+
+// Blends the list positions [start, end) front to back, up to the whole-tile
+// exit checked every CADENCE Gaussians.  Returns whether the tile has a
+// Gaussian; `last` is the list position of the last one blended.  SPLIT > 1:
+// the CTA's warps each hold a strip of the tile's rows and exit together.
+template <int TX, int TY, int CADENCE, bool QUAD, int SPLIT>
+__device__ __forceinline__ bool blend_list(Pixels<TX, TY>& px, BlendRing<SPLIT == 1>& R, const Features& f, int start,
+                                           int end, uint32_t sub_bit, unsigned lane, bool& bad, int& last)
+{
+    static_assert(kBatch % CADENCE == 0, "the exit checks fall on the same Gaussian of every full batch");
+    Feed<QUAD, false, SPLIT == 1> feed;
+    feed.open(f, start, end, sub_bit, lane);
+    feed.fetch(R, f, lane, bad);
+    bool any = false;
+    while (feed.n > 0) {
+        const int n = feed.n, where = feed.where;
+        __syncwarp();
+        feed.store(R, lane);
+        __syncwarp();
+        feed.fetch(R, f, lane, bad);
+        any = true;
+        int done = n;
+        bool stop = false;
+        for (int g0 = 0; g0 < n; g0 += CADENCE) {
+            if (g0 + CADENCE <= n) {
+#pragma unroll 2
+                for (int g = g0; g < g0 + CADENCE; g++) px.blend(read_record(R, g));
+                const bool sat = px.saturated();
+                if (SPLIT > 1 ? __syncthreads_and(sat) != 0 : __all_sync(GSR_FULL_MASK, sat) != 0) {
+                    done = g0 + CADENCE;
+                    stop = true;
+                    break;
+                }
+            } else {
+                for (int g = g0; g < n; g++) px.blend(read_record(R, g));
+            }
+        }
+        last = __shfl_sync(GSR_FULL_MASK, where, done - 1);
+        if (stop) break;
+    }
+    __syncwarp();
+    return any;
+}
+
+// A render of few tiles, where a tile per warp would not even fill the warps
+// that fit on the GPU at once (4 CTAs of 4 per SM), takes a tile per CTA, four
+// rows to a warp: each tile's chain of Gaussians is then a quarter of the work
+// per step.  With more tiles the fourfold record reads cost more than the
+// shorter chains give.  Training steps, render backward, tile per warp against
+// tile per CTA: 1900 tiles 408 / 294 us, 2400 tiles 339 / 274 us, 3600 tiles
+// 362 / 522 us, 28800 tiles 1873 / 3698 us; the forwards cross at the same
+// place.
+static bool split_tiles(long long tiles) { return tiles <= 16LL * device_sm_count(); }
+
+// Persistent render, a tile per warp; with SPLIT = 4 a tile per CTA and no
+// queue.
+template <int BX, int BY, int CADENCE, int RANGE_MODE, bool BATCH, bool QUAD, int SPLIT>
+__global__ __launch_bounds__(kRenderWarps * 32, BX * BY == 256 ? 4 : 1) void k_blend(const RenderParams p)
+{
+    static_assert(!QUAD || (BX == 16 && BY == 16), "quad renders: 16x16 tiles");
+    static_assert(SPLIT == 1 || (SPLIT == kRenderWarps && BY == 16), "a tile per warp, or per CTA");
+    constexpr int TX = BX / 8, TY = BY / 4 / SPLIT;
+    __shared__ BlendRing<SPLIT == 1> rings[kRenderWarps];
+    const unsigned lane = threadIdx.x & 31u;
+    const int warp = threadIdx.x >> 5;
+    BlendRing<SPLIT == 1>& R = rings[warp];
+    const long long nl = p.d_num ? (long long)*p.d_num : (long long)p.n_host;
+    const int n = (int)max(0LL, min(nl, p.cap));
+    const int cb = (int)(lane & 7u) * TX;
+    const int rb = (SPLIT > 1 ? warp * (BY / SPLIT) : 0) + (int)(lane >> 3) * TY;
+    const Features f{p.xy, p.con, p.rgbd, p.vals, (uint32_t)p.P};
+    bool bad = false;
+
+    int item = SPLIT > 1 ? (int)blockIdx.x : (int)blockIdx.x * kRenderWarps + warp;
+    while (item < p.items) {
+        const int tile = QUAD ? (item >> 2) : item;  // key tile id (a quad's id for QUAD)
+        const int sub = item & 3;                     // QUAD: which tile of the quad
+        int W = p.W, H = p.H, gx = p.gx, ltile = tile;
+        float3 bg = p.bg;
+        uchar3* out = p.out;
+        if (BATCH) {
+            // the view holding this global tile: last tile_base <= tile
+            int lo = 0, hi = p.n_views - 1;
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if (__ldg(&p.views[mid].tile_base) <= tile) lo = mid;
+                else hi = mid - 1;
+            }
+            const RenderView& v = p.views[lo];
+            W = v.W;
+            H = v.H;
+            gx = max(1, v.gx);
+            ltile = tile - v.tile_base;
+            bg = make_float3(v.bg[0], v.bg[1], v.bg[2]);
+            out = reinterpret_cast<uchar3*>(v.out);
+        }
+        const int ox = QUAD ? (ltile % gx) * 32 + (sub & 1) * 16 : (ltile % gx) * BX;
+        const int oy = QUAD ? (ltile / gx) * 32 + (sub >> 1) * 16 : (ltile / gx) * BY;
+        if (!QUAD || (ox < W && oy < H)) {  // a quad's tile beyond the image edge has no pixels
+            int start, end;
+            if (RANGE_MODE == 0) {
+                const int2 r = __ldg(p.ranges + tile);
+                // ranges come from the caller: keep them inside [0, n]
+                start = min(max(r.x, 0), n);
+                end = min(max(r.y, start), n);
+            } else {
+                start = warp_bound<false>(p.keys, 0, n, (uint32_t)tile, lane);
+                end = warp_bound<true>(p.keys, start, n, (uint32_t)tile, lane);
+            }
+            Pixels<TX, TY> px;
+            px.reset(ox + cb, oy + rb);
+            int last = 0;
+            const bool any = blend_list<TX, TY, CADENCE, QUAD, SPLIT>(
+                px, R, f, start, end, QUAD ? (1u << (kQuadShift + sub)) : 0u, lane, bad, last);
+#pragma unroll
+            for (int i = 0; i < TY; i++)
+#pragma unroll
+                for (int j = 0; j < TX; j++) {
+                    const int x = ox + cb + j, y = oy + rb + i;
+                    auto half = [&](f32x2 v) { return (j & 1) ? hi_of(v) : lo_of(v); };
+                    const float c[3] = {half(px.C[i][j / 2][0]), half(px.C[i][j / 2][1]), half(px.C[i][j / 2][2])};
+                    if (x < W && y < H) out[(size_t)y * W + x] = encode_px(c, half(px.T[i][j / 2]), any, bg);
+                }
+        }
+        if (SPLIT > 1) break;
+        int next = 0;
+        if (lane == 0) next = (int)atomicAdd(p.queue, 1u) + (int)gridDim.x * kRenderWarps;
+        item = __shfl_sync(GSR_FULL_MASK, next, 0);
+    }
+    if (__any_sync(GSR_FULL_MASK, bad) && lane == 0) record_error(p.status, kErrBadInput);
+}
+
+template <int BX, int BY, int CADENCE, int RANGE_MODE, bool BATCH, bool QUAD = false>
+cudaError_t launch_blend(const RenderParams& p, cudaStream_t stream)
+{
+    if constexpr (BX == 16 && BY == 16) {
+        if (split_tiles(p.items)) {
+            k_blend<BX, BY, CADENCE, RANGE_MODE, BATCH, QUAD, kRenderWarps>
+                <<<p.items, kRenderWarps * 32, 0, stream>>>(p);
+            return cudaGetLastError();
+        }
+    }
+    auto kern = k_blend<BX, BY, CADENCE, RANGE_MODE, BATCH, QUAD, 1>;
+    // per device; host threads may race to fill it with the same value
+    static std::atomic<int> per_sm_cache[kMaxDevices];
+    const int dev = current_device();
+    if (dev < 0) return cudaErrorInvalidDevice;
+    int per_sm = per_sm_cache[dev].load(std::memory_order_relaxed);
+    if (per_sm == 0) {
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kRenderWarps * 32, 0) != cudaSuccess ||
+            per_sm < 1)
+            per_sm = 1;
+        per_sm_cache[dev].store(per_sm, std::memory_order_relaxed);
+    }
+    const int grid = max(1, min(device_sm_count() * per_sm, div_up(p.items, kRenderWarps)));
+    kern<<<grid, kRenderWarps * 32, 0, stream>>>(p);
+    return cudaGetLastError();
+}
+
 template <int BX, int BY, int CADENCE, int SHADER, bool DT, int RANGE_MODE, bool TMA, bool BATCH = false,
           int EXIT = 0, bool QUAD = false>
 cudaError_t launch_variant(const RenderParams& p, cudaStream_t stream)
@@ -475,6 +865,17 @@ cudaError_t launch_variant(const RenderParams& p, cudaStream_t stream)
     return cudaGetLastError();
 }
 
+// TMA staging, the distance-thresholded and the split renders, the general
+// shader (SH 1) and 24-wide tiles take the scalar kernel; the rest take the
+// paired one.
+template <int BX, int BY, int CADENCE, int SHADER, int RANGE_MODE>
+cudaError_t launch_whole(bool tma, const RenderParams& p, cudaStream_t stream)
+{
+    if (tma) return launch_variant<BX, BY, CADENCE, SHADER, false, RANGE_MODE, true>(p, stream);
+    if constexpr (SHADER == 0 && BX % 16 == 0) return launch_blend<BX, BY, CADENCE, RANGE_MODE, false>(p, stream);
+    else return launch_variant<BX, BY, CADENCE, SHADER, false, RANGE_MODE, false>(p, stream);
+}
+
 template <int BX, int BY>
 cudaError_t dispatch_shape(int variant, bool tma, const RenderParams& p, cudaStream_t stream)
 {
@@ -483,24 +884,12 @@ cudaError_t dispatch_shape(int variant, bool tma, const RenderParams& p, cudaStr
     // (the same [lower, upper) bounds, so the same image)
     const bool ranges = p.ranges != nullptr;
     switch (variant) {
-    case GSR_RENDER_PERSISTENT_RANGES:
-        return tma ? launch_variant<BX, BY, 8, 0, false, 0, true>(p, stream)
-                   : launch_variant<BX, BY, 8, 0, false, 0, false>(p, stream);
+    case GSR_RENDER_PERSISTENT_RANGES: return launch_whole<BX, BY, 8, 0, 0>(tma, p, stream);
     case GSR_RENDER_PERSISTENT_FUSED:
-        if (ranges)
-            return tma ? launch_variant<BX, BY, 16, 0, false, 0, true>(p, stream)
-                       : launch_variant<BX, BY, 16, 0, false, 0, false>(p, stream);
-        return tma ? launch_variant<BX, BY, 16, 0, false, 1, true>(p, stream)
-                   : launch_variant<BX, BY, 16, 0, false, 1, false>(p, stream);
+        return ranges ? launch_whole<BX, BY, 16, 0, 0>(tma, p, stream) : launch_whole<BX, BY, 16, 0, 1>(tma, p, stream);
     case GSR_RENDER_DEFAULT:
-        if (ranges)
-            return tma ? launch_variant<BX, BY, 2, SH, false, 0, true>(p, stream)
-                       : launch_variant<BX, BY, 2, SH, false, 0, false>(p, stream);
-        return tma ? launch_variant<BX, BY, 2, SH, false, 1, true>(p, stream)
-                   : launch_variant<BX, BY, 2, SH, false, 1, false>(p, stream);
-    case GSR_RENDER_RANGES_CADENCE2:
-        return tma ? launch_variant<BX, BY, 2, SH, false, 0, true>(p, stream)
-                   : launch_variant<BX, BY, 2, SH, false, 0, false>(p, stream);
+        return ranges ? launch_whole<BX, BY, 2, SH, 0>(tma, p, stream) : launch_whole<BX, BY, 2, SH, 1>(tma, p, stream);
+    case GSR_RENDER_RANGES_CADENCE2: return launch_whole<BX, BY, 2, SH, 0>(tma, p, stream);
     case GSR_RENDER_DT:
         return tma ? launch_variant<BX, BY, 8, 0, true, 0, true>(p, stream)
                    : launch_variant<BX, BY, 8, 0, true, 0, false>(p, stream);
@@ -519,14 +908,14 @@ cudaError_t dispatch_quad(int variant, const RenderParams& p, cudaStream_t strea
 {
     const bool ranges = p.ranges != nullptr;
     switch (variant) {
-    case GSR_RENDER_PERSISTENT_RANGES: return launch_variant<16, 16, 8, 0, false, 0, false, BATCH, 0, true>(p, stream);
+    case GSR_RENDER_PERSISTENT_RANGES: return launch_blend<16, 16, 8, 0, BATCH, true>(p, stream);
     case GSR_RENDER_PERSISTENT_FUSED:
-        if (ranges || BATCH) return launch_variant<16, 16, 16, 0, false, 0, false, BATCH, 0, true>(p, stream);
-        return launch_variant<16, 16, 16, 0, false, 1, false, false, 0, true>(p, stream);
+        if (ranges || BATCH) return launch_blend<16, 16, 16, 0, BATCH, true>(p, stream);
+        return launch_blend<16, 16, 16, 1, false, true>(p, stream);
     case GSR_RENDER_DEFAULT:
-        if (ranges || BATCH) return launch_variant<16, 16, 2, 0, false, 0, false, BATCH, 0, true>(p, stream);
-        return launch_variant<16, 16, 2, 0, false, 1, false, false, 0, true>(p, stream);
-    case GSR_RENDER_RANGES_CADENCE2: return launch_variant<16, 16, 2, 0, false, 0, false, BATCH, 0, true>(p, stream);
+        if (ranges || BATCH) return launch_blend<16, 16, 2, 0, BATCH, true>(p, stream);
+        return launch_blend<16, 16, 2, 1, false, true>(p, stream);
+    case GSR_RENDER_RANGES_CADENCE2: return launch_blend<16, 16, 2, 0, BATCH, true>(p, stream);
     case GSR_RENDER_DT: return launch_variant<16, 16, 8, 0, true, 0, false, BATCH, 0, true>(p, stream);
     default: return cudaErrorInvalidValue;
     }
@@ -539,10 +928,12 @@ cudaError_t dispatch_batch(int variant, const RenderParams& p, cudaStream_t stre
 {
     constexpr int SH = (BX == 16 && BY == 16) ? 0 : 1;
     switch (variant) {
-    case GSR_RENDER_PERSISTENT_RANGES: return launch_variant<BX, BY, 8, 0, false, 0, false, true>(p, stream);
-    case GSR_RENDER_PERSISTENT_FUSED: return launch_variant<BX, BY, 16, 0, false, 0, false, true>(p, stream);
+    case GSR_RENDER_PERSISTENT_RANGES: return launch_blend<BX, BY, 8, 0, true>(p, stream);
+    case GSR_RENDER_PERSISTENT_FUSED: return launch_blend<BX, BY, 16, 0, true>(p, stream);
     case GSR_RENDER_DEFAULT:
-    case GSR_RENDER_RANGES_CADENCE2: return launch_variant<BX, BY, 2, SH, false, 0, false, true>(p, stream);
+    case GSR_RENDER_RANGES_CADENCE2:
+        if constexpr (SH == 0) return launch_blend<BX, BY, 2, 0, true>(p, stream);
+        else return launch_variant<BX, BY, 2, SH, false, 0, false, true>(p, stream);
     case GSR_RENDER_DT: return launch_variant<BX, BY, 8, 0, true, 0, false, true>(p, stream);
     default: return cudaErrorInvalidValue;
     }
@@ -576,151 +967,179 @@ namespace {
 constexpr int kTrainWarps = 4;
 constexpr int kTrainCadence = 8;
 
-struct TrainBatch {
-    float2 xy[32];
-    float4 con[32];
-    float4 rgb[32];
-    uint32_t gid[32];
-    uint32_t use[32];  // the entry belongs to this tile (quad keys: its bit is set)
-};
-
 // Where tile (tx, ty) of `view` finds its list: its own range, or with quad
 // keys its quad's range, whose entries carry the bit `qbit` when they
 // belong to this tile.
-__device__ __forceinline__ int train_list(const TrainRenderArgs& a, int view, int tile, int tx, int ty, int gx, int gy,
-                                          uint32_t& qbit)
+template <bool QUAD>
+__device__ __forceinline__ int train_list(int view, int tile, int tx, int ty, int gx, int gy, uint32_t& qbit)
 {
     qbit = 0u;
-    if (!a.quad) return tile;
+    if (!QUAD) return tile;
     const int qgx = quad_cols(gx), qpv = qgx * quad_cols(gy);
     qbit = 1u << (kQuadShift + ((tx & 1) | ((ty & 1) << 1)));
     return view * qpv + (ty >> 1) * qgx + (tx >> 1);
 }
 
-// One list entry: false when it is another tile's (quad keys), else its
-// Gaussian in g.
-__device__ __forceinline__ bool train_entry(const TrainRenderArgs& a, uint32_t v, uint32_t qbit, uint32_t& g)
-{
-    if (!a.quad) {
-        g = v;
+// The tile (or strip of a tile) of a warp of the training kernels.
+template <bool QUAD, int SPLIT>
+struct TrainTile {
+    int tile, start, stop, ox, oy, cb, rb;
+    size_t pix0;
+    uint32_t qbit;
+
+    __device__ __forceinline__ bool open(const TrainRenderArgs& a, unsigned lane, int warp)
+    {
+        // tile: global over the views; lt: within its view
+        const int gx = (a.W + 15) / 16, gy = (a.H + 15) / 16, tiles = gx * gy;
+        tile = SPLIT > 1 ? (int)blockIdx.x : (int)blockIdx.x * kTrainWarps + warp;
+        if (tile >= tiles * max(a.n_views, 1)) return false;
+        const int view = tile / tiles, lt = tile - view * tiles;
+        pix0 = (size_t)view * a.W * a.H;
+        const int n = (int)max(0LL, min((long long)*a.d_num, a.cap));
+        const int tx = lt % gx, ty = lt / gx;
+        ox = tx * 16;
+        oy = ty * 16;
+        cb = (int)(lane & 7u) * 2;
+        rb = (SPLIT > 1 ? warp * (16 / SPLIT) : 0) + (int)(lane >> 3) * (4 / SPLIT);
+        const int2 rg = __ldg(a.ranges + train_list<QUAD>(view, tile, tx, ty, gx, gy, qbit));
+        start = min(max(rg.x, 0), n);
+        stop = min(max(rg.y, start), n);
         return true;
     }
-    g = v & kQuadGidMask;
-    return (v & qbit) != 0u;
-}
+};
 
-__global__ __launch_bounds__(kTrainWarps * 32) void k_render_train(const TrainRenderArgs a)
+template <bool QUAD, int SPLIT>
+__global__ __launch_bounds__(kTrainWarps * 32, 4) void k_render_train(const TrainRenderArgs a)
 {
-    __shared__ TrainBatch sb[kTrainWarps];
+    static_assert(SPLIT == 1 || SPLIT == kTrainWarps, "a tile per warp, or per CTA");
+    constexpr int TY = 4 / SPLIT;
+    __shared__ BlendRing<SPLIT == 1> rings[kTrainWarps];
     const unsigned lane = threadIdx.x & 31u;
     const int warp = threadIdx.x >> 5;
-    TrainBatch& B = sb[warp];
-    // tile: global over the views; lt: within its view
-    const int gx = (a.W + 15) / 16, gy = (a.H + 15) / 16, tiles = gx * gy;
-    const int tile = blockIdx.x * kTrainWarps + warp;
-    if (tile >= tiles * max(a.n_views, 1)) return;
-    const int view = tile / tiles, lt = tile - view * tiles;
-    const size_t pix0 = (size_t)view * a.W * a.H;
-    const int n = (int)max(0LL, min((long long)*a.d_num, a.cap));
-    const int tx = lt % gx, ty = lt / gx;
-    const int ox = tx * 16, oy = ty * 16;
-    const int cb = (int)(lane & 7u) * 2, rb = (int)(lane >> 3) * 4;
-    uint32_t qbit;
-    const int2 rg = __ldg(a.ranges + train_list(a, view, tile, tx, ty, gx, gy, qbit));
-    const int start = min(max(rg.x, 0), n), end = min(max(rg.y, start), n);
-    float T[4][2], C[4][2][3];
+    TrainTile<QUAD, SPLIT> t;
+    if (!t.open(a, lane, warp)) return;
+    const Features f{a.xy, a.con, a.rgbd, a.vals, (uint32_t)a.P};
+    Pixels<2, TY> px;
+    px.reset(t.ox + t.cb, t.oy + t.rb);
+    bool bad = false;
+    int last = 0;
+    const bool any =
+        blend_list<2, TY, kTrainCadence, QUAD, SPLIT>(px, rings[warp], f, t.start, t.stop, t.qbit, lane, bad, last);
+    // list positions up to the last Gaussian blended: what the backward replays
+    if (lane == 0 && (SPLIT == 1 || warp == 0)) a.n_tile[t.tile] = any ? last - t.start + 1 : 0;
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+    for (int i = 0; i < TY; i++)
 #pragma unroll
         for (int j = 0; j < 2; j++) {
-            T[i][j] = 1.0f;
-            C[i][j][0] = C[i][j][1] = C[i][j][2] = 0.0f;
-        }
-    // processed: Gaussians blended (the exit cadence counts these); used:
-    // list positions up to the last one blended, what the backward replays
-    int processed = 0, used = 0;
-    bool exit_now = false;
-    for (int pos = start; pos < end && !exit_now; pos += 32) {
-        const int cnt = min(32, end - pos);
-        __syncwarp();
-        if ((int)lane < cnt) {
-            uint32_t g;
-            const bool mine = train_entry(a, __ldg(a.vals + pos + lane), qbit, g);
-            B.use[lane] = mine ? 1u : 0u;
-            if (mine && g < (uint32_t)a.P) {
-                B.xy[lane] = __ldg(a.xy + g);
-                B.con[lane] = __ldg(a.con + g);
-                B.rgb[lane] = __ldg(a.rgbd + g);
-            } else {  // another tile's, or outside the feature arrays: a transparent stand-in
-                B.xy[lane] = make_float2(0.f, 0.f);
-                B.con[lane] = make_float4(0.f, 0.f, 0.f, -1e30f);
-                B.rgb[lane] = make_float4(0.f, 0.f, 0.f, 0.f);
-            }
-        }
-        __syncwarp();
-        for (int k = 0; k < cnt; k++) {
-            if (!B.use[k]) continue;
-            const float4 rgb = B.rgb[k];
-            shade<2, 4, 0, false>(C, T, ox, oy, cb, rb, B.xy[k], B.con[k], make_float3(rgb.x, rgb.y, rgb.z));
-            ++processed;
-            used = pos - start + k + 1;
-            if (processed % kTrainCadence == 0) {
-                bool sat = true;
-#pragma unroll
-                for (int i = 0; i < 4; i++)
-#pragma unroll
-                    for (int j = 0; j < 2; j++) sat = sat && T[i][j] < 0.0001f;
-                if (__all_sync(GSR_FULL_MASK, sat)) {
-                    exit_now = true;
-                    break;
-                }
-            }
-        }
-    }
-    if (lane == 0) a.n_tile[tile] = used;
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 2; j++) {
-            const int px = ox + cb + j, py = oy + rb + i;
-            if (px >= a.W || py >= a.H) continue;
-            const size_t o = pix0 + (size_t)py * a.W + px;
-            const float t = T[i][j], tt = t < 0.0001f ? 0.0f : t;
-            a.T_final[o] = t;
-            a.image[3 * o + 0] = C[i][j][0] + tt * a.bg[0];
-            a.image[3 * o + 1] = C[i][j][1] + tt * a.bg[1];
-            a.image[3 * o + 2] = C[i][j][2] + tt * a.bg[2];
+            const int x = t.ox + t.cb + j, y = t.oy + t.rb + i;
+            if (x >= a.W || y >= a.H) continue;
+            auto half = [&](f32x2 v) { return j ? hi_of(v) : lo_of(v); };
+            const size_t o = t.pix0 + (size_t)y * a.W + x;
+            const float T = half(px.T[i][0]), tt = T < 0.0001f ? 0.0f : T;
+            a.T_final[o] = T;
+            a.image[3 * o + 0] = half(px.C[i][0][0]) + tt * a.bg[0];
+            a.image[3 * o + 1] = half(px.C[i][0][1]) + tt * a.bg[1];
+            a.image[3 * o + 2] = half(px.C[i][0][2]) + tt * a.bg[2];
         }
 }
 
-__device__ __forceinline__ float warp_sum(float v)
+// One step of a spread sum: lanes whose bit `d` is set keep b and send a, the
+// others keep a and send b.
+__device__ __forceinline__ float spread(float a, float b, bool up, int d)
 {
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(GSR_FULL_MASK, v, d);
-    return v;
+    return (up ? b : a) + __shfl_xor_sync(GSR_FULL_MASK, up ? a : b, d);
 }
 
-// Sums of eight values over the warp in 9 shuffles instead of 40: at each of
-// the first three steps a lane keeps half of its partial sums and sends the
-// other half to its partner.  Lane l returns the total of
-// v[((l >> 4) & 1) * 4 + ((l >> 3) & 1) * 2 + ((l >> 2) & 1)], that is
-// v[l >> 2] for every lane l with l & 3 == 0.
-__device__ __forceinline__ float warp_sum8_spread(const float (&v)[8], unsigned lane)
+// Sums of sixteen values over the warp in 16 shuffles: at each of the first
+// four steps a lane keeps half of its partial sums and sends the other half
+// to its partner.  Lane l returns the total of v[l >> 1].
+__device__ __forceinline__ float warp_sum16_spread(const float (&v)[16], unsigned lane)
 {
-    const bool b4 = (lane & 16u) != 0u, b3 = (lane & 8u) != 0u, b2 = (lane & 4u) != 0u;
-    float h[4];
+    float h[8], q[4], p[2];
 #pragma unroll
-    for (int k = 0; k < 4; k++)
-        h[k] = (b4 ? v[k + 4] : v[k]) + __shfl_xor_sync(GSR_FULL_MASK, b4 ? v[k] : v[k + 4], 16);
-    float q[2];
+    for (int k = 0; k < 8; k++) h[k] = spread(v[k], v[k + 8], (lane & 16u) != 0u, 16);
 #pragma unroll
-    for (int k = 0; k < 2; k++)
-        q[k] = (b3 ? h[k + 2] : h[k]) + __shfl_xor_sync(GSR_FULL_MASK, b3 ? h[k] : h[k + 2], 8);
-    float t = (b2 ? q[1] : q[0]) + __shfl_xor_sync(GSR_FULL_MASK, b2 ? q[0] : q[1], 4);
-    t += __shfl_xor_sync(GSR_FULL_MASK, t, 2);
-    t += __shfl_xor_sync(GSR_FULL_MASK, t, 1);
+    for (int k = 0; k < 4; k++) q[k] = spread(h[k], h[k + 4], (lane & 8u) != 0u, 8);
+#pragma unroll
+    for (int k = 0; k < 2; k++) p[k] = spread(q[k], q[k + 2], (lane & 4u) != 0u, 4);
+    const float t = spread(p[0], p[1], (lane & 2u) != 0u, 2);
+    return t + __shfl_xor_sync(GSR_FULL_MASK, t, 1);
+}
+
+// Sums of two values: lane l returns the total of v[l >> 4].
+__device__ __forceinline__ float warp_sum2_spread(float a, float b, unsigned lane)
+{
+    float t = spread(a, b, (lane & 16u) != 0u, 16);
+#pragma unroll
+    for (int d = 8; d > 0; d >>= 1) t += __shfl_xor_sync(GSR_FULL_MASK, t, d);
     return t;
 }
+
+// A lane's TY x 2 pixels of the reverse walk, columns in pairs.  R . G is
+// carried as one number per pixel: the walk only needs the colour behind a
+// Gaussian through its product with the pixel's gradient.
+template <int TY>
+struct BackPixels {
+    f32x2 T[TY], RG[TY], G[TY][3];
+    f32x2 ncol, nrow[TY];
+
+    // The sums of one Gaussian over the lane's pixels: gradients of its conic
+    // (xx, xy, yy) and log2 opacity, centre (x, y), then colour (r, g | b).
+    // T goes from behind the Gaussian to before it, RG from behind it to
+    // composited with it.
+    __device__ __forceinline__ void step(const PairRecord& q, float* v8, float& blue)
+    {
+        const f32x2 minus1 = pair(-1.0f, -1.0f), one = pair(1.0f, 1.0f);
+        // the forward's per-pixel power, term for term (Pixels::blend)
+        const f32x2 dx = add2(q.x, ncol);
+        const f32x2 xw = fma2(mul2(q.a, dx), dx, q.w);
+        const f32x2 xb = mul2(q.b, dx);
+        // dx depends on the column only and dy on the row only, so the conic
+        // and centre gradients need three sums per column over this lane's
+        // rows: of dp, dp dy and dp dy^2
+        const f32x2 zero = pair(0.0f, 0.0f);
+        f32x2 s0 = zero, s1 = zero, s2 = zero, gr = zero, gg = zero, gb = zero;
+#pragma unroll
+        for (int i = 0; i < TY; i++) {
+            const f32x2 dy = add2(q.y, nrow[i]);
+            const f32x2 alpha = ex2_2(fma2(xb, dy, fma2(mul2(q.c, dy), dy, xw)));
+            float m0, m1, t0, t1, a0, a1;
+            split(fma2(alpha, minus1, one), m0, m1);  // 1 - alpha
+            split(T[i], t0, t1);
+            split(mul2(T[i], pair(rcp_approx_ftz(m0), rcp_approx_ftz(m1))), a0, a1);
+            const f32x2 Tb = pair(m0 > 0.0f ? fminf(1.0f, a0) : t0, m1 > 0.0f ? fminf(1.0f, a1) : t1);
+            T[i] = Tb;
+            const f32x2 w = mul2(alpha, Tb);
+            // (c - R) . G
+            const f32x2 d = fma2(RG[i], minus1, fma2(q.bl, G[i][2], fma2(q.g, G[i][1], mul2(q.r, G[i][0]))));
+            RG[i] = fma2(alpha, d, RG[i]);  // (alpha c + (1 - alpha) R) . G
+            gr = fma2(w, G[i][0], gr);
+            gg = fma2(w, G[i][1], gg);
+            gb = fma2(w, G[i][2], gb);
+            // d power of this pixel, without its factor ln 2 (applied to the totals)
+            const f32x2 dp = mul2(d, w);
+            const f32x2 dpy = mul2(dp, dy);
+            s0 = add2(s0, dp);
+            s1 = add2(s1, dpy);
+            s2 = fma2(dpy, dy, s2);
+        }
+        // d power / d (conic x, y, z, w) = (dx^2, dx dy, dy^2, 1);
+        // d power / d centre = (2 a dx + b dy, 2 c dy + b dx)
+        const f32x2 x0 = mul2(dx, s0);
+        const f32x2 xx = mul2(dx, x0), xy = mul2(dx, s1);
+        const float a = lo_of(q.a), b = lo_of(q.b), c = lo_of(q.c);
+        const float sx = lo_of(x0) + hi_of(x0), sy = lo_of(s1) + hi_of(s1);
+        v8[0] = lo_of(xx) + hi_of(xx);
+        v8[1] = lo_of(xy) + hi_of(xy);
+        v8[2] = lo_of(s2) + hi_of(s2);
+        v8[3] = lo_of(s0) + hi_of(s0);
+        v8[4] = fmaf(2.0f * a, sx, b * sy);
+        v8[5] = fmaf(2.0f * c, sy, b * sx);
+        v8[6] = lo_of(gr) + hi_of(gr);
+        v8[7] = lo_of(gg) + hi_of(gg);
+        blue = lo_of(gb) + hi_of(gb);
+    }
+};
 
 // Reverse traversal of each tile's blended Gaussians.  With T_after the
 // transmittance behind Gaussian i and alpha_i recomputed bit for bit,
@@ -731,160 +1150,104 @@ __device__ __forceinline__ float warp_sum8_spread(const float (&v)[8], unsigned 
 //   dL/dc_i     = sum_px alpha_i T_before dL/dC
 //   dL/dalpha_i = T_before (c_i - R) . dL/dC,   d alpha/d power = alpha ln 2
 // and the power's derivatives give the conic/opacity and centre gradients.
-// The 9 per-Gaussian sums are reduced over the warp (eight of them spread
-// over the lanes, warp_sum8_spread) and added atomically: by three lanes as
-// 16-byte adds into the Gaussian's 12-float record (grad_rec), or by nine
-// lanes into the three arrays.
-// Five CTAs of 128 threads per SM (96 registers, a few bytes spilled): the
-// kernel is bound by instruction issue with few warps resident, and the
-// fifth CTA measured 1-2% faster per training step (8 views of 1 M Gaussians
-// at 1280x720) than four at 120 registers.
-__global__ __launch_bounds__(kTrainWarps * 32, 5) void k_render_backward(const TrainRenderArgs a)
+//
+// The kernel is bound by the FMA pipe and instruction issue: the pixels go in
+// column pairs (see Pixels), and the 9 sums of two Gaussians at a time are
+// reduced over the warp together, sixteen of them spread over the lanes
+// (warp_sum16_spread), which leaves each lane pair with one total to add:
+// eight consecutive floats of each Gaussian's 12-float record (grad_rec), or
+// entries of the three arrays.
+template <bool QUAD, int SPLIT>
+__global__ __launch_bounds__(kTrainWarps * 32, 4) void k_render_backward(const TrainRenderArgs a)
 {
-    __shared__ TrainBatch sb[kTrainWarps];
+    static_assert(SPLIT == 1 || SPLIT == kTrainWarps, "a tile per warp, or per CTA");
+    constexpr int TY = 4 / SPLIT;
+    __shared__ BlendRing<SPLIT == 1> rings[kTrainWarps];
     const unsigned lane = threadIdx.x & 31u;
     const int warp = threadIdx.x >> 5;
-    TrainBatch& B = sb[warp];
-    const int gx = (a.W + 15) / 16, gy = (a.H + 15) / 16, tiles = gx * gy;
-    const int tile = blockIdx.x * kTrainWarps + warp;
-    if (tile >= tiles * max(a.n_views, 1)) return;
-    const int view = tile / tiles, lt = tile - view * tiles;
-    const size_t pix0 = (size_t)view * a.W * a.H;
-    const int n = (int)max(0LL, min((long long)*a.d_num, a.cap));
-    const int tx = lt % gx, ty = lt / gx;
-    const int ox = tx * 16, oy = ty * 16;
-    const int cb = (int)(lane & 7u) * 2, rb = (int)(lane >> 3) * 4;
-    uint32_t qbit;
-    const int2 rg = __ldg(a.ranges + train_list(a, view, tile, tx, ty, gx, gy, qbit));
-    const int start = min(max(rg.x, 0), n);
-    const int count = min(max(__ldg(a.n_tile + tile), 0), max(0, min(max(rg.y, start), n) - start));
-    float T[4][2], R[4][2][3], G[4][2][3];
+    BlendRing<SPLIT == 1>& R = rings[warp];
+    TrainTile<QUAD, SPLIT> t;
+    if (!t.open(a, lane, warp)) return;
+    const int count = min(max(__ldg(a.n_tile + t.tile), 0), t.stop - t.start);
+    BackPixels<TY> px;
+    px.ncol = pair(-(float)(t.ox + t.cb), -(float)(t.ox + t.cb + 1));
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+    for (int i = 0; i < TY; i++) {
+        float T[2], rg[2], g[2][3];
+        const int y = t.oy + t.rb + i;
+        px.nrow[i] = pair(-(float)y, -(float)y);
 #pragma unroll
         for (int j = 0; j < 2; j++) {
-            const int px = ox + cb + j, py = oy + rb + i;
-            const bool in = px < a.W && py < a.H;
-            const size_t o = in ? pix0 + (size_t)py * a.W + px : 0;
-            const float t = in ? __ldg(a.T_final + o) : 1.0f;
-            T[i][j] = t;
+            const int x = t.ox + t.cb + j;
+            const bool in = x < a.W && y < a.H;
+            const size_t o = in ? t.pix0 + (size_t)y * a.W + x : 0;
+            T[j] = in ? __ldg(a.T_final + o) : 1.0f;
 #pragma unroll
-            for (int ch = 0; ch < 3; ch++) {
-                R[i][j][ch] = t < 0.0001f ? 0.0f : a.bg[ch];
-                G[i][j][ch] = in ? __ldg(a.grad_image + 3 * o + ch) : 0.0f;
-            }
+            for (int ch = 0; ch < 3; ch++) g[j][ch] = in ? __ldg(a.grad_image + 3 * o + ch) : 0.0f;
+            rg[j] = T[j] < 0.0001f ? 0.0f : a.bg[0] * g[j][0] + a.bg[1] * g[j][1] + a.bg[2] * g[j][2];
         }
-    const float LN2 = 0.69314718055994531f;
-    for (int hi = start + count; hi > start; hi -= 32) {
-        const int lo = max(start, hi - 32), cnt = hi - lo;
+        px.T[i] = pair(T[0], T[1]);
+        px.RG[i] = pair(rg[0], rg[1]);
+#pragma unroll
+        for (int ch = 0; ch < 3; ch++) px.G[i][ch] = pair(g[0][ch], g[1][ch]);
+    }
+    // where a lane's total goes: lane l has value (l >> 1) & 7 of the first
+    // (l < 16) or second Gaussian; lanes 0 and 16 add the blue sums as well
+    const int slot = (int)(lane >> 1) & 7;
+    const bool first = lane < 16u;
+    const float unit = slot < 6 ? 0.69314718055994531f : 1.0f;  // the ln 2 of d power
+    const Features f{a.xy, a.con, a.rgbd, a.vals, (uint32_t)a.P};
+    bool bad = false;
+    Feed<QUAD, true, SPLIT == 1> feed;
+    feed.open(f, t.start, t.start + count, t.qbit, lane);
+    feed.fetch(R, f, lane, bad);
+    while (feed.n > 0) {
+        const int n = feed.n;
         __syncwarp();
-        if ((int)lane < cnt) {
-            uint32_t g;
-            const bool mine = train_entry(a, __ldg(a.vals + lo + lane), qbit, g);
-            const bool ok = mine && g < (uint32_t)a.P;
-            B.use[lane] = mine ? 1u : 0u;
-            B.gid[lane] = ok ? g : 0xFFFFFFFFu;
-            B.xy[lane] = ok ? __ldg(a.xy + g) : make_float2(0.f, 0.f);
-            B.con[lane] = ok ? __ldg(a.con + g) : make_float4(0.f, 0.f, 0.f, -1e30f);
-            B.rgb[lane] = ok ? __ldg(a.rgbd + g) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
+        feed.store(R, lane);
         __syncwarp();
-        for (int k = cnt - 1; k >= 0; k--) {
-            if (!B.use[k]) continue;  // another tile of the quad
-            const float2 xy = B.xy[k];
-            const float4 co = B.con[k];
-            const float4 c4 = B.rgb[k];
-            const float col[3] = {c4.x, c4.y, c4.z};
-            float gc[3] = {0.f, 0.f, 0.f};
-            // dx depends on the column only and dy on the row only, so the
-            // conic and centre gradients need three sums over this lane's
-            // pixels of dp (per column, per row) and of dp * dx (per row)
-            float s_col[2] = {0.f, 0.f}, g_w = 0.f, g_yy = 0.f, g_xy = 0.f, sy = 0.f, sx = 0.f;
-            // the forward's per-pixel power, term for term (shade<>, SHADER 0)
-            float xs[2], xc[2], dxs[2];
+        feed.fetch(R, f, lane, bad);
+        for (int k = 0; k < n; k += 2) {
+            float v[16], b0, b1 = 0.0f;
+            px.step(read_record(R, k), v, b0);
+            if (k + 1 < n) {
+                px.step(read_record(R, k + 1), v + 8, b1);
+            } else {
 #pragma unroll
-            for (int j = 0; j < 2; j++) {
-                const float dx = xy.x - (float)(ox + cb + j);
-                dxs[j] = dx;
-                xs[j] = co.x * dx * dx;
-                xc[j] = co.y * dx;
+                for (int q = 8; q < 16; q++) v[q] = 0.0f;
             }
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const float dy = xy.y - (float)(oy + rb + i);
-                const float ys = co.z * dy * dy;
-                float r = 0.f, q = 0.f;
-#pragma unroll
-                for (int j = 0; j < 2; j++) {
-                    const float power = fmaf(xc[j], dy, co.w + xs[j] + ys);
-                    const float alpha = ex2_approx_ftz(power);
-                    const float one_m = 1.0f - alpha;
-                    const float Tb = one_m > 0.0f ? fminf(1.0f, T[i][j] / one_m) : T[i][j];
-                    const float w = alpha * Tb;
-                    float dalpha = 0.0f;
-#pragma unroll
-                    for (int ch = 0; ch < 3; ch++) {
-                        const float d = col[ch] - R[i][j][ch];
-                        gc[ch] = fmaf(w, G[i][j][ch], gc[ch]);
-                        dalpha = fmaf(d, G[i][j][ch], dalpha);
-                        R[i][j][ch] = fmaf(alpha, d, R[i][j][ch]);  // alpha c + (1 - alpha) R
-                    }
-                    T[i][j] = Tb;
-                    // d power of this pixel, without its factor ln 2 (applied to the totals)
-                    const float dp = dalpha * w;
-                    r += dp;
-                    q = fmaf(dp, dxs[j], q);
-                    s_col[j] += dp;
+            const float t16 = unit * warp_sum16_spread(v, lane);
+            const float t2 = warp_sum2_spread(b0, b1, lane);
+            const uint32_t gid = first ? R.gid[k] : (k + 1 < n ? R.gid[k + 1] : 0xFFFFFFFFu);
+            if (gid != 0xFFFFFFFFu) {
+                if (a.grad_rec) {
+                    float* rec = a.grad_rec + 12 * (size_t)gid;
+                    if ((lane & 1u) == 0u) atomicAdd(rec + slot, t16);
+                    if ((lane & 15u) == 1u) atomicAdd(rec + 8, t2);
+                } else {
+                    float* dst = slot < 4   ? a.grad_con + 4 * (size_t)gid + slot
+                                 : slot < 6 ? a.grad_xy + 2 * (size_t)gid + (slot - 4)
+                                            : a.grad_rgb + 3 * (size_t)gid + (slot - 6);
+                    if ((lane & 1u) == 0u) atomicAdd(dst, t16);
+                    if ((lane & 15u) == 1u) atomicAdd(a.grad_rgb + 3 * (size_t)gid + 2, t2);
                 }
-                g_w += r;
-                g_yy = fmaf(dy * dy, r, g_yy);
-                g_xy = fmaf(dy, q, g_xy);
-                sy = fmaf(dy, r, sy);
-                sx += q;
-            }
-            // d power / d (conic x, y, z, w) = (dx^2, dx dy, dy^2, 1);
-            // d power / d centre = (2 co.x dx + co.y dy, 2 co.z dy + co.y dx)
-            float v[8];
-            v[0] = LN2 * fmaf(dxs[0] * dxs[0], s_col[0], dxs[1] * dxs[1] * s_col[1]);
-            v[1] = LN2 * g_xy;
-            v[2] = LN2 * g_yy;
-            v[3] = LN2 * g_w;
-            v[4] = LN2 * fmaf(2.0f * co.x, sx, co.y * sy);
-            v[5] = LN2 * fmaf(2.0f * co.z, sy, co.y * sx);
-            v[6] = gc[0];
-            v[7] = gc[1];
-            const float t8 = warp_sum8_spread(v, lane);
-            const float t9 = warp_sum(gc[2]);
-            // lanes 0, 4, .., 28 hold the totals of v[lane / 4]; every lane the ninth
-            const uint32_t gid = B.gid[k];
-            if (a.grad_rec) {
-                // lane L < 3 adds slots 4L .. 4L + 3 of the Gaussian's record
-                float r4[4];
-#pragma unroll
-                for (int c = 0; c < 4; c++) {
-                    const int slot = 4 * (int)(lane & 3u) + c;
-                    const float x = __shfl_sync(GSR_FULL_MASK, t8, slot < 8 ? 4 * slot : 0);
-                    r4[c] = slot < 8 ? x : (slot == 8 ? t9 : 0.0f);
-                }
-                if (lane < 3u && gid != 0xFFFFFFFFu)
-                    atomicAdd(reinterpret_cast<float4*>(a.grad_rec + 12 * (size_t)gid) + lane,
-                              make_float4(r4[0], r4[1], r4[2], r4[3]));
-            } else if (gid != 0xFFFFFFFFu) {
-                float* dst = nullptr;
-                float val = t8;
-                if ((lane & 3u) == 0u) {
-                    const int q8 = (int)(lane >> 2);
-                    dst = q8 < 4 ? a.grad_con + 4 * (size_t)gid + q8
-                        : q8 < 6 ? a.grad_xy + 2 * (size_t)gid + (q8 - 4)
-                                 : a.grad_rgb + 3 * (size_t)gid + (q8 - 6);
-                } else if (lane == 1u) {
-                    dst = a.grad_rgb + 3 * (size_t)gid + 2;
-                    val = t9;
-                }
-                if (dst) atomicAdd(dst, val);
             }
         }
     }
+}
+
+template <bool QUAD>
+cudaError_t launch_train(const TrainRenderArgs& a, bool backward, int tiles, cudaStream_t stream)
+{
+    const dim3 block(kTrainWarps * 32);
+    if (backward) {
+        if (split_tiles(tiles)) k_render_backward<QUAD, kTrainWarps><<<tiles, block, 0, stream>>>(a);
+        else k_render_backward<QUAD, 1><<<div_up(tiles, kTrainWarps), block, 0, stream>>>(a);
+    } else {
+        if (split_tiles(tiles)) k_render_train<QUAD, kTrainWarps><<<tiles, block, 0, stream>>>(a);
+        else k_render_train<QUAD, 1><<<div_up(tiles, kTrainWarps), block, 0, stream>>>(a);
+    }
+    return cudaGetLastError();
 }
 
 }  // namespace
@@ -894,10 +1257,8 @@ cudaError_t launch_render_train(const TrainRenderArgs& a, bool backward, cudaStr
     const long long tiles = (long long)((a.W + 15) / 16) * ((a.H + 15) / 16) * max(a.n_views, 1);
     if (tiles <= 0) return cudaSuccess;
     if (tiles > INT32_MAX - kTrainWarps) return cudaErrorInvalidValue;
-    const int grid = div_up((int)tiles, kTrainWarps);
-    if (backward) k_render_backward<<<grid, kTrainWarps * 32, 0, stream>>>(a);
-    else k_render_train<<<grid, kTrainWarps * 32, 0, stream>>>(a);
-    return cudaGetLastError();
+    return a.quad ? launch_train<true>(a, backward, (int)tiles, stream)
+                  : launch_train<false>(a, backward, (int)tiles, stream);
 }
 
 cudaError_t launch_render(const RenderArgs& a, cudaStream_t stream)
