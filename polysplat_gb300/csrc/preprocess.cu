@@ -13,6 +13,7 @@
 
 #include "gsr_internal.h"
 #include "ndc.h"
+#include "tile_test.h"
 
 namespace gsr {
 namespace {
@@ -170,56 +171,6 @@ __device__ __forceinline__ V3 sh_color(int idx, V3 p, V3 cam, const void* shs)
     result.y = fmaxf(result.y, 0.0f);
     result.z = fmaxf(result.z, 0.0f);
     return result;
-}
-
-// Ellipse / tile-box tests (preprocess.cu:257-311).
-//
-// The arithmetic is written with explicit rounding intrinsics, one per
-// operation of the reference's expressions, fused where those expressions
-// contract under fast math (x * y + z -> fma(x, y, z); x * x - y * z ->
-// fma(x, x, -(y * z))).  Left to the compiler, the fusion of the same
-// expression can differ between the kernels that inline it, and a tile on
-// the ellipse's edge then passes in one kernel and fails in another: the
-// depth-first pipeline counts a Gaussian's tiles in one kernel and emits
-// them in another, so the two must agree bit for bit.
-__device__ __forceinline__ bool seg_hits_ellipse(float a, float b, float c, float d, float l, float r)
-{
-    const float two_a = __fmul_rn(2.0f, a);
-    const float delta = __fmaf_rn(b, b, -__fmul_rn(__fmul_rn(4.0f, a), c));
-    const float t1 = __fmaf_rn(__fsub_rn(l, d), two_a, b);
-    const float t2 = __fmaf_rn(__fsub_rn(r, d), two_a, b);
-    return delta >= 0.0f && (t1 <= 0.0f || __fmul_rn(t1, t1) <= delta) &&
-           (t2 >= 0.0f || __fmul_rn(t2, t2) <= delta);
-}
-
-__device__ __forceinline__ bool box_hits_ellipse(int2 pmin, int2 pmax, float2 ctr, float3 con, float power)
-{
-    float a, b, c, dx, dy;
-    const float w = __fmul_rn(2.0f, power);
-    if (ctr.x * 2.0f < (float)(pmin.x + pmax.x)) dx = __fsub_rn(ctr.x, (float)pmin.x);
-    else dx = __fsub_rn(ctr.x, (float)pmax.x);
-    a = con.z;
-    b = __fmul_rn(__fmul_rn(-2.0f, con.y), dx);
-    c = __fmaf_rn(__fmul_rn(con.x, dx), dx, -w);
-    if (seg_hits_ellipse(a, b, c, ctr.y, (float)pmin.y, (float)pmax.y)) return true;
-    if (ctr.y * 2.0f < (float)(pmin.y + pmax.y)) dy = __fsub_rn(ctr.y, (float)pmin.y);
-    else dy = __fsub_rn(ctr.y, (float)pmax.y);
-    a = con.x;
-    b = __fmul_rn(__fmul_rn(-2.0f, con.y), dy);
-    c = __fmaf_rn(__fmul_rn(con.z, dy), dy, -w);
-    return seg_hits_ellipse(a, b, c, ctr.x, (float)pmin.x, (float)pmax.x);
-}
-
-__device__ __forceinline__ bool box_has_centre(int2 pmin, int2 pmax, float2 c)
-{
-    return c.x >= pmin.x && c.x <= pmax.x && c.y >= pmin.y && c.y <= pmax.y;
-}
-
-__device__ __forceinline__ bool tile_hit(int x, int y, int bx, int by, float2 ctr, float3 con, float power)
-{
-    int2 pmin = {x * bx, y * by};
-    int2 pmax = {pmin.x + bx - 1, pmin.y + by - 1};
-    return box_has_centre(pmin, pmax, ctr) || (power > 0.0f && box_hits_ellipse(pmin, pmax, ctr, con, power));
 }
 
 // Tiles of quad (qx, qy) that lie in the Gaussian's rectangle [rmin, rmax)
@@ -681,81 +632,10 @@ __global__ __launch_bounds__(kThreads, VIEWS ? 6 : 5) void k_preprocess(const __
 }
 
 // ---------------------------------------------------------------------------
-// Queued Gaussians with large tile rectangles (k_emit_massive).  For a
-// well-conditioned ellipse only the tiles of each tile row that lie within a
-// margin of the ellipse's x-extent over that row get the exact test; tiles
-// farther out cannot pass it.
+// Queued Gaussians with large tile rectangles (k_emit_massive).  Only the
+// candidate tiles of each tile row (band_columns, tile_test.h) get the exact
+// test; tiles farther out cannot pass it.
 constexpr int kMaxBandRows = 1024;  // tile rows of a CTA-swept rectangle that get candidate bands
-
-// Ellipse A dx^2 + 2B dx dy + C dy^2 <= w (w = 2 power) in float.
-//
-// Which tiles can pass the exact test.  In exact arithmetic the test
-// (box_has_centre / box_hits_ellipse) only accepts tiles whose box meets the
-// ellipse.  In float it can also accept a tile just outside.  On a box edge
-// at offset dx from the centre, the test accepts a point of the edge where
-// the computed quadratic is <= 0; the computed discriminant errs by a few
-// 2^-24 of its terms' size, (B^2 + AC) dx^2 + C w, so every accepted point
-// satisfies Q <= w (1 + k u (1 + kappa)), with u = 2^-24, kappa = 2AC / det
-// >= (B^2 + AC) / det and k about 10 (the same holds for the horizontal
-// edge).  The candidate bands are therefore the exact row extents of the
-// ellipse inflated to w (1 + tau), tau = 64 u (1 + kappa), plus half a pixel
-// and a relative 1e-5 for the rounding of the band arithmetic itself and of
-// pixel coordinates.
-//
-// det = AC - B^2 is formed with a single rounding (Kahan's fused difference
-// of products), and the half-width at height dy as sqrt(det (dymax - dy)
-// (dymax + dy)) / A, which does not cancel near the top and bottom, so every
-// extent carries a few ulp of relative error.  Ill-conditioned ellipses
-// (det <= 1e-6 AC) and non-finite values get every tile of the rectangle
-// tested.
-struct Band {
-    float B, inv_a, det, dymax, dxmax, dyr, cx, cy, m;
-    bool ok;
-};
-
-__device__ __forceinline__ Band make_band(float3 q, float power, float2 c)
-{
-    Band b;
-    const float A = q.x, B = q.y, C = q.z, w = 2.0f * power;
-    const float bb = B * B;
-    const float det = fmaf(A, C, -bb) + fmaf(-B, B, bb);
-    const float kappa = 2.0f * (A * C) / det;
-    const float wb = w * (1.0f + 64.0f * 5.9604645e-8f * (1.0f + kappa));  // inflated for the test's rounding
-    b.B = B;
-    b.inv_a = 1.0f / A;
-    b.det = det;
-    b.dymax = sqrtf(wb * A / det);
-    b.dxmax = sqrtf(wb * C / det);
-    b.dyr = -B * sqrtf(wb / (C * det));  // dy where the ellipse reaches its largest x
-    b.cx = c.x;
-    b.cy = c.y;
-    b.m = 0.5f + 1e-5f * fmaxf(b.dxmax, b.dymax);
-    b.ok = A > 0.0f && C > 0.0f && w > 0.0f && det > 1e-6f * (A * C) && b.dymax < 1e6f && b.dxmax < 1e6f &&
-           fabsf(b.dyr) < 1e6f && fabsf(c.x) < 1e7f && fabsf(c.y) < 1e7f;
-    return b;
-}
-
-// Candidate tile columns [c_lo, c_hi] of tile row `ty`: the ellipse's x-extent
-// over the row's pixel band, widened by m pixels on every side.  False when
-// the widened band misses the ellipse.
-__device__ __forceinline__ bool band_columns(const Band& e, int ty, int by, int bx, int x_lo, int x_hi, int& c_lo,
-                                             int& c_hi)
-{
-    const float p = fmaxf((float)(ty * by) - e.m - e.cy, -e.dymax);
-    const float q = fminf((float)(ty * by + by - 1) + e.m - e.cy, e.dymax);
-    if (!(p <= q)) return false;
-    auto half = [&](float dy) {
-        return sqrtf(e.det * fmaxf(0.0f, e.dymax - dy) * fmaxf(0.0f, e.dymax + dy)) * e.inv_a;
-    };
-    const float hp = half(p), hq = half(q);
-    const float mp = -e.B * p * e.inv_a, mq = -e.B * q * e.inv_a;  // centre line of the ellipse at p, q
-    const float xr = (e.dyr >= p && e.dyr <= q) ? e.dxmax : fmaxf(mp + hp, mq + hq);
-    const float xl = (-e.dyr >= p && -e.dyr <= q) ? -e.dxmax : fminf(mp - hp, mq - hq);
-    const float lo = floorf((e.cx + xl - e.m) / (float)bx), hi = floorf((e.cx + xr + e.m) / (float)bx);
-    c_lo = (int)fmaxf((float)x_lo, lo);
-    c_hi = (int)fminf((float)(x_hi - 1), hi);
-    return c_lo <= c_hi;
-}
 
 // The CTA's flattened sweep of `rows` rows of candidate columns (s_band[r] =
 // [lo, hi], empty when hi < lo): a block-wide prefix of the rows' counts
@@ -826,8 +706,8 @@ __device__ __forceinline__ void sweep_cta(const MassiveEntry& me, const Preproce
     const int x_lo = me.rect.x & 0xFFFF, x_hi = me.rect.y, y_lo = me.rect.z, y_hi = me.rect.w;
     const int w = x_hi - x_lo;
     // every thread forms the same band from the same inputs: a uniform branch
-    const Band eb = make_band(q, pw, c);
-    if (eb.ok && (y_hi - y_lo) <= kMaxBandRows) {
+    const Band eb = make_band(q, pw, c, x_lo, x_hi, a.bx);
+    if (eb.kind != kBandFull && (y_hi - y_lo) <= kMaxBandRows) {
         for (int r = threadIdx.x; r < y_hi - y_lo; r += kThreads) {
             int clo = 0, chi = -1;
             if (!band_columns(eb, y_lo + r, a.by, a.bx, x_lo, x_hi, clo, chi)) {
@@ -875,8 +755,8 @@ __device__ __forceinline__ void sweep_warp(const MassiveEntry& me, const Preproc
     const float pw = me.ctr_power_depth.z;
     const float3 q = {me.conic_gid.x, me.conic_gid.y, me.conic_gid.z};
     const int x_lo = me.rect.x & 0xFFFF, x_hi = me.rect.y, y_lo = me.rect.z, y_hi = me.rect.w;
-    const Band eb = make_band(q, pw, c);
-    if (eb.ok) {
+    const Band eb = make_band(q, pw, c, x_lo, x_hi, a.bx);
+    if (eb.kind != kBandFull) {
         for (int r0 = y_lo; r0 < y_hi; r0 += 32) {
             const int y = r0 + (int)lane;
             int clo = 0, n = 0;
@@ -961,8 +841,8 @@ __device__ __forceinline__ void sweep_cta_quad(const MassiveEntry& me, const Pre
     const int x_lo = me.rect.x & 0xFFFF, x_hi = me.rect.y, y_lo = me.rect.z, y_hi = me.rect.w;
     const int2 rmin = make_int2(x_lo, y_lo), rmax = make_int2(x_hi, y_hi);
     const int qx_lo = quad_lo(x_lo), qx_hi = quad_hi(x_hi), qy_lo = quad_lo(y_lo), qy_hi = quad_hi(y_hi);
-    const Band eb = make_band(q, pw, c);
-    if (eb.ok && (qy_hi - qy_lo) <= kMaxBandRows) {
+    const Band eb = make_band(q, pw, c, x_lo, x_hi, a.bx);
+    if (eb.kind != kBandFull && (qy_hi - qy_lo) <= kMaxBandRows) {
         for (int r = threadIdx.x; r < qy_hi - qy_lo; r += kThreads) {
             int lo = 0, hi = -1;
             if (!band_quads(eb, qy_lo + r, a.by, a.bx, x_lo, x_hi, y_lo, y_hi, lo, hi)) {
@@ -1011,8 +891,8 @@ __device__ __forceinline__ void sweep_warp_quad(const MassiveEntry& me, const Pr
     const int x_lo = me.rect.x & 0xFFFF, x_hi = me.rect.y, y_lo = me.rect.z, y_hi = me.rect.w;
     const int2 rmin = make_int2(x_lo, y_lo), rmax = make_int2(x_hi, y_hi);
     const int qx_lo = quad_lo(x_lo), qx_hi = quad_hi(x_hi), qy_lo = quad_lo(y_lo), qy_hi = quad_hi(y_hi);
-    const Band eb = make_band(q, pw, c);
-    if (eb.ok) {
+    const Band eb = make_band(q, pw, c, x_lo, x_hi, a.bx);
+    if (eb.kind != kBandFull) {
         for (int r0 = qy_lo; r0 < qy_hi; r0 += 32) {
             const int qy = r0 + (int)lane;
             int clo = 0, n = 0;
