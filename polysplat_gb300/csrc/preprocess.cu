@@ -635,127 +635,16 @@ __global__ __launch_bounds__(kThreads, VIEWS ? 6 : 5) void k_preprocess(const __
 // Queued Gaussians with large tile rectangles (k_emit_massive).  Only the
 // candidate tiles of each tile row (band_columns, tile_test.h) get the exact
 // test; tiles farther out cannot pass it.
-constexpr int kMaxBandRows = 1024;  // tile rows of a CTA-swept rectangle that get candidate bands
-
-// The CTA's flattened sweep of `rows` rows of candidate columns (s_band[r] =
-// [lo, hi], empty when hi < lo): a block-wide prefix of the rows' counts
-// into s_pref, then each warp takes 32 consecutive candidates at a time, so
-// a narrow row shares a step with its neighbours instead of taking a step of
-// its own.  step(valid, x, r) is called by all lanes of a warp together.
-template <typename F>
-__device__ __forceinline__ void sweep_flat_cta(int rows, const short2* s_band, int* s_pref, int* s_wsum,
-                                               unsigned lane, int warp, F&& step)
-{
-    constexpr int kPer = kMaxBandRows / kThreads;  // rows per thread in the scan
-    const int r0 = (int)threadIdx.x * kPer;
-    int cnt[kPer];
-    int local = 0;
-#pragma unroll
-    for (int k = 0; k < kPer; k++) {
-        const int r = r0 + k;
-        cnt[k] = r < rows ? max(0, (int)s_band[r].y - (int)s_band[r].x + 1) : 0;
-        local += cnt[k];
-    }
-    int incl = local;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const int t = __shfl_up_sync(GSR_FULL_MASK, incl, d);
-        if ((int)lane >= d) incl += t;
-    }
-    if (lane == 31) s_wsum[warp] = incl;
-    __syncthreads();
-    int run = incl - local, total = 0;
-#pragma unroll
-    for (int w = 0; w < kWarps; w++) {
-        if (w < warp) run += s_wsum[w];
-        total += s_wsum[w];
-    }
-#pragma unroll
-    for (int k = 0; k < kPer; k++) {
-        run += cnt[k];
-        if (r0 + k < rows) s_pref[r0 + k] = run;  // inclusive prefix of the rows' counts
-    }
-    __syncthreads();
-    for (int base = warp * 32; base < total; base += kWarps * 32) {
-        const int task = base + (int)lane;
-        // owner row: the first row whose inclusive prefix exceeds the task
-        int lo = 0, hi = rows - 1;
-#pragma unroll
-        for (int it = 0; it < 10; it++) {  // 2^10 = kMaxBandRows
-            if (lo < hi) {
-                const int mid = (lo + hi) >> 1;
-                if (s_pref[mid] > task) hi = mid;
-                else lo = mid + 1;
-            }
-        }
-        const short2 b = s_band[lo];
-        const int x = (int)b.x + task - (s_pref[lo] - ((int)b.y - (int)b.x + 1));
-        step(task < total, x, lo);
-    }
-}
-
-// Sweep the tiles of one huge queued Gaussian with the whole CTA; on_step(v,
-// x, y) is called by every lane of a warp together, v = the tile's exact test.
-template <typename F>
-__device__ __forceinline__ void sweep_cta(const MassiveEntry& me, const PreprocessParams& a, short2* s_band,
-                                          int* s_pref, int* s_wsum, unsigned lane, int warp, F&& on_step)
-{
-    const float2 c = {me.ctr_power_depth.x, me.ctr_power_depth.y};
-    const float pw = me.ctr_power_depth.z;
-    const float3 q = {me.conic_gid.x, me.conic_gid.y, me.conic_gid.z};
-    const int x_lo = me.rect.x & 0xFFFF, x_hi = me.rect.y, y_lo = me.rect.z, y_hi = me.rect.w;
-    const int w = x_hi - x_lo;
-    // every thread forms the same band from the same inputs: a uniform branch
-    const Band eb = make_band(q, pw, c, x_lo, x_hi, a.bx);
-    if (eb.kind != kBandFull && (y_hi - y_lo) <= kMaxBandRows) {
-        for (int r = threadIdx.x; r < y_hi - y_lo; r += kThreads) {
-            int clo = 0, chi = -1;
-            if (!band_columns(eb, y_lo + r, a.by, a.bx, x_lo, x_hi, clo, chi)) {
-                clo = 0;
-                chi = -1;
-            }
-            s_band[r] = make_short2((short)clo, (short)chi);
-        }
-        __syncthreads();
-        sweep_flat_cta(y_hi - y_lo, s_band, s_pref, s_wsum, lane, warp, [&](bool valid, int x, int r) {
-            on_step(valid && tile_hit(x, y_lo + r, a.bx, a.by, c, q, pw), x, y_lo + r);
-        });
-        __syncthreads();  // s_band, s_pref and on_step's shared counters are reused by the next entry
-        return;
-    }
-    // Otherwise the CTA sweeps the rectangle in windows of (cols x rows)
-    // tiles, cols a power of two fitted to the rectangle's width, so narrow
-    // rectangles still fill the lanes and no per-tile integer division is
-    // needed.
-    int lg = 5;
-    while (lg > 0 && (1 << (lg - 1)) >= w) lg--;
-    const int cols = 1 << lg;              // columns per warp row
-    const int rows_w = 32 >> lg;           // rows per warp
-    const int rows_cta = rows_w * kWarps;  // rows per CTA step
-    const int lx = (int)lane & (cols - 1);
-    const int ly = warp * rows_w + ((int)lane >> lg);
-    for (int wy = y_lo; wy < y_hi; wy += rows_cta) {
-        const int y = wy + ly;
-        for (int wx = x_lo; wx < x_hi; wx += cols) {
-            const int x = wx + lx;
-            const bool v = y < y_hi && x < x_hi && tile_hit(x, y, a.bx, a.by, c, q, pw);
-            on_step(v, x, y);
-        }
-    }
-    __syncthreads();  // on_step's shared counters are reused by the next entry
-}
-
 // Sweep the tiles of one large queued Gaussian with one warp: the candidate
 // tiles of 32 rows at a time form one flattened task list, 32 tests per step.
 template <typename F>
-__device__ __forceinline__ void sweep_warp(const MassiveEntry& me, const PreprocessParams& a, unsigned lane,
-                                           F&& on_step)
+__device__ __forceinline__ void sweep_warp(const MassiveEntry& me, const Band& eb, const PreprocessParams& a,
+                                           unsigned lane, F&& on_step)
 {
     const float2 c = {me.ctr_power_depth.x, me.ctr_power_depth.y};
     const float pw = me.ctr_power_depth.z;
     const float3 q = {me.conic_gid.x, me.conic_gid.y, me.conic_gid.z};
     const int x_lo = me.rect.x & 0xFFFF, x_hi = me.rect.y, y_lo = me.rect.z, y_hi = me.rect.w;
-    const Band eb = make_band(q, pw, c, x_lo, x_hi, a.bx);
     if (eb.kind != kBandFull) {
         for (int r0 = y_lo; r0 < y_hi; r0 += 32) {
             const int y = r0 + (int)lane;
@@ -828,12 +717,11 @@ __device__ __forceinline__ bool band_quads(const Band& e, int qy, int by, int bx
     return hi >= lo;
 }
 
-// sweep_cta over quads: on_step(v, qx, qy, mask) with mask = quad_mask() of
-// the quad and v = mask != 0.  A tile that passes the exact test lies in its
-// row's band, so its quad lies in the quad row's band.
+// sweep_warp over quads.  A tile that passes the exact test lies in its row's
+// band, so its quad lies in the quad row's band.
 template <typename F>
-__device__ __forceinline__ void sweep_cta_quad(const MassiveEntry& me, const PreprocessParams& a, short2* s_band,
-                                               int* s_pref, int* s_wsum, unsigned lane, int warp, F&& on_step)
+__device__ __forceinline__ void sweep_warp_quad(const MassiveEntry& me, const Band& eb, const PreprocessParams& a,
+                                                unsigned lane, F&& on_step)
 {
     const float2 c = {me.ctr_power_depth.x, me.ctr_power_depth.y};
     const float pw = me.ctr_power_depth.z;
@@ -841,57 +729,6 @@ __device__ __forceinline__ void sweep_cta_quad(const MassiveEntry& me, const Pre
     const int x_lo = me.rect.x & 0xFFFF, x_hi = me.rect.y, y_lo = me.rect.z, y_hi = me.rect.w;
     const int2 rmin = make_int2(x_lo, y_lo), rmax = make_int2(x_hi, y_hi);
     const int qx_lo = quad_lo(x_lo), qx_hi = quad_hi(x_hi), qy_lo = quad_lo(y_lo), qy_hi = quad_hi(y_hi);
-    const Band eb = make_band(q, pw, c, x_lo, x_hi, a.bx);
-    if (eb.kind != kBandFull && (qy_hi - qy_lo) <= kMaxBandRows) {
-        for (int r = threadIdx.x; r < qy_hi - qy_lo; r += kThreads) {
-            int lo = 0, hi = -1;
-            if (!band_quads(eb, qy_lo + r, a.by, a.bx, x_lo, x_hi, y_lo, y_hi, lo, hi)) {
-                lo = 0;
-                hi = -1;
-            }
-            s_band[r] = make_short2((short)lo, (short)hi);
-        }
-        __syncthreads();
-        sweep_flat_cta(qy_hi - qy_lo, s_band, s_pref, s_wsum, lane, warp, [&](bool valid, int qx, int r) {
-            const uint32_t m = valid ? quad_mask(qx, qy_lo + r, rmin, rmax, a.bx, a.by, c, q, pw) : 0u;
-            on_step(m != 0u, qx, qy_lo + r, m);
-        });
-        __syncthreads();
-        return;
-    }
-    // windows of (cols x rows) quads, as sweep_cta does for tiles
-    const int w = qx_hi - qx_lo;
-    int lg = 5;
-    while (lg > 0 && (1 << (lg - 1)) >= w) lg--;
-    const int cols = 1 << lg;
-    const int rows_w = 32 >> lg;
-    const int rows_cta = rows_w * kWarps;
-    const int lx = (int)lane & (cols - 1);
-    const int ly = warp * rows_w + ((int)lane >> lg);
-    for (int wy = qy_lo; wy < qy_hi; wy += rows_cta) {
-        const int qy = wy + ly;
-        for (int wx = qx_lo; wx < qx_hi; wx += cols) {
-            const int qx = wx + lx;
-            const uint32_t m =
-                (qy < qy_hi && qx < qx_hi) ? quad_mask(qx, qy, rmin, rmax, a.bx, a.by, c, q, pw) : 0u;
-            on_step(m != 0u, qx, qy, m);
-        }
-    }
-    __syncthreads();
-}
-
-// sweep_warp over quads (see sweep_cta_quad).
-template <typename F>
-__device__ __forceinline__ void sweep_warp_quad(const MassiveEntry& me, const PreprocessParams& a, unsigned lane,
-                                                F&& on_step)
-{
-    const float2 c = {me.ctr_power_depth.x, me.ctr_power_depth.y};
-    const float pw = me.ctr_power_depth.z;
-    const float3 q = {me.conic_gid.x, me.conic_gid.y, me.conic_gid.z};
-    const int x_lo = me.rect.x & 0xFFFF, x_hi = me.rect.y, y_lo = me.rect.z, y_hi = me.rect.w;
-    const int2 rmin = make_int2(x_lo, y_lo), rmax = make_int2(x_hi, y_hi);
-    const int qx_lo = quad_lo(x_lo), qx_hi = quad_hi(x_hi), qy_lo = quad_lo(y_lo), qy_hi = quad_hi(y_hi);
-    const Band eb = make_band(q, pw, c, x_lo, x_hi, a.bx);
     if (eb.kind != kBandFull) {
         for (int r0 = qy_lo; r0 < qy_hi; r0 += 32) {
             const int qy = r0 + (int)lane;
@@ -943,6 +780,12 @@ __device__ __forceinline__ void sweep_warp_quad(const MassiveEntry& me, const Pr
     }
 }
 
+__device__ __forceinline__ Band entry_band(const MassiveEntry& me, int bx)
+{
+    return make_band(make_float3(me.conic_gid.x, me.conic_gid.y, me.conic_gid.z), me.ctr_power_depth.z,
+                     make_float2(me.ctr_power_depth.x, me.ctr_power_depth.y), me.rect.x & 0xFFFF, me.rect.y, bx);
+}
+
 // Where the depth-first pipeline's emission pass writes a queued Gaussian.
 struct DfEmit {
     const uint32_t* offsets;  // [V] first output position of the s-th Gaussian in depth order
@@ -954,27 +797,39 @@ struct DfEmit {
 
 enum : int { kMassiveEmit64 = 0, kMassiveCount = 1, kMassiveEmitDf = 2 };
 
-// Queued Gaussians: persistent CTAs first take the huge rectangles one at a
-// time with all 256 threads, then each warp takes large rectangles on its
-// own.  MODE: emit 64-bit keys, count the hit tiles (depth-first counting
-// pass), or write depth-first pairs at the Gaussian's offset.
+// Queued Gaussians.  Persistent CTAs first take huge rectangles, kWarps at a
+// time; after that each warp takes large rectangles on its own.  MODE: emit
+// 64-bit keys, count the hit tiles (depth-first counting pass), or write
+// depth-first pairs at the Gaussian's offset.
 //
-// QUAD: the sweeps run over quads (sweep_cta_quad / sweep_warp_quad); a quad
-// whose mask is not empty counts as one, and is written as (quad id, index |
-// mask << kQuadShift).
+// Huge rectangles hold from a few hundred to all of the frame's tiles as
+// candidates, so the CTA shares them out: each warp lists the candidate rows of
+// one rectangle (up to kSegRows at a time), then the CTA's warps take equal
+// shares of all the candidates, 32 to a step.  A step's rows follow each other
+// in the list, so one or-reduction of the rows' ends gives every lane its row.
+// With the candidate bands of tile_test.h: 87 us at 3 M Gaussians and 1080p (61 M
+// warp instructions for 6.6 M keys; bound by issue) and 613 us for 8 served
+// views.  A CTA per rectangle spent most of its time on the block-wide set-up
+// of a few hundred candidates, and a warp per rectangle on waiting for the
+// largest (203 against 113 us at 1080p with the same bands).  Four CTAs per SM
+// (64 registers, some spilled) against three: 87 / 103 and 613 / 651 us.
+//
+// QUAD: rows, candidates and keys are quads; a quad whose mask is not empty
+// counts as one, and is written as (quad id, index | mask << kQuadShift).
+constexpr int kSegRows = 128;
+
 template <int MODE, bool VIEWS, bool QUAD = false>
-__global__ __launch_bounds__(kThreads) void k_emit_massive(const __grid_constant__ PreprocessParams a, const DfEmit df)
+__global__ __launch_bounds__(kThreads, 4) void k_emit_massive(const __grid_constant__ PreprocessParams a, const DfEmit df)
 {
     __shared__ uint64_t s_keys[MODE == kMassiveEmit64 ? kWarps : 1][kStage];
     __shared__ uint32_t s_vals[MODE == kMassiveEmit64 ? kWarps : 1][kStage];
     __shared__ int s_fill[kWarps];
     __shared__ long long s_base[kWarps];
     __shared__ int s_entry;
-    __shared__ uint32_t s_pos;
-    __shared__ uint32_t s_wcnt[kWarps];
-    __shared__ short2 s_band[kMaxBandRows];
-    __shared__ int s_pref[kMaxBandRows];
-    __shared__ int s_wsum[kWarps];
+    __shared__ uint32_t s_pos[kWarps];             // per rectangle of the CTA: hits counted or written
+    __shared__ int s_start[kWarps][kSegRows + 1];  // candidates before each listed row
+    __shared__ uint32_t s_row[kWarps][kSegRows];   // the row's first candidate | row << 16
+    __shared__ int s_rows[kWarps];                 // rows listed
     const unsigned lane = threadIdx.x & 31u;
     const int warp = threadIdx.x >> 5;
     Stage st{s_keys[MODE == kMassiveEmit64 ? warp : 0], s_vals[MODE == kMassiveEmit64 ? warp : 0], 0};
@@ -982,86 +837,159 @@ __global__ __launch_bounds__(kThreads) void k_emit_massive(const __grid_constant
     uint32_t* head = a.mq.head + (MODE == kMassiveEmitDf ? 2 : 0);
     const int n_huge = (int)min(a.mq.count[0], (uint32_t)a.mq.huge_capacity);
     const int n_large = (int)min(a.mq.count[1], (uint32_t)(a.mq.capacity - a.mq.huge_capacity));
+    auto view_ok = [&](const MassiveEntry& me) { return !VIEWS || ((uint32_t)me.rect.x >> 16) < (uint32_t)a.n_views; };
 
-    // (1) huge rectangles, one CTA each
+    // (1) huge rectangles, kWarps of them to a CTA
     for (;;) {
-        if (threadIdx.x == 0) {
-            s_entry = (int)atomicAdd(&head[0], 1u);
-            s_pos = 0u;
+        if (threadIdx.x == 0) s_entry = (int)atomicAdd(&head[0], (uint32_t)kWarps);
+        if (lane == 0) s_pos[warp] = 0u;
+        __syncthreads();
+        const int e0 = s_entry;
+        if (e0 >= n_huge) break;
+        int row = 0, row_end = 0;  // of this warp's rectangle: next row (or quad row) to list
+        MassiveEntry mine;
+        Band eb;
+        if (e0 + warp < n_huge) {
+            mine = a.mq.entries[e0 + warp];
+            if (view_ok(mine)) {
+                eb = entry_band(mine, a.bx);
+                row = QUAD ? quad_lo(mine.rect.z) : mine.rect.z;
+                row_end = QUAD ? quad_hi(mine.rect.w) : mine.rect.w;
+            }
         }
-        __syncthreads();
-        const int e = s_entry;
-        __syncthreads();
-        if (e >= n_huge) break;
-        const MassiveEntry me = a.mq.entries[e];
-        const uint32_t db = __float_as_uint(me.ctr_power_depth.w);
-        const uint32_t gid = __float_as_uint(me.conic_gid.w);
-        if (VIEWS && ((uint32_t)me.rect.x >> 16) >= (uint32_t)a.n_views) continue;
-        const PreprocessParams& av = VIEWS ? a.views[(uint32_t)me.rect.x >> 16] : a;
-        if (MODE == kMassiveEmit64 && QUAD) {
-            const int qgx = quad_cols(av.gx);
-            sweep_cta_quad(me, av, s_band, s_pref, s_wsum, lane, warp, [&](bool v, int qx, int qy, uint32_t m) {
-                uint64_t key = ((uint64_t)(uint32_t)(av.tile_base + qy * qgx + qx) << 32) | db;
-                stage_emit(st, out, v, key, gid | (m << kQuadShift), lane);
-            });
-        } else if (MODE == kMassiveEmit64) {
-            sweep_cta(me, av, s_band, s_pref, s_wsum, lane, warp, [&](bool v, int x, int y) {
-                uint64_t key = ((uint64_t)(uint32_t)(av.tile_base + y * av.gx + x) << 32) | db;
-                stage_emit(st, out, v, key, gid, lane);
-            });
-        } else if (MODE == kMassiveCount) {
-            uint32_t cnt = 0;
-            if (QUAD)
-                sweep_cta_quad(me, a, s_band, s_pref, s_wsum, lane, warp, [&](bool v, int, int, uint32_t) {
-                    cnt += __popc(__ballot_sync(GSR_FULL_MASK, v));
-                });
-            else
-                sweep_cta(me, a, s_band, s_pref, s_wsum, lane, warp, [&](bool v, int, int) {
-                    cnt += __popc(__ballot_sync(GSR_FULL_MASK, v));
-                });
-            if (lane == 0) s_wcnt[warp] = cnt;
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                uint32_t t = 0;
-                for (int w = 0; w < kWarps; w++) t += s_wcnt[w];
-                a.df.count[gid] = t;
-            }
-        } else {
-            // Gaussians that hit no tile were not ranked
-            const uint32_t count = a.df.count[gid];
-            if (count == 0u) continue;
-            const long long base = df.offsets[df.rank[gid]];
-            // a pair (tile id, value) at the next of the Gaussian's own slots
-            auto put = [&](bool v, uint32_t tile, uint32_t val) {
-                const unsigned m = __ballot_sync(GSR_FULL_MASK, v);
-                if (!m) return;
-                uint32_t w0 = 0;
-                if (lane == 0) w0 = atomicAdd(&s_pos, (uint32_t)__popc(m));
-                w0 = __shfl_sync(GSR_FULL_MASK, w0, 0);
-                const uint32_t k = w0 + __popc(m & lanemask_lt());
-                if (v && k < count && base + k < df.cap) {  // never past the Gaussian's own slots
-                    df.tiles[base + k] = tile;
-                    df.vals[base + k] = val;
+        for (;;) {
+            // ---- list this warp's next rows that have candidates ----
+            int listed = 0, total = 0;
+            while (row < row_end && listed + 32 <= kSegRows) {
+                const int y = row + (int)lane;
+                const int x_lo = mine.rect.x & 0xFFFF, x_hi = mine.rect.y;
+                int lo = 0, n = 0;
+                if (y < row_end) {
+                    int hi = -1;
+                    bool any;
+                    if (eb.kind == kBandFull) {
+                        lo = QUAD ? quad_lo(x_lo) : x_lo;
+                        hi = (QUAD ? quad_hi(x_hi) : x_hi) - 1;
+                        any = true;
+                    } else if (QUAD) {
+                        any = band_quads(eb, y, a.by, a.bx, x_lo, x_hi, mine.rect.z, mine.rect.w, lo, hi);
+                    } else {
+                        any = band_columns(eb, y, a.by, a.bx, x_lo, x_hi, lo, hi);
+                    }
+                    if (any) n = hi - lo + 1;
                 }
-            };
-            if (QUAD) {
-                const int qgx = quad_cols(a.gx);
-                sweep_cta_quad(me, a, s_band, s_pref, s_wsum, lane, warp, [&](bool v, int qx, int qy, uint32_t m) {
-                    put(v, (uint32_t)(qy * qgx + qx), gid | (m << kQuadShift));
-                });
-            } else {
-                sweep_cta(me, a, s_band, s_pref, s_wsum, lane, warp,
-                          [&](bool v, int x, int y) { put(v, (uint32_t)(y * a.gx + x), gid); });
-            }
-            // sweep_cta ended on a barrier, so s_pos is final; every thread
-            // reads it before thread 0 resets it for the next entry
-            const uint32_t filled = s_pos;
-            __syncthreads();
-            for (uint32_t k = filled + threadIdx.x; k < count; k += kThreads)  // pad unfilled slots
-                if (base + k < df.cap) {
-                    df.tiles[base + k] = kTileSentinel;
-                    df.vals[base + k] = kTileSentinel;
+                int incl = n;
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const int t = __shfl_up_sync(GSR_FULL_MASK, incl, d);
+                    if ((int)lane >= d) incl += t;
                 }
+                const unsigned m = __ballot_sync(GSR_FULL_MASK, n > 0);
+                if (n > 0) {
+                    const int k = listed + __popc(m & lanemask_lt());
+                    s_start[warp][k] = total + incl - n;
+                    s_row[warp][k] = (uint32_t)lo | ((uint32_t)y << 16);
+                }
+                listed += __popc(m);
+                total += __shfl_sync(GSR_FULL_MASK, incl, 31);
+                row += 32;
+            }
+            if (lane == 0) {
+                s_start[warp][listed] = total;
+                s_rows[warp] = listed;
+            }
+            const int more = __syncthreads_or(row < row_end);
+
+            // ---- this warp's share of all the candidates ----
+            int all = 0;
+#pragma unroll
+            for (int w = 0; w < kWarps; w++) all += s_start[w][s_rows[w]];
+            const int share = ((all + kWarps * 32 - 1) / (kWarps * 32)) * 32;
+            const int from = warp * share, to = min(all, from + share);
+            int seg0 = 0;  // candidates before rectangle w
+            for (int w = 0; w < kWarps && seg0 < to; w++) {
+                const int rows = s_rows[w], n = s_start[w][rows];
+                const int t1 = min(n, to - seg0);
+                int t = max(0, from - seg0);
+                seg0 += n;
+                if (t >= t1) continue;
+                const MassiveEntry me = a.mq.entries[e0 + w];
+                const PreprocessParams& av = VIEWS ? a.views[(uint32_t)me.rect.x >> 16] : a;
+                const uint32_t db = __float_as_uint(me.ctr_power_depth.w);
+                const uint32_t gid = __float_as_uint(me.conic_gid.w);
+                const float2 c = {me.ctr_power_depth.x, me.ctr_power_depth.y};
+                const float pw = me.ctr_power_depth.z;
+                const float3 q = {me.conic_gid.x, me.conic_gid.y, me.conic_gid.z};
+                const int2 rmin = make_int2(me.rect.x & 0xFFFF, me.rect.z), rmax = make_int2(me.rect.y, me.rect.w);
+                const int cols = QUAD ? quad_cols(av.gx) : av.gx;
+                uint32_t count = 0;
+                long long base = 0;
+                if (MODE == kMassiveEmitDf) {
+                    // Gaussians that hit no tile were not ranked
+                    count = a.df.count[gid];
+                    if (count == 0u) continue;
+                    base = df.offsets[df.rank[gid]];
+                }
+                // the listed row holding candidate t
+                int r0 = 0, hi = rows - 1;
+                while (r0 < hi) {
+                    const int mid = (r0 + hi + 1) >> 1;
+                    if (s_start[w][mid] <= t) r0 = mid;
+                    else hi = mid - 1;
+                }
+                uint32_t hits = 0;
+                for (; t < t1; t += 32) {
+                    // rows after r0 that begin within this step
+                    const int k = r0 + 1 + (int)lane;
+                    const int at = k < rows ? s_start[w][k] - t : 64;
+                    const unsigned begins = __reduce_or_sync(GSR_FULL_MASK, at < 32 ? 1u << at : 0u);
+                    const int r = r0 + __popc(begins & (lanemask_lt() | (1u << lane)));
+                    r0 += __popc(__ballot_sync(GSR_FULL_MASK, at <= 32));
+                    const bool ok = t + (int)lane < t1;
+                    const uint32_t rw = s_row[w][r];
+                    const int x = (int)(rw & 0xFFFFu) + t + (int)lane - s_start[w][r], y = (int)(rw >> 16);
+                    uint32_t m = 0u;
+                    if (ok) {
+                        if (QUAD) m = quad_mask(x, y, rmin, rmax, a.bx, a.by, c, q, pw);
+                        else m = tile_hit(x, y, a.bx, a.by, c, q, pw) ? 1u : 0u;
+                    }
+                    const uint32_t tile = (uint32_t)(y * cols + x);
+                    const uint32_t val = QUAD ? gid | (m << kQuadShift) : gid;
+                    if (MODE == kMassiveEmit64) {
+                        stage_emit(st, out, m != 0u, ((uint64_t)(tile + (uint32_t)av.tile_base) << 32) | db, val, lane);
+                    } else {
+                        const unsigned mm = __ballot_sync(GSR_FULL_MASK, m != 0u);
+                        if (MODE == kMassiveCount) {
+                            hits += __popc(mm);
+                        } else if (mm) {  // the next of the Gaussian's own slots
+                            uint32_t p = 0;
+                            if (lane == 0) p = atomicAdd(&s_pos[w], (uint32_t)__popc(mm));
+                            p = __shfl_sync(GSR_FULL_MASK, p, 0) + __popc(mm & lanemask_lt());
+                            if (m != 0u && p < count && base + p < df.cap) {
+                                df.tiles[base + p] = tile;
+                                df.vals[base + p] = val;
+                            }
+                        }
+                    }
+                }
+                if (MODE == kMassiveCount && lane == 0 && hits) atomicAdd(&s_pos[w], hits);
+            }
+            __syncthreads();  // the lists are rewritten, s_pos is complete
+            if (!more) break;
+        }
+        if (row_end > 0 && MODE != kMassiveEmit64) {
+            const uint32_t gid = __float_as_uint(mine.conic_gid.w);
+            if (MODE == kMassiveCount) {
+                if (lane == 0) a.df.count[gid] = s_pos[warp];
+            } else if (const uint32_t count = a.df.count[gid]) {
+                const long long base = df.offsets[df.rank[gid]];
+                for (uint32_t k = s_pos[warp] + lane; k < count; k += 32)  // pad unfilled slots
+                    if (base + k < df.cap) {
+                        df.tiles[base + k] = kTileSentinel;
+                        df.vals[base + k] = kTileSentinel;
+                    }
+            }
+            __syncwarp();  // s_pos[warp] has been read
         }
     }
 
@@ -1072,28 +1000,30 @@ __global__ __launch_bounds__(kThreads) void k_emit_massive(const __grid_constant
         e = __shfl_sync(GSR_FULL_MASK, e, 0);
         if (e >= n_large) break;
         const MassiveEntry me = a.mq.entries[a.mq.huge_capacity + e];
+        if (!view_ok(me)) continue;
+        const Band eb = entry_band(me, a.bx);
         const uint32_t db = __float_as_uint(me.ctr_power_depth.w);
         const uint32_t gid = __float_as_uint(me.conic_gid.w);
-        if (VIEWS && ((uint32_t)me.rect.x >> 16) >= (uint32_t)a.n_views) continue;
         const PreprocessParams& av = VIEWS ? a.views[(uint32_t)me.rect.x >> 16] : a;
         if (MODE == kMassiveEmit64 && QUAD) {
             const int qgx = quad_cols(av.gx);
-            sweep_warp_quad(me, av, lane, [&](bool v, int qx, int qy, uint32_t m) {
+            sweep_warp_quad(me, eb, av, lane, [&](bool v, int qx, int qy, uint32_t m) {
                 uint64_t key = ((uint64_t)(uint32_t)(av.tile_base + qy * qgx + qx) << 32) | db;
                 stage_emit(st, out, v, key, gid | (m << kQuadShift), lane);
             });
         } else if (MODE == kMassiveEmit64) {
-            sweep_warp(me, av, lane, [&](bool v, int x, int y) {
+            sweep_warp(me, eb, av, lane, [&](bool v, int x, int y) {
                 uint64_t key = ((uint64_t)(uint32_t)(av.tile_base + y * av.gx + x) << 32) | db;
                 stage_emit(st, out, v, key, gid, lane);
             });
         } else if (MODE == kMassiveCount) {
             uint32_t cnt = 0;
             if (QUAD)
-                sweep_warp_quad(me, a, lane,
+                sweep_warp_quad(me, eb, a, lane,
                                 [&](bool v, int, int, uint32_t) { cnt += __popc(__ballot_sync(GSR_FULL_MASK, v)); });
             else
-                sweep_warp(me, a, lane, [&](bool v, int, int) { cnt += __popc(__ballot_sync(GSR_FULL_MASK, v)); });
+                sweep_warp(me, eb, a, lane,
+                           [&](bool v, int, int) { cnt += __popc(__ballot_sync(GSR_FULL_MASK, v)); });
             if (lane == 0) a.df.count[gid] = cnt;
         } else {
             const uint32_t count = a.df.count[gid];
@@ -1103,7 +1033,7 @@ __global__ __launch_bounds__(kThreads) void k_emit_massive(const __grid_constant
             auto put = [&](bool v, uint32_t tile, uint32_t val) {
                 const unsigned m = __ballot_sync(GSR_FULL_MASK, v);
                 const uint32_t k = wpos + __popc(m & lanemask_lt());
-                if (v && k < count && base + k < df.cap) {
+                if (v && k < count && base + k < df.cap) {  // never past the Gaussian's own slots
                     df.tiles[base + k] = tile;
                     df.vals[base + k] = val;
                 }
@@ -1111,13 +1041,13 @@ __global__ __launch_bounds__(kThreads) void k_emit_massive(const __grid_constant
             };
             if (QUAD) {
                 const int qgx = quad_cols(a.gx);
-                sweep_warp_quad(me, a, lane, [&](bool v, int qx, int qy, uint32_t m) {
+                sweep_warp_quad(me, eb, a, lane, [&](bool v, int qx, int qy, uint32_t m) {
                     put(v, (uint32_t)(qy * qgx + qx), gid | (m << kQuadShift));
                 });
             } else {
-                sweep_warp(me, a, lane, [&](bool v, int x, int y) { put(v, (uint32_t)(y * a.gx + x), gid); });
+                sweep_warp(me, eb, a, lane, [&](bool v, int x, int y) { put(v, (uint32_t)(y * a.gx + x), gid); });
             }
-            for (uint32_t k = wpos + lane; k < count; k += 32)
+            for (uint32_t k = wpos + lane; k < count; k += 32)  // pad unfilled slots
                 if (base + k < df.cap) {
                     df.tiles[base + k] = kTileSentinel;
                     df.vals[base + k] = kTileSentinel;
@@ -1477,7 +1407,7 @@ __global__ __launch_bounds__(256) void k_es_pass_b(int P, int bx, int by, int gx
         const int x1 = min(gx, (int)(int16_t)(r.y & 0xFFFF)), y1 = (int)(int16_t)((r.y >> 16) & 0xFFFF);
         me.rect = make_int4(x0, max(x0, x1), y0, max(y0, y1));
         uint32_t wpos = 0;
-        sweep_warp(me, pp, lane, [&](bool v, int x, int y) {
+        sweep_warp(me, entry_band(me, bx), pp, lane, [&](bool v, int x, int y) {
             const unsigned m = __ballot_sync(GSR_FULL_MASK, v);
             if (v) {
                 const long long pos = base + wpos + __popc(m & lanemask_lt());

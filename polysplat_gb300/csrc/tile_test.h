@@ -92,27 +92,34 @@ GSR_TT_FN bool tile_hit(int x, int y, int bx, int by, float2 ctr, float3 con, fl
 // dy)) / A, which does not cancel near the top and bottom, so every extent
 // carries a few ulp of relative error.
 //
-// kBandNeedle: A, C > 0 but AC - B^2 is below 1e-6 AC, or negative, or the
-// ellipse is beyond the above's range.  The float discriminant says little
-// there, but an accepted edge still lies near the conic's axis.  Write D(t, a,
-// p) = a w (1 + e) + t^2 (max(0, -det) + e (AC + B^2)) with e = 16 u: the
-// computed discriminant is at most 4 D (each of its operations errs by u of
-// terms that sum to at most (AC + B^2) t^2 + a w, four of them in all).  The
-// test accepts the row's pixels [l, r] on a vertical edge at offset dx = cx -
-// ex only if t1 <= 2 sqrt(D) and t2 >= -2 sqrt(D) up to their rounding, that
-// is if (B / C) dx lies within E = sqrt(D(dx, C)) / C + 4u (|l - cy| +
-// |B dx| / C) of [l - cy, r - cy], so ex lies in an interval; and a horizontal
-// edge at offset dy only if the tile's columns meet cx + (B / A) dy -+ E' with
-// the same form.  E is taken at the rectangle's largest |dx|.  The row's
+// kBandNeedle: A and C of one sign, with AC - B^2 below 1e-6 AC, or negative,
+// or the ellipse beyond the above's range (FP32 covariances whose determinant
+// cancelled, to a few ulp or to below zero).  The float discriminant says
+// little there, but an accepted edge still lies near the conic's axis.  Write
+// D(t, a) = max(a, 0) w + e |a| w + t^2 (max(0, -det) + e (AC + B^2)) with e =
+// 16 u: the computed discriminant is at most 4 D (each of its operations errs
+// by u of terms that sum to at most (AC + B^2) t^2 + |a| w, four of them in
+// all).  With a > 0 the test accepts the row's pixels [l, r] on a vertical edge
+// at offset dx = cx - ex only if t1 <= 2 sqrt(D) and t2 >= -2 sqrt(D) up to
+// their rounding, that is if (B / C) dx lies within E = sqrt(D(dx, C)) / |C| +
+// 4u (|l - cy| + |B dx / C|) of [l - cy, r - cy]; with a < 0 the inequalities
+// turn round and ask that [l - cy, r - cy] lie within E of it, which implies
+// the same.  So ex lies in an interval; and a horizontal edge at offset dy is
+// accepted only if the tile's columns meet cx + (B / A) dy -+ E' with the same
+// form.  E is taken at the rectangle's largest |dx|.  The row's
 // candidates are the hull of both intervals and of the centre's tile, widened
 // by a pixel and a relative 1e-5.  One clustered 3 M-Gaussian 1080p frame
 // holds about 3200 rectangles of 8000 tiles each that are no well-conditioned
-// ellipse; sweeping all their tiles was two thirds of the emission's tests.
+// ellipse; sweeping all their tiles was two thirds of the emission's tests, and
+// the 40% of them with negative A and C hit a tile in four of them.
 //
-// kBandCentre: a NaN in the conic makes every discriminant NaN, and without
-// power > 0 no edge is tested: only the tile holding the centre can pass.
+// kBandCentre: a NaN in the conic makes every discriminant NaN, as do a conic
+// of infinities alone (a determinant of zero; inf - inf) with A and C of one
+// sign, and without power > 0 no edge is tested: only the tile holding the
+// centre can pass.
 //
-// kBandFull: everything else (A or C not positive, infinite): every tile.
+// kBandFull: everything else (A and C of different signs, zero, infinite):
+// every tile.
 enum : int { kBandFull = 0, kBandEllipse = 1, kBandNeedle = 2, kBandCentre = 3 };
 
 struct Band {
@@ -143,19 +150,22 @@ GSR_TT_FN Band make_band(float3 q, float power, float2 c, int x_lo, int x_hi, in
     b.e_h0 = b.e_h1 = b.e_v = 0.0f;
     b.kind = kBandFull;
     const bool near = fabsf(c.x) < 1e7f && fabsf(c.y) < 1e7f;
-    if (!(A == A) || !(B == B) || !(C == C) || !(power > 0.0f)) {
+    const bool infinite = fabsf(A) > 3.4028235e38f && fabsf(B) > 3.4028235e38f && fabsf(C) > 3.4028235e38f;
+    if (!(A == A) || !(B == B) || !(C == C) || !(power > 0.0f) || (infinite && A * C > 0.0f)) {
         b.kind = kBandCentre;
     } else if (A > 0.0f && C > 0.0f && det > 1e-6f * (A * C) && b.dymax < 1e6f && b.dxmax < 1e6f &&
                fabsf(b.dyr) < 1e6f && near) {
         b.kind = kBandEllipse;
-    } else if (near && A > 1e-15f && C > 1e-15f && A < 1e15f && C < 1e15f && fabsf(B) < 1e15f && w < 1e15f) {
+    } else if (near && A * C > 0.0f && fabsf(A) > 1e-15f && fabsf(C) > 1e-15f && fabsf(A) < 1e15f && fabsf(C) < 1e15f &&
+               fabsf(B) < 1e15f && w < 1e15f) {
         b.kind = kBandNeedle;
         const float e = 16.0f * u;
         const float grow = fmaxf(0.0f, -det) + e * GSR_TT_FMA(A, C, bb);
         const float dxm = fmaxf(fabsf(c.x - (float)(x_lo * bx)), fabsf(c.x - (float)(x_hi * bx)));
-        b.e_h0 = A * w * (1.0f + e);
+        b.e_h0 = (fmaxf(A, 0.0f) + e * fabsf(A)) * w;
         b.e_h1 = grow;
-        b.e_v = sqrtf(C * w * (1.0f + e) + grow * dxm * dxm) * b.inv_c + 4.0f * u * fabsf(B) * dxm * b.inv_c;
+        b.e_v = (sqrtf((fmaxf(C, 0.0f) + e * fabsf(C)) * w + grow * dxm * dxm) + 4.0f * u * fabsf(B) * dxm) *
+                fabsf(b.inv_c);
         b.dxmax = dxm;
     }
     return b;
@@ -189,7 +199,7 @@ GSR_TT_FN bool band_columns(const Band& e, int ty, int by, int bx, int x_lo, int
             // horizontal edge: the test's dy, its middle and half-width
             const float dy = e.cy * 2.0f < l + r ? e.cy - l : e.cy - r;
             const float mid = e.B * dy * e.inv_a;
-            const float eh = sqrtf(e.e_h0 + e.e_h1 * dy * dy) * e.inv_a + 4.0f * u * (e.dxmax + fabsf(mid));
+            const float eh = sqrtf(e.e_h0 + e.e_h1 * dy * dy) * fabsf(e.inv_a) + 4.0f * u * (e.dxmax + fabsf(mid));
             const float mh = 1.0f + 1e-5f * (fabsf(e.cx) + fabsf(mid) + eh);
             lo = fminf(lo, e.cx + mid - eh - mh);
             hi = fmaxf(hi, e.cx + mid + eh + mh);

@@ -46,6 +46,9 @@ def _conics(rng, n):
     con[k:2 * k, 0] = np.inf
     con[2 * k:3 * k, 1] = 0.0
     con[3 * k:4 * k] = 0.0
+    con[5 * k:6 * k] *= np.float32(-1.0)  # both diagonal entries negative
+    con[6 * k:7 * k, 0] *= np.float32(-1.0)  # of different signs
+    con[7 * k:8 * k] = rng.choice([np.inf, -np.inf], (k, 3))
     power[4 * k:5 * k] = rng.choice([0.0, -1.0, np.nan], k)
     return con, power
 
