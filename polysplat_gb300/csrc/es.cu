@@ -172,8 +172,8 @@ gsr_status gsr_es_pass_a(int P, const float* pos, const void* shs, int shs_half,
     p.points_xy = reinterpret_cast<float2*>(points_xy);
     p.rgb_depth = reinterpret_cast<float4*>(rgb_depth);
     p.conic_opacity = reinterpret_cast<float4*>(conic_opacity);
-    // no large-Gaussian queue (the thresholds exceed every area): every count
-    // is made by the Gaussian's own warp, and no queue counter is touched
+    // no large-Gaussian queue (its capacity is 0): every count is made by the
+    // Gaussian's own warp, and no queue counter is touched
     p.massive_area = INT_MAX;
     p.huge_area = INT_MAX;
     p.df.count = reinterpret_cast<uint32_t*>(tiles_per_gauss);

@@ -173,22 +173,6 @@ __device__ __forceinline__ V3 sh_color(int idx, V3 p, V3 cam, const void* shs)
     return result;
 }
 
-// Tiles of quad (qx, qy) that lie in the Gaussian's rectangle [rmin, rmax)
-// and pass tile_hit: bit (x & 1) | (y & 1) << 1 per hit tile.  These are
-// exactly the tiles the per-tile emission would give keys.
-__device__ __forceinline__ uint32_t quad_mask(int qx, int qy, int2 rmin, int2 rmax, int bx, int by, float2 ctr,
-                                              float3 con, float power)
-{
-    uint32_t m = 0u;
-#pragma unroll
-    for (int s = 0; s < 4; s++) {
-        const int x = 2 * qx + (s & 1), y = 2 * qy + (s >> 1);
-        if (x >= rmin.x && x < rmax.x && y >= rmin.y && y < rmax.y && tile_hit(x, y, bx, by, ctr, con, power))
-            m |= 1u << s;
-    }
-    return m;
-}
-
 // Quad-rectangle [q0, q1) covering tile columns (or rows) [t0, t1), t1 > t0.
 __device__ __forceinline__ int quad_lo(int t0) { return t0 >> 1; }
 __device__ __forceinline__ int quad_hi(int t1) { return ((t1 - 1) >> 1) + 1; }
@@ -250,12 +234,21 @@ __device__ __forceinline__ void stage_emit(Stage& s, const EmitOut& o, bool vali
 // Dispatch thresholds (PreprocessParams::massive_area / huge_area; the
 // defaults are kDefaultMassiveArea / kDefaultHugeArea): tile rectangles at
 // least massive_area tiles large are queued for k_emit_massive, and of those
-// the ones of at least huge_area tiles are swept by a whole CTA.  They only
+// the ones of at least huge_area tiles are swept by a whole CTA.  A threshold
+// above kPoolArea acts as kPoolArea, the most the warp's pool takes.  They only
 // decide which scheme tests a rectangle's tiles, never which keys come out.
 
-// Block-wide final flush of every warp's staged keys with one atomic per CTA.
-__device__ __forceinline__ void block_flush(Stage& st, const EmitOut& out, int* s_fill, long long* s_base,
-                                            unsigned lane, int warp)
+// a / b for 0 <= a < 2^12, 0 < b < 2^7: (a + 1/2) / b is at least 1/256 away from
+// an integer, far more than the division's error.
+__device__ __forceinline__ int small_div(int a, int b) { return (int)__fdividef((float)a + 0.5f, (float)b); }
+
+constexpr int kPoolArea = 128;
+
+// Block-wide final flush of every warp's staged keys with one atomic per CTA:
+// the reservation, whose round trip the preprocess hides behind its colours,
+// and the copy.
+__device__ __forceinline__ void block_reserve(const Stage& st, const EmitOut& out, int* s_fill, long long* s_base,
+                                              unsigned lane, int warp)
 {
     if (lane == 0) s_fill[warp] = st.fill;
     __syncthreads();
@@ -273,6 +266,11 @@ __device__ __forceinline__ void block_flush(Stage& st, const EmitOut& out, int* 
         base = __shfl_sync(GSR_FULL_MASK, base, 0);
         if (lane < kWarps) s_base[lane] = base + incl - f;
     }
+}
+
+__device__ __forceinline__ void block_copy(Stage& st, const EmitOut& out, const long long* s_base, unsigned lane,
+                                           int warp)
+{
     __syncthreads();
     const long long wb = s_base[warp];
     for (int i = lane; i < st.fill; i += 32) {
@@ -324,7 +322,7 @@ __global__ __launch_bounds__(kThreads, VIEWS ? 6 : 5) void k_preprocess(const __
     __shared__ int s_fill[kWarps];
     __shared__ long long s_base[kWarps];
     __shared__ uint32_t s_hit[kWarps];
-    __shared__ int s_pref[kWarps][32];
+    __shared__ uint8_t s_owner[kWarps][32];  // lanes of the pool's Gaussians, in order
     __shared__ uint32_t s_cnt[kWarps][32];
 
     const unsigned lane = threadIdx.x & 31u;
@@ -413,8 +411,8 @@ __global__ __launch_bounds__(kThreads, VIEWS ? 6 : 5) void k_preprocess(const __
     // warp tests the Gaussian itself over an 8x4 tile window (the reference's
     // "massive" scheme, preprocess.cu:444-519).  Every scheme tests every
     // tile of the rectangle with the same test, so the key set is the same.
-    bool massive = point_valid && area >= a.massive_area;
-    {
+    bool massive = point_valid && area >= min(a.massive_area, kPoolArea);
+    if (a.mq.capacity > 0) {  // the ES layout and callers without a workspace have no queue
         // huge rectangles first try the CTA-swept region, then the warp one
         int slot = -1;
         const bool want_huge = massive && area >= a.huge_area;
@@ -461,6 +459,7 @@ __global__ __launch_bounds__(kThreads, VIEWS ? 6 : 5) void k_preprocess(const __
         const uint32_t db = __shfl_sync(GSR_FULL_MASK, depth_bits, i);
         const float pw = __shfl_sync(GSR_FULL_MASK, power, i);
         const uint32_t gid = (uint32_t)(a.gid_base + warp_first + i);
+        bool hit = a.mq.capacity > 0;  // features are written for Gaussians that belong to a queue
         if (QUAD) {
             const int qx_lo = quad_lo(x_lo), qx_hi = quad_hi(x_hi), qy_lo = quad_lo(y_lo), qy_hi = quad_hi(y_hi);
             for (int y0 = qy_lo; y0 < qy_hi; y0 += 4) {
@@ -471,6 +470,7 @@ __global__ __launch_bounds__(kThreads, VIEWS ? 6 : 5) void k_preprocess(const __
                                            ? quad_mask(qx, qy, make_int2(x_lo, y_lo), make_int2(x_hi, y_hi), a.bx,
                                                        a.by, c, q, pw)
                                            : 0u;
+                    hit = hit || m != 0u;
                     if (COUNT) {
                         const unsigned mm = __ballot_sync(GSR_FULL_MASK, m != 0u);
                         if (lane == 0) s_cnt[warp][i] += __popc(mm);
@@ -486,6 +486,7 @@ __global__ __launch_bounds__(kThreads, VIEWS ? 6 : 5) void k_preprocess(const __
                 for (int x0 = x_lo; x0 < x_hi; x0 += 8) {
                     const int x = x0 + tx;
                     bool v = y < y_hi && x < x_hi && tile_hit(x, y, a.bx, a.by, c, q, pw);
+                    hit = hit || v;
                     if (COUNT) {
                         const unsigned m = __ballot_sync(GSR_FULL_MASK, v);
                         if (lane == 0) s_cnt[warp][i] += __popc(m);
@@ -496,7 +497,8 @@ __global__ __launch_bounds__(kThreads, VIEWS ? 6 : 5) void k_preprocess(const __
                 }
             }
         }
-        if (lane == 0) atomicOr(&s_hit[warp], 1u << i);
+        hit = __any_sync(GSR_FULL_MASK, hit);
+        if (lane == 0 && hit) atomicOr(&s_hit[warp], 1u << i);
     }
     point_valid = point_valid && !massive;
 
@@ -514,25 +516,26 @@ __global__ __launch_bounds__(kThreads, VIEWS ? 6 : 5) void k_preprocess(const __
             if ((int)lane >= d) prefix += n;
         }
         const int total = __shfl_sync(GSR_FULL_MASK, prefix, 31);
-        s_pref[warp][lane] = prefix;  // inclusive prefix of the tile counts
+        prefix -= my_tiles;  // the Gaussian's first task
+        if (point_valid) s_owner[warp][__popc(multi & lanemask_lt())] = (uint8_t)lane;
         __syncwarp();
-        prefix -= my_tiles;
+        // what a task needs of its owner beyond the test's operands
+        const uint32_t corner = (uint32_t)rect_min.x | ((uint32_t)rect_min.y << 16);
+        const uint32_t extent = (uint32_t)prefix | ((uint32_t)(rect_max.x - rect_min.x) << 12) |
+                                ((uint32_t)(rect_max.y - rect_min.y) << 19);  // areas below kPoolArea
         for (int base = 0; base < total; base += 32) {
             const int task = base + (int)lane;
             const bool task_ok = task < total;
-            // owner = first lane whose inclusive prefix exceeds the task index
-            int lo = 0, hi = 31;
-#pragma unroll
-            for (int step = 0; step < 5; step++) {
-                const int mid = (lo + hi) >> 1;
-                if (s_pref[warp][mid] > task) hi = mid;
-                else lo = mid + 1;
-            }
-            const int owner = task_ok ? lo : __ffs(multi) - 1;
-            const int ox = __shfl_sync(GSR_FULL_MASK, rect_min.x, owner);
-            const int oy = __shfl_sync(GSR_FULL_MASK, rect_min.y, owner);
-            const int ow = __shfl_sync(GSR_FULL_MASK, rect_max.x, owner) - ox;
-            const int op = __shfl_sync(GSR_FULL_MASK, prefix, owner);
+            // the owners' first tasks follow each other: those at or before
+            // `base`, and one bit for each later one in this step
+            const int at = prefix - base;
+            const int before = __popc(__ballot_sync(GSR_FULL_MASK, point_valid && at <= 0));
+            const unsigned begins = __reduce_or_sync(GSR_FULL_MASK, point_valid && at > 0 && at < 32 ? 1u << at : 0u);
+            const int owner = s_owner[warp][before - 1 + __popc(begins & (lanemask_lt() | (1u << lane)))];
+            const uint32_t oc = __shfl_sync(GSR_FULL_MASK, corner, owner);
+            const uint32_t oe = __shfl_sync(GSR_FULL_MASK, extent, owner);
+            const int ox = (int)(oc & 0xFFFFu), oy = (int)(oc >> 16);
+            const int ow = (int)(oe >> 12) & 127, local = task - (int)(oe & 4095u);
             const float2 c = {__shfl_sync(GSR_FULL_MASK, point_xy.x, owner),
                               __shfl_sync(GSR_FULL_MASK, point_xy.y, owner)};
             const float3 q = {__shfl_sync(GSR_FULL_MASK, conic.x, owner), __shfl_sync(GSR_FULL_MASK, conic.y, owner),
@@ -543,19 +546,17 @@ __global__ __launch_bounds__(kThreads, VIEWS ? 6 : 5) void k_preprocess(const __
             bool v = false;
             uint32_t qm = 0u;
             if (QUAD) {
-                const int oy1 = __shfl_sync(GSR_FULL_MASK, rect_max.y, owner);
                 const int oqx = quad_lo(ox), oqw = quad_hi(ox + ow) - oqx;
                 if (task_ok) {
-                    const int local = task - op;
-                    const int row = oqw > 0 ? local / oqw : 0;
+                    const int row = small_div(local, oqw);
                     x = oqx + (local - row * oqw);
                     y = quad_lo(oy) + row;
-                    qm = quad_mask(x, y, make_int2(ox, oy), make_int2(ox + ow, oy1), a.bx, a.by, c, q, pw);
+                    qm = quad_mask(x, y, make_int2(ox, oy), make_int2(ox + ow, oy + (int)(oe >> 19)), a.bx, a.by, c, q,
+                                   pw);
                     v = qm != 0u;
                 }
             } else if (task_ok) {
-                const int local = task - op;
-                const int row = ow > 0 ? local / ow : 0;
+                const int row = small_div(local, ow);
                 x = ox + (local - row * ow);
                 y = oy + row;
                 v = tile_hit(x, y, a.bx, a.by, c, q, pw);
@@ -573,6 +574,7 @@ __global__ __launch_bounds__(kThreads, VIEWS ? 6 : 5) void k_preprocess(const __
         }
     }
     __syncwarp();
+    if (!COUNT) block_reserve(st, out, s_fill, s_base, lane, warp);
 
     // (3) render features for every Gaussian that emitted at least one key.
     const bool emitted = (s_hit[warp] >> lane) & 1u;
@@ -626,8 +628,8 @@ __global__ __launch_bounds__(kThreads, VIEWS ? 6 : 5) void k_preprocess(const __
             }
         }
     } else {
-        // (4) block-wide final flush: one atomic per CTA.
-        block_flush(st, out, s_fill, s_base, lane, warp);
+        // (4) the staged keys, to the place reserved before the features
+        block_copy(st, out, s_base, lane, warp);
     }
 }
 
@@ -1054,7 +1056,10 @@ __global__ __launch_bounds__(kThreads, 4) void k_emit_massive(const __grid_const
                 }
         }
     }
-    if (MODE == kMassiveEmit64) block_flush(st, out, s_fill, s_base, lane, warp);
+    if (MODE == kMassiveEmit64) {
+        block_reserve(st, out, s_fill, s_base, lane, warp);
+        block_copy(st, out, s_base, lane, warp);
+    }
 }
 
 // Depth-first emission of the Gaussians that were not queued, taken in depth
