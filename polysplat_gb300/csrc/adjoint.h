@@ -132,7 +132,8 @@ struct Tape {
     bool clamp_rgb[3];
 };
 
-template <typename T>
+// COLOR = false leaves the colour out (see color_adjoint).
+template <typename T, bool COLOR = true>
 GSR_HD void forward(const T m[3], const T ls[3], const T q[4], T logit, const T* sh, const Cam<T>& cam, Fwd<T>& f,
                     Tape<T>& tp)
 {
@@ -192,6 +193,7 @@ GSR_HD void forward(const T m[3], const T ls[3], const T q[4], T logit, const T*
     f.xy[0] = ((tp.ph[0] / tp.w + 1) * cam.W - 1) * (T)0.5;
     f.xy[1] = ((tp.ph[1] / tp.w + 1) * cam.H - 1) * (T)0.5;
     f.depth = tp.t[2];
+    if (!COLOR) return;
     // colour
     T v[3] = {m[0] - cam.campos[0], m[1] - cam.campos[1], m[2] - cam.campos[2]};
     tp.vlen = t_sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
@@ -205,10 +207,35 @@ GSR_HD void forward(const T m[3], const T ls[3], const T q[4], T logit, const T*
     }
 }
 
-// Gradients of the raw parameters from those of xy, con and rgb.  ADD_SH:
-// add the SH gradient to g_sh instead of writing it (a caller summing over
-// views needs no second 48-entry array).
-template <typename T, bool ADD_SH = false>
+// The colour's share of the adjoint on its own: adds its part of dL/dmean to
+// g_m and gives the colour gradient behind the clamp, with which the SH
+// gradient is B[k] g[ch] (B: sh_basis of the view direction).
+template <typename T>
+GSR_HD void color_adjoint(const T m[3], const T campos[3], const T* sh, const T g_rgb[3], T g_m[3], T g[3])
+{
+    T v[3] = {m[0] - campos[0], m[1] - campos[1], m[2] - campos[2]};
+    const T vlen = t_sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
+    T dir[3];
+    for (int i = 0; i < 3; i++) dir[i] = v[i] / vlen;
+    T B[16], dB[16][3];
+    sh_basis(dir[0], dir[1], dir[2], B, dB);
+    for (int ch = 0; ch < 3; ch++) {
+        T r = (T)0.5;
+        for (int k = 0; k < 16; k++) r += B[k] * sh[3 * k + ch];
+        g[ch] = r < 0 ? (T)0 : g_rgb[ch];
+    }
+    T g_dir[3] = {0, 0, 0};
+    for (int k = 0; k < 16; k++) {
+        const T s = sh[3 * k] * g[0] + sh[3 * k + 1] * g[1] + sh[3 * k + 2] * g[2];
+        for (int d = 0; d < 3; d++) g_dir[d] += dB[k][d] * s;
+    }
+    const T dd = g_dir[0] * dir[0] + g_dir[1] * dir[1] + g_dir[2] * dir[2];
+    for (int i = 0; i < 3; i++) g_m[i] += (g_dir[i] - dir[i] * dd) / vlen;
+}
+
+// Gradients of the raw parameters from those of xy, con and rgb.  COLOR =
+// false leaves the colour's part (and g_sh) out.
+template <typename T, bool COLOR = true>
 GSR_HD void backward(const T m[3], const T* sh, const Cam<T>& cam, const Tape<T>& tp, const T g_xy[2], const T g_con[4],
                      const T g_rgb[3], T g_m[3], T g_ls[3], T g_q[4], T& g_logit, T* g_sh)
 {
@@ -303,13 +330,13 @@ GSR_HD void backward(const T m[3], const T* sh, const Cam<T>& cam, const Tape<T>
     g_ph[3] = -(g_xy[0] * (T)0.5 * cam.W * tp.ph[0] + g_xy[1] * (T)0.5 * cam.H * tp.ph[1]) / (tp.w * tp.w);
     for (int col = 0; col < 3; col++)
         for (int r4 = 0; r4 < 4; r4++) g_m[col] += P[4 * col + r4] * g_ph[r4];
+    if (!COLOR) return;
     // colour
     T g_dir[3] = {0, 0, 0};
     for (int ch = 0; ch < 3; ch++) {
         const T g = tp.clamp_rgb[ch] ? (T)0 : g_rgb[ch];
         for (int k = 0; k < 16; k++) {
-            if (ADD_SH) g_sh[3 * k + ch] += tp.B[k] * g;
-            else g_sh[3 * k + ch] = tp.B[k] * g;
+            g_sh[3 * k + ch] = tp.B[k] * g;
             for (int d = 0; d < 3; d++) g_dir[d] += tp.dB[k][d] * sh[3 * k + ch] * g;
         }
     }

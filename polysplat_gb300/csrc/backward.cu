@@ -11,76 +11,12 @@
 namespace gsr {
 namespace {
 
-struct PreBackArgs {
-    int P;
-    const float* means;
-    const float* log_scales;
-    const float* quats;
-    const float* logits;
-    const float* shs;  // [P,48] f32
-    gsr_adj::Cam<float> cam;
-    const float* gxy;
-    const float* gcon;
-    const float* grgb;
-    float* g_means;
-    float* g_log_scales;
-    float* g_quats;
-    float* g_logits;
-    float* g_shs;
-    int accumulate;
-};
-
-// One thread per Gaussian: recompute the forward, apply the adjoint.
-// Gaussians that reached no pixel carry zero gradients and are skipped
-// (written as zeros unless accumulating).
-__global__ __launch_bounds__(128) void k_preprocess_backward(const __grid_constant__ PreBackArgs a)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.P) return;
-    float gxy[2] = {a.gxy[2 * (size_t)i], a.gxy[2 * (size_t)i + 1]};
-    float gcon[4], grgb[3];
-    bool any = gxy[0] != 0.f || gxy[1] != 0.f;
-    for (int k = 0; k < 4; k++) {
-        gcon[k] = a.gcon[4 * (size_t)i + k];
-        any |= gcon[k] != 0.f;
-    }
-    for (int k = 0; k < 3; k++) {
-        grgb[k] = a.grgb[3 * (size_t)i + k];
-        any |= grgb[k] != 0.f;
-    }
-    float gm[3] = {0.f, 0.f, 0.f}, gls[3] = {0.f, 0.f, 0.f}, gq[4] = {0.f, 0.f, 0.f, 0.f}, glogit = 0.f;
-    float gsh[48];
-    for (int k = 0; k < 48; k++) gsh[k] = 0.f;
-    if (any) {
-        float m[3], ls[3], q[4], sh[48];
-        for (int k = 0; k < 3; k++) {
-            m[k] = a.means[3 * (size_t)i + k];
-            ls[k] = a.log_scales[3 * (size_t)i + k];
-        }
-        for (int k = 0; k < 4; k++) q[k] = a.quats[4 * (size_t)i + k];
-        for (int k = 0; k < 48; k++) sh[k] = a.shs[48 * (size_t)i + k];
-        gsr_adj::Fwd<float> f;
-        gsr_adj::Tape<float> tp;
-        gsr_adj::forward(m, ls, q, a.logits[i], sh, a.cam, f, tp);
-        gsr_adj::backward(m, sh, a.cam, tp, gxy, gcon, grgb, gm, gls, gq, glogit, gsh);
-    } else if (a.accumulate) {
-        return;
-    }
-    auto put = [&](float* dst, size_t off, float v) { dst[off] = a.accumulate ? dst[off] + v : v; };
-    for (int k = 0; k < 3; k++) {
-        put(a.g_means, 3 * (size_t)i + k, gm[k]);
-        put(a.g_log_scales, 3 * (size_t)i + k, gls[k]);
-    }
-    for (int k = 0; k < 4; k++) put(a.g_quats, 4 * (size_t)i + k, gq[k]);
-    put(a.g_logits, i, glogit);
-    for (int k = 0; k < 48; k++) put(a.g_shs, 48 * (size_t)i + k, gsh[k]);
-}
-
-// Views of one multi-view adjoint launch (more views take several launches,
-// the later ones accumulating).
+// Views of one adjoint launch (more views take several launches, the later
+// ones accumulating).
 constexpr int kAdjViews = 16;
+constexpr int kAdjThreads = 128;
 
-struct PreBackViewsArgs {
+struct PreBackArgs {
     int P, n_views;
     const float* means;
     const float* log_scales;
@@ -92,6 +28,10 @@ struct PreBackViewsArgs {
     // opacity, xy, colour; 12 floats): view v's rows start at v * P (of the
     // launch's first view)
     const float4* grec;
+    // or one view's gradients in three arrays
+    const float* gxy;
+    const float* gcon;
+    const float* grgb;
     float* g_means;
     float* g_log_scales;
     float* g_quats;
@@ -100,56 +40,181 @@ struct PreBackViewsArgs {
     int accumulate;
 };
 
-// One thread per Gaussian over all views of the launch: the parameters are
-// read once, each view that saw the Gaussian replays its forward and adds
-// its adjoint, and the sums are written once.
-__global__ __launch_bounds__(128) void k_preprocess_backward_views(const __grid_constant__ PreBackViewsArgs a)
+// Gradients of Gaussian i's features in view v; false when all are zero (it
+// reached no pixel of the view).
+template <bool RECORDS>
+__device__ __forceinline__ bool feature_grads(const PreBackArgs& a, int i, int v, float (&gxy)[2], float (&gcon)[4],
+                                              float (&grgb)[3])
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.P) return;
-    float gm[3] = {0.f, 0.f, 0.f}, gls[3] = {0.f, 0.f, 0.f}, gq[4] = {0.f, 0.f, 0.f, 0.f}, glogit = 0.f;
-    float gsh[48];
-    for (int k = 0; k < 48; k++) gsh[k] = 0.f;
-    float m[3], ls[3], q[4], sh[48], logit = 0.f;
-    bool loaded = false;
-    for (int v = 0; v < a.n_views; v++) {
-        const size_t r = (size_t)v * a.P + i;
-        const float4 q0 = a.grec[3 * r], q1 = a.grec[3 * r + 1], q2 = a.grec[3 * r + 2];
-        float gcon[4] = {q0.x, q0.y, q0.z, q0.w}, gxy[2] = {q1.x, q1.y}, grgb[3] = {q1.z, q1.w, q2.x};
-        const bool any = gcon[0] != 0.f || gcon[1] != 0.f || gcon[2] != 0.f || gcon[3] != 0.f || gxy[0] != 0.f ||
-                         gxy[1] != 0.f || grgb[0] != 0.f || grgb[1] != 0.f || grgb[2] != 0.f;
-        if (!any) continue;
-        if (!loaded) {
+    if (RECORDS) {
+        const size_t r = 3 * ((size_t)v * a.P + i);
+        const float4 q0 = __ldg(a.grec + r), q1 = __ldg(a.grec + r + 1);
+        const float blue = __ldg(reinterpret_cast<const float*>(a.grec + r + 2));
+        gcon[0] = q0.x;
+        gcon[1] = q0.y;
+        gcon[2] = q0.z;
+        gcon[3] = q0.w;
+        gxy[0] = q1.x;
+        gxy[1] = q1.y;
+        grgb[0] = q1.z;
+        grgb[1] = q1.w;
+        grgb[2] = blue;
+    } else {
+        for (int k = 0; k < 4; k++) gcon[k] = __ldg(a.gcon + 4 * (size_t)i + k);
+        for (int k = 0; k < 2; k++) gxy[k] = __ldg(a.gxy + 2 * (size_t)i + k);
+        for (int k = 0; k < 3; k++) grgb[k] = __ldg(a.grgb + 3 * (size_t)i + k);
+    }
+    return gcon[0] != 0.f || gcon[1] != 0.f || gcon[2] != 0.f || gcon[3] != 0.f || gxy[0] != 0.f || gxy[1] != 0.f ||
+           grgb[0] != 0.f || grgb[1] != 0.f || grgb[2] != 0.f;
+}
+
+// A CTA takes 128 Gaussians.  A view sees few of them (saturated tiles stop
+// before most), so a thread per Gaussian that walks its views left 27 of 32
+// lanes idle (603 us for 1 M Gaussians and 8 views).  Instead the CTA lists its
+// (Gaussian, view) pairs with a gradient, and takes them a pair to a thread: the
+// forward replayed and its adjoint, without the SH gradients, which are the
+// product of 16 basis values and 3 colour gradients and are formed when each
+// Gaussian's thread sums its pairs, in view order, and writes its 59
+// gradients.  Rounds take up to 128 pairs and whole Gaussians.
+template <bool RECORDS>
+__global__ __launch_bounds__(kAdjThreads) void k_preprocess_backward(const __grid_constant__ PreBackArgs a)
+{
+    constexpr int kOut = 15;  // 11 gradients, 3 of the colour, and a stride without bank conflicts
+    __shared__ uint16_t s_pair[kAdjThreads * kAdjViews];  // Gaussian | view << 8
+    __shared__ float s_out[kAdjThreads][kOut];
+    __shared__ int s_warp[kAdjThreads / 32];
+    __shared__ int s_end;
+    const int tid = (int)threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int i0 = (int)blockIdx.x * kAdjThreads, i = i0 + tid;
+    // SH rows are 192 bytes: 16-byte accesses when both arrays start on 16 bytes
+    const bool wide = ((reinterpret_cast<uintptr_t>(a.shs) | reinterpret_cast<uintptr_t>(a.g_shs)) & 15u) == 0;
+
+    // ---- list the pairs ----
+    uint32_t seen = 0u;
+    if (i < a.P)
+        for (int v = 0; v < a.n_views; v++) {
+            float gxy[2], gcon[4], grgb[3];
+            if (feature_grads<RECORDS>(a, i, v, gxy, gcon, grgb)) seen |= 1u << v;
+        }
+    const int n = __popc(seen);
+    int incl = n;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int t = __shfl_up_sync(GSR_FULL_MASK, incl, d);
+        if (lane >= d) incl += t;
+    }
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    int first = incl - n, total = 0;
+#pragma unroll
+    for (int w = 0; w < kAdjThreads / 32; w++) {
+        if (w < warp) first += s_warp[w];
+        total += s_warp[w];
+    }
+    {
+        int k = first;
+        for (uint32_t m = seen; m; m &= m - 1) s_pair[k++] = (uint16_t)(tid | ((__ffs(m) - 1) << 8));
+    }
+    if (n == 0 && i < a.P && !a.accumulate) {  // never seen: zeros
+        for (int k = 0; k < 3; k++) a.g_means[3 * (size_t)i + k] = a.g_log_scales[3 * (size_t)i + k] = 0.f;
+        for (int k = 0; k < 4; k++) a.g_quats[4 * (size_t)i + k] = 0.f;
+        a.g_logits[i] = 0.f;
+        if (wide) {
+            for (int k = 0; k < 12; k++)
+                reinterpret_cast<float4*>(a.g_shs + 48 * (size_t)i)[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        } else {
+            for (int k = 0; k < 48; k++) a.g_shs[48 * (size_t)i + k] = 0.f;
+        }
+    }
+
+    for (int begin = 0; begin < total;) {
+        // the round: the Gaussians whose pairs end within 128 of `begin`
+        __syncthreads();  // s_pair is complete, s_out and s_end of the last round have been read
+        if (tid == 0) s_end = begin;
+        __syncthreads();
+        const bool mine = n > 0 && first >= begin && first + n <= begin + kAdjThreads;
+        if (mine) atomicMax(&s_end, first + n);
+        __syncthreads();
+        const int end = s_end;
+
+        // ---- a pair to a thread ----
+        if (begin + tid < end) {
+            const int pr = s_pair[begin + tid], v = pr >> 8;
+            const size_t j = (size_t)i0 + (pr & 0xFF);
+            float gxy[2], gcon[4], grgb[3];
+            feature_grads<RECORDS>(a, (int)j, v, gxy, gcon, grgb);
+            float m[3], ls[3], q[4], gm[3], gls[3], gq[4], glogit, g[3];
             for (int k = 0; k < 3; k++) {
-                m[k] = a.means[3 * (size_t)i + k];
-                ls[k] = a.log_scales[3 * (size_t)i + k];
+                m[k] = __ldg(a.means + 3 * j + k);
+                ls[k] = __ldg(a.log_scales + 3 * j + k);
             }
-            for (int k = 0; k < 4; k++) q[k] = a.quats[4 * (size_t)i + k];
-            for (int k = 0; k < 48; k++) sh[k] = a.shs[48 * (size_t)i + k];
-            logit = a.logits[i];
-            loaded = true;
+            for (int k = 0; k < 4; k++) q[k] = __ldg(a.quats + 4 * j + k);
+            gsr_adj::Fwd<float> f;
+            gsr_adj::Tape<float> tp;
+            gsr_adj::forward<float, false>(m, ls, q, __ldg(a.logits + j), nullptr, a.cam[v], f, tp);
+            gsr_adj::backward<float, false>(m, nullptr, a.cam[v], tp, gxy, gcon, grgb, gm, gls, gq, glogit, nullptr);
+            float sh[48];
+            const float* row = a.shs + 48 * j;
+            if (wide) {
+#pragma unroll
+                for (int k = 0; k < 12; k++) {
+                    const float4 r = __ldg(reinterpret_cast<const float4*>(row) + k);
+                    sh[4 * k] = r.x;
+                    sh[4 * k + 1] = r.y;
+                    sh[4 * k + 2] = r.z;
+                    sh[4 * k + 3] = r.w;
+                }
+            } else {
+#pragma unroll
+                for (int k = 0; k < 48; k++) sh[k] = __ldg(row + k);
+            }
+            gsr_adj::color_adjoint(m, a.cam[v].campos, sh, grgb, gm, g);
+            float* o = s_out[tid];
+            for (int k = 0; k < 3; k++) {
+                o[k] = gm[k];
+                o[3 + k] = gls[k];
+                o[11 + k] = g[k];
+            }
+            for (int k = 0; k < 4; k++) o[6 + k] = gq[k];
+            o[10] = glogit;
         }
-        gsr_adj::Fwd<float> f;
-        gsr_adj::Tape<float> tp;
-        gsr_adj::forward(m, ls, q, logit, sh, a.cam[v], f, tp);
-        float vm[3], vls[3], vq[4], vlogit;
-        gsr_adj::backward<float, true>(m, sh, a.cam[v], tp, gxy, gcon, grgb, vm, vls, vq, vlogit, gsh);
-        for (int k = 0; k < 3; k++) {
-            gm[k] += vm[k];
-            gls[k] += vls[k];
+        __syncthreads();
+
+        // ---- each Gaussian's sum over its views ----
+        if (mine) {
+            float sum[11], sh[48], m[3];
+            for (int k = 0; k < 11; k++) sum[k] = 0.f;
+            for (int k = 0; k < 48; k++) sh[k] = 0.f;
+            for (int k = 0; k < 3; k++) m[k] = __ldg(a.means + 3 * (size_t)i + k);
+            for (int k = first; k < first + n; k++) {
+                const float* o = s_out[k - begin];
+                for (int c = 0; c < 11; c++) sum[c] += o[c];
+                const float* campos = a.cam[s_pair[k] >> 8].campos;
+                float d[3] = {m[0] - campos[0], m[1] - campos[1], m[2] - campos[2]};
+                const float len = sqrtf(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
+                float B[16], dB[16][3];
+                gsr_adj::sh_basis(d[0] / len, d[1] / len, d[2] / len, B, dB);
+                for (int c = 0; c < 16; c++)
+                    for (int ch = 0; ch < 3; ch++) sh[3 * c + ch] += B[c] * o[11 + ch];
+            }
+            auto put = [&](float* dst, size_t off, float v) { dst[off] = a.accumulate ? dst[off] + v : v; };
+            for (int k = 0; k < 3; k++) {
+                put(a.g_means, 3 * (size_t)i + k, sum[k]);
+                put(a.g_log_scales, 3 * (size_t)i + k, sum[3 + k]);
+            }
+            for (int k = 0; k < 4; k++) put(a.g_quats, 4 * (size_t)i + k, sum[6 + k]);
+            put(a.g_logits, i, sum[10]);
+            if (wide && !a.accumulate) {
+                float4* row = reinterpret_cast<float4*>(a.g_shs + 48 * (size_t)i);
+#pragma unroll
+                for (int k = 0; k < 12; k++)
+                    row[k] = make_float4(sh[4 * k], sh[4 * k + 1], sh[4 * k + 2], sh[4 * k + 3]);
+            } else {
+                for (int k = 0; k < 48; k++) put(a.g_shs, 48 * (size_t)i + k, sh[k]);
+            }
         }
-        for (int k = 0; k < 4; k++) gq[k] += vq[k];
-        glogit += vlogit;
+        begin = end;
     }
-    if (!loaded && a.accumulate) return;
-    auto put = [&](float* dst, size_t off, float v) { dst[off] = a.accumulate ? dst[off] + v : v; };
-    for (int k = 0; k < 3; k++) {
-        put(a.g_means, 3 * (size_t)i + k, gm[k]);
-        put(a.g_log_scales, 3 * (size_t)i + k, gls[k]);
-    }
-    for (int k = 0; k < 4; k++) put(a.g_quats, 4 * (size_t)i + k, gq[k]);
-    put(a.g_logits, i, glogit);
-    for (int k = 0; k < 48; k++) put(a.g_shs, 48 * (size_t)i + k, gsh[k]);
 }
 
 gsr_adj::Cam<float> adj_camera(int W, int H, const float* cam_pos, const float* cam_rot, float fx, float fy,
@@ -274,14 +339,15 @@ gsr_status gsr_train_backward(int P, const float* means, const float* log_scales
     ra.grad_con = grad_con;
     ra.grad_rgb = grad_rgb;
     if ((e = launch_render_train(ra, true, s)) != cudaSuccess) return GSR_CUDA_ERROR;
-    PreBackArgs pa;
+    PreBackArgs pa = {};
     pa.P = P;
+    pa.n_views = 1;
     pa.means = means;
     pa.log_scales = log_scales;
     pa.quats = quats;
     pa.logits = logits;
     pa.shs = shs;
-    pa.cam = adj_camera(width, height, cam_pos, cam_rot, focal_x, focal_y, z_far, z_near);
+    pa.cam[0] = adj_camera(width, height, cam_pos, cam_rot, focal_x, focal_y, z_far, z_near);
     pa.gxy = grad_xy;
     pa.gcon = grad_con;
     pa.grgb = grad_rgb;
@@ -291,7 +357,7 @@ gsr_status gsr_train_backward(int P, const float* means, const float* log_scales
     pa.g_logits = g_logits;
     pa.g_shs = g_shs;
     pa.accumulate = accumulate;
-    k_preprocess_backward<<<div_up(P, 128), 128, 0, s>>>(pa);
+    k_preprocess_backward<false><<<div_up(P, kAdjThreads), kAdjThreads, 0, s>>>(pa);
     return cudaGetLastError() == cudaSuccess ? GSR_OK : GSR_CUDA_ERROR;
 }
 
@@ -443,7 +509,7 @@ gsr_status gsr_train_backward_views(int P, const float* means, const float* log_
     ra.grad_rec = grad_feat;
     if ((e = launch_render_train(ra, true, s)) != cudaSuccess) return GSR_CUDA_ERROR;
     for (int v0 = 0; v0 < n_views; v0 += kAdjViews) {
-        PreBackViewsArgs pa;
+        PreBackArgs pa = {};
         pa.P = P;
         pa.n_views = std::min(kAdjViews, n_views - v0);
         pa.means = means;
@@ -464,7 +530,7 @@ gsr_status gsr_train_backward_views(int P, const float* means, const float* log_
         pa.g_logits = g_logits;
         pa.g_shs = g_shs;
         pa.accumulate = (accumulate || v0 > 0) ? 1 : 0;
-        k_preprocess_backward_views<<<div_up(P, 128), 128, 0, s>>>(pa);
+        k_preprocess_backward<true><<<div_up(P, kAdjThreads), kAdjThreads, 0, s>>>(pa);
         if (cudaGetLastError() != cudaSuccess) return GSR_CUDA_ERROR;
     }
     return GSR_OK;
