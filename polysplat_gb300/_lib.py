@@ -25,6 +25,7 @@ RENDER_RANGES_CADENCE2 = 3
 RENDER_DT = 4
 RENDER_SPLIT = 5
 QUAD_KEYS = 0x100  # GSR_QUAD_KEYS: one key per 2x2 group of 16x16 tiles
+EXPAND_QUADS = 0x200  # GSR_EXPAND_QUADS: sort those, write per-tile lists
 
 
 class GsrError(RuntimeError):

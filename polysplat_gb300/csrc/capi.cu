@@ -103,6 +103,7 @@ gsr_status preprocess_params(PreprocessParams& p, int P, const float* pos, const
     p.huge_area = kDefaultHugeArea;
     p.quad = 0;
     p.interleave = 0;
+    p.pair_count = nullptr;
     p.P = P;
     p.pos = pos;
     p.shs = shs;
@@ -269,7 +270,8 @@ static gsr_status preprocess_impl(int P, const float* pos, const void* shs, int 
                                   const float* cam_pos, const float* cam_rot, float fx, float fy, float zfar,
                                   float znear, float* points_xy, float* rgb_depth, float* conic_opacity,
                                   uint64_t* keys, uint32_t* values, int64_t cap, int32_t* curr_offset,
-                                  void* workspace, size_t workspace_bytes, cudaStream_t s, bool quad = false)
+                                  void* workspace, size_t workspace_bytes, cudaStream_t s, bool quad = false,
+                                  unsigned long long* pair_count = nullptr)
 {
     PreprocessParams p;
     const gsr_status st = preprocess_params(p, P, pos, shs, opacity, cov3d, width, height, block_x, block_y, cam_pos,
@@ -277,6 +279,7 @@ static gsr_status preprocess_impl(int P, const float* pos, const void* shs, int 
                                             values, cap, curr_offset, workspace, workspace_bytes);
     if (st != GSR_OK) return st;
     p.quad = quad ? 1 : 0;
+    p.pair_count = pair_count;
     return from_cuda(launch_preprocess(p, shs_half != 0, s));
 }
 
@@ -414,7 +417,9 @@ gsr_status gsr_forward(int variant, int P, const float* pos, const void* shs, in
     cudaStream_t s = (cudaStream_t)stream;
     // GSR_QUAD_KEYS: one key per 2x2 group of 16x16 tiles, same image
     const bool quad = (variant & GSR_QUAD_KEYS) != 0;
-    variant &= ~GSR_QUAD_KEYS;
+    // GSR_EXPAND_QUADS: quad keys sorted, per-tile lists out (expand.cu)
+    const bool may_expand = (variant & GSR_EXPAND_QUADS) != 0 && !quad;
+    variant &= ~(GSR_QUAD_KEYS | GSR_EXPAND_QUADS);
     if (!workspace || !curr_offset || !valid_tile_shape(block_x, block_y)) return GSR_INVALID_ARG;
     if (quad && (block_x != 16 || block_y != 16 || variant == GSR_RENDER_SPLIT || P > (int)kQuadGidMask))
         return GSR_INVALID_ARG;
@@ -425,6 +430,61 @@ gsr_status gsr_forward(int variant, int P, const float* pos, const void* shs, in
     if (e == cudaSuccess) e = cudaMemsetAsync(curr_offset, 0, sizeof(int32_t), s);
     if (e != cudaSuccess) return from_cuda(e);
     profile_mark(s);
+    const int tiles16 = width > 0 && height > 0 ? tiles_of(width, height, 16, 16) : 0;
+    const bool expand = may_expand && tiles16 > 0 && block_x == 16 && block_y == 16 && variant >= 0 &&
+                        variant < GSR_RENDER_SPLIT && P > 0 && P <= (int)kQuadGidMask && key_capacity < (1LL << 30) &&
+                        (ranges || tiles16 <= kWorkspaceRangeTiles) && keys_unsorted && values_unsorted &&
+                        keys_sorted && values_sorted && keys_unsorted != keys_sorted &&
+                        values_unsorted != values_sorted &&
+                        (size_t)key_capacity * sizeof(uint64_t) >=
+                            expand_scratch_bytes(div_up(width, 16), div_up(height, 16));
+    if (expand) {
+        WorkspaceHeader* h = reinterpret_cast<WorkspaceHeader*>(workspace);
+        gsr_status st = preprocess_impl(P, pos, shs, shs_half, opacity, cov3d, width, height, 16, 16, cam_pos, cam_rot,
+                                        focal_x, focal_y, z_far, z_near, points_xy, rgb_depth, conic_opacity,
+                                        keys_unsorted, values_unsorted, key_capacity, curr_offset, workspace,
+                                        workspace_bytes, s, true, &h->pair_count);
+        if (st != GSR_OK) return st;
+        profile_mark(s);
+        // the digit passes go back and forth between the caller's sorted arrays
+        // and the workspace, and end in the workspace
+        const int gx = div_up(width, 16), gy = div_up(height, 16);
+        SortScratch sc = workspace_sort_scratch(workspace, key_capacity);
+        uint64_t* quad_keys = reinterpret_cast<uint64_t*>(sc.alt_keys);
+        uint32_t* quad_vals = sc.alt_vals;
+        sc.alt_keys = keys_sorted;
+        sc.alt_vals = values_sorted;
+        OrderMap order;
+        order.kind = kOrderDepthCompressed64;
+        order.end_bit = 32 + bits_for((uint32_t)(quad_cols(gx) * quad_cols(gy)));
+        order.tile_from_bit = 32;
+        const int passes = (order.end_bit + 7) / 8;
+        e = launch_sort64(0, reinterpret_cast<const int32_t*>(&h->pair_count), key_capacity, order, passes,
+                          keys_unsorted, values_unsorted, quad_keys, quad_vals, sc, s);
+        if (e != cudaSuccess) return from_cuda(e);
+        // a recorded frame has one stage per digit pass of the per-tile order
+        for (int p = passes; p < (32 + (int)bits_for((uint32_t)tiles16) + 7) / 8; p++) profile_mark(s);
+        if (!ranges) ranges = reinterpret_cast<int32_t*>(workspace_ranges(workspace, key_capacity));
+        ExpandArgs x;
+        x.keys = quad_keys;
+        x.vals = quad_vals;
+        x.count = &h->pair_count;
+        x.cap = key_capacity;
+        x.gx = gx;
+        x.gy = gy;
+        x.scratch = keys_unsorted;
+        x.scratch_bytes = (size_t)key_capacity * sizeof(uint64_t);
+        x.out_keys = keys_sorted;
+        x.out_vals = values_sorted;
+        x.ranges = reinterpret_cast<int2*>(ranges);
+        x.total = curr_offset;
+        if ((e = launch_quad_expand(x, s)) != cudaSuccess) return from_cuda(e);
+        profile_mark(s);
+        st = render_impl(variant, 0, curr_offset, key_capacity, width, height, 16, 16, P, points_xy, rgb_depth,
+                         conic_opacity, keys_sorted, values_sorted, ranges, bg_color, out_color, workspace, s);
+        if (st == GSR_OK) profile_mark(s);
+        return st;
+    }
     gsr_status st = preprocess_impl(P, pos, shs, shs_half, opacity, cov3d, width, height, block_x, block_y, cam_pos,
                                     cam_rot, focal_x, focal_y, z_far, z_near, points_xy, rgb_depth, conic_opacity,
                                     keys_unsorted, values_unsorted, key_capacity, curr_offset, workspace,

@@ -86,6 +86,9 @@ struct PreprocessParams {
     // views' blocks over one range of Gaussians run side by side and the
     // range's parameters come from DRAM once and from L2 for the other views.
     int interleave = 0;
+    // Quad keys that are expanded to per-tile lists after the sort: counts the
+    // keys (low half) and the hit tiles (high half) in place of `counter`.
+    unsigned long long* pair_count = nullptr;
 };
 // Quad keys: bit (x & 1) | (y & 1) << 1 of value >> kQuadShift is set when
 // the Gaussian hits tile (x, y) of the quad, by the same exact tile test the
@@ -143,13 +146,15 @@ struct WorkspaceHeader {
     uint32_t mq_count[2];     // massive-Gaussian queue: entries pushed per class
     uint32_t mq_head[2][2];   // massive-Gaussian queue: entries taken per pass and class
     uint32_t depth_hi;        // largest depth bit pattern of an emitting Gaussian
-    uint32_t pad[7];
+    uint32_t pad0;
+    unsigned long long pair_count;  // quad keys emitted | hit tiles << 32 (PreprocessParams::pair_count)
+    uint32_t pad[4];
     // sort region (cleared by every sort)
     uint32_t pass_counter[8]; // per radix pass tile counter
     uint32_t hist[8][256];    // per-pass digit histograms
 };
 constexpr size_t kPreprocessRegionOffset = 2 * sizeof(uint32_t);
-constexpr size_t kPreprocessRegionBytes = 7 * sizeof(uint32_t);
+constexpr size_t kPreprocessRegionBytes = 10 * sizeof(uint32_t);
 constexpr size_t kSortRegionOffset = 16 * sizeof(uint32_t);
 constexpr size_t kHeaderBytes = 16384;
 static_assert(sizeof(WorkspaceHeader) <= kHeaderBytes, "header too large");
@@ -247,6 +252,25 @@ cudaError_t launch_tile_ranges32(const int32_t* d_num, long long cap, int tiles,
 cudaError_t launch_gather(int num, const int32_t* d_num, const uint32_t* values, const float2* sxy,
                           const float4* srgbd, const float4* scon, float2* dxy, float4* drgbd, float4* dcon,
                           long long cap, cudaStream_t stream);
+
+// Per-tile lists and ranges of a gx x gy grid of 16x16 tiles from sorted quad
+// keys (expand.cu).  `count` is PreprocessParams::pair_count's word; its high
+// half goes to `total`.
+struct ExpandArgs {
+    const uint64_t* keys;
+    const uint32_t* vals;
+    const unsigned long long* count;
+    long long cap;  // of both key buffers
+    int gx, gy;
+    void* scratch;
+    size_t scratch_bytes;
+    uint64_t* out_keys;
+    uint32_t* out_vals;
+    int2* ranges;
+    int32_t* total;
+};
+size_t expand_scratch_bytes(int gx, int gy);
+cudaError_t launch_quad_expand(const ExpandArgs& e, cudaStream_t stream);
 
 struct RenderArgs {
     int variant;

@@ -186,10 +186,13 @@ constexpr int kWarps = 8;
 constexpr int kThreads = kWarps * 32;
 constexpr int kStage = 256;
 
+// HITS (quad keys of one view): the tiles the keys name are counted too.
+template <bool HITS>
 struct Stage {
     uint64_t* k;
     uint32_t* v;
     int fill;
+    uint32_t hits = 0;  // HITS: hit tiles of the quad keys this lane appended
 };
 
 struct EmitOut {
@@ -197,13 +200,24 @@ struct EmitOut {
     uint32_t* vals;
     long long cap;
     int* counter;
+    unsigned long long* pairs;  // PreprocessParams::pair_count
 };
 
-__device__ __forceinline__ void stage_flush(Stage& s, const EmitOut& o, unsigned lane)
+// Reserve n slots of the key buffer, and add `hits` to the hit tiles where
+// those are counted.
+template <bool HITS>
+__device__ __forceinline__ int reserve_keys(const EmitOut& o, int n, uint32_t hits)
+{
+    if (HITS && o.pairs) return (int)(uint32_t)atomicAdd(o.pairs, (unsigned long long)hits << 32 | (uint32_t)n);
+    return atomicAdd(o.counter, n);
+}
+
+template <bool HITS>
+__device__ __forceinline__ void stage_flush(Stage<HITS>& s, const EmitOut& o, unsigned lane)
 {
     __syncwarp();
     int base = 0;
-    if (lane == 0) base = atomicAdd(o.counter, s.fill);
+    if (lane == 0) base = reserve_keys<HITS>(o, s.fill, 0u);
     base = __shfl_sync(GSR_FULL_MASK, base, 0);
     for (int i = lane; i < s.fill; i += 32) {
         long long pos = (long long)base + i;
@@ -216,7 +230,8 @@ __device__ __forceinline__ void stage_flush(Stage& s, const EmitOut& o, unsigned
     s.fill = 0;
 }
 
-__device__ __forceinline__ void stage_emit(Stage& s, const EmitOut& o, bool valid, uint64_t key, uint32_t val,
+template <bool HITS>
+__device__ __forceinline__ void stage_emit(Stage<HITS>& s, const EmitOut& o, bool valid, uint64_t key, uint32_t val,
                                            unsigned lane)
 {
     unsigned mask = __ballot_sync(GSR_FULL_MASK, valid);
@@ -227,6 +242,7 @@ __device__ __forceinline__ void stage_emit(Stage& s, const EmitOut& o, bool vali
         int slot = s.fill + __popc(mask & lanemask_lt());
         s.k[slot] = key;
         s.v[slot] = val;
+        if (HITS) s.hits += __popc(val >> kQuadShift);
     }
     s.fill += n;
 }
@@ -247,9 +263,14 @@ constexpr int kPoolArea = 128;
 // Block-wide final flush of every warp's staged keys with one atomic per CTA:
 // the reservation, whose round trip the preprocess hides behind its colours,
 // and the copy.
-__device__ __forceinline__ void block_reserve(const Stage& st, const EmitOut& out, int* s_fill, long long* s_base,
-                                              unsigned lane, int warp)
+template <bool HITS>
+__device__ __forceinline__ void block_reserve(const Stage<HITS>& st, const EmitOut& out, int* s_fill,
+                                              long long* s_base, unsigned lane, int warp)
 {
+    if (HITS && out.pairs) {
+        const uint32_t h = __reduce_add_sync(GSR_FULL_MASK, st.hits);
+        if (lane == 0) s_base[warp] = h;
+    }
     if (lane == 0) s_fill[warp] = st.fill;
     __syncthreads();
     if (warp == 0) {
@@ -261,14 +282,17 @@ __device__ __forceinline__ void block_reserve(const Stage& st, const EmitOut& ou
             if ((int)lane >= d) incl += n;
         }
         int total = __shfl_sync(GSR_FULL_MASK, incl, 31);
+        uint32_t hits = 0;
+        if (HITS && out.pairs) hits = __reduce_add_sync(GSR_FULL_MASK, lane < kWarps ? (uint32_t)s_base[lane] : 0u);
         long long base = 0;
-        if (lane == 0 && total > 0) base = atomicAdd(out.counter, total);
+        if (lane == 0 && (total > 0 || hits > 0)) base = reserve_keys<HITS>(out, total, hits);
         base = __shfl_sync(GSR_FULL_MASK, base, 0);
         if (lane < kWarps) s_base[lane] = base + incl - f;
     }
 }
 
-__device__ __forceinline__ void block_copy(Stage& st, const EmitOut& out, const long long* s_base, unsigned lane,
+template <bool HITS>
+__device__ __forceinline__ void block_copy(Stage<HITS>& st, const EmitOut& out, const long long* s_base, unsigned lane,
                                            int warp)
 {
     __syncthreads();
@@ -374,8 +398,8 @@ __global__ __launch_bounds__(kThreads, VIEWS ? 6 : 5) void k_preprocess(const __
             point_valid = (rect_max.x - rect_min.x) * (rect_max.y - rect_min.y) > 0;
         } while (false);
     }
-    Stage st{s_keys[COUNT ? 0 : warp], s_vals[COUNT ? 0 : warp], 0};
-    const EmitOut out{a.keys, a.vals, a.cap, a.counter};
+    Stage<QUAD && !VIEWS> st{s_keys[COUNT ? 0 : warp], s_vals[COUNT ? 0 : warp], 0};
+    const EmitOut out{a.keys, a.vals, a.cap, a.counter, a.pair_count};
     if (lane == 0) s_hit[warp] = 0u;
     s_cnt[warp][lane] = 0u;
     __syncwarp();
@@ -834,8 +858,8 @@ __global__ __launch_bounds__(kThreads, 4) void k_emit_massive(const __grid_const
     __shared__ int s_rows[kWarps];                 // rows listed
     const unsigned lane = threadIdx.x & 31u;
     const int warp = threadIdx.x >> 5;
-    Stage st{s_keys[MODE == kMassiveEmit64 ? warp : 0], s_vals[MODE == kMassiveEmit64 ? warp : 0], 0};
-    const EmitOut out{a.keys, a.vals, a.cap, a.counter};
+    Stage<QUAD && !VIEWS> st{s_keys[MODE == kMassiveEmit64 ? warp : 0], s_vals[MODE == kMassiveEmit64 ? warp : 0], 0};
+    const EmitOut out{a.keys, a.vals, a.cap, a.counter, a.pair_count};
     uint32_t* head = a.mq.head + (MODE == kMassiveEmitDf ? 2 : 0);
     const int n_huge = (int)min(a.mq.count[0], (uint32_t)a.mq.huge_capacity);
     const int n_large = (int)min(a.mq.count[1], (uint32_t)(a.mq.capacity - a.mq.huge_capacity));

@@ -17,6 +17,7 @@ import os
 import numpy as np
 import torch
 
+from . import _lib as R
 from . import ops
 
 
@@ -182,9 +183,23 @@ class Rasterizer:
             return False
         return P > self._es_threshold_N_firstcall
 
+    def _expand_quads(self, scene):
+        """Whether the fused forward sorts one key per 2x2 group of tiles and
+        expands them to per-tile lists, going by the last frame's key count M
+        (a first frame sorts per-tile keys; the results are the same): the
+        digit passes move fewer pairs, three more kernels write all M.
+
+        The line, frame times sorting per tile and expanding (us):
+          M 9.5 M = 3.2 P   754 / 612      M 5.2 M = 1.7 P   556 / 512
+          M 2.0 M = 2.0 P   353 / 332      M 1.5 M = 3.1 P   314 / 310
+          M 3.7 M = 1.2 P   489 / 477      M 26 M = 1.3 P   4267 / 4328
+          M 2.6 M = 1.3 P   719 / 750      M 0.3 M = 3.3 P   259 / 278
+        Below 1.5 P most Gaussians hit one tile of a quad."""
+        M = self._es_last_M
+        return M is not None and M >= 1_500_000 and M >= 1.5 * scene.num_vertex
+
     @staticmethod
     def _df_variant(render_variant):
-        from . import _lib as R
         if render_variant.endswith("_dt"):
             return R.RENDER_DT
         if render_variant == LITE or render_variant.startswith("preranges_smem_persistent"):
@@ -235,18 +250,16 @@ class Rasterizer:
             used_es = True
             fused = lambda: self._forward_depth_first(scene, args_cam, render_variant, bg_color, out)
         elif not measuring:
-            if render_variant == E2E:
-                fused = lambda: ops.forward_fused_e2e(scene.position, scene.shs_half, scene.opacity, scene.cov3d,
-                                                      *args_cam, self.curr_offset, self.list_sorting_space, *bufs,
-                                                      *feats, bg_color, out)
-            elif render_variant == E2E_PRERANGES:
-                fused = lambda: ops.forward_fused_e2e_preranges(
-                    scene.position, scene.shs_half, scene.opacity, scene.cov3d, *args_cam, self.curr_offset,
-                    self.list_sorting_space, *bufs, *feats, self.tile_ranges_buf, bg_color, out)
-            elif render_variant in ("default", "unroll2", "split"):
-                fused = lambda: ops.forward_fused(scene.position, scene.shs, scene.opacity, scene.cov3d,
-                                                  *args_cam[:4], *args_cam[4:], render_variant, self.curr_offset,
-                                                  self.list_sorting_space, *bufs, *feats, bg_color, out)
+            code = {E2E: R.RENDER_PERSISTENT_FUSED, E2E_PRERANGES: R.RENDER_PERSISTENT_RANGES, "default": R.RENDER_DEFAULT,
+                    "unroll2": R.RENDER_DEFAULT, "split": R.RENDER_DEFAULT}.get(render_variant)
+            if code is not None:
+                half = render_variant in (E2E, E2E_PRERANGES)
+                if self._expand_quads(scene):
+                    code |= R.EXPAND_QUADS
+                ranges = self.tile_ranges_buf if render_variant == E2E_PRERANGES else None
+                fused = lambda: ops._forward(code, half, scene.position, scene.shs_half if half else scene.shs,
+                                             scene.opacity, scene.cov3d, *args_cam, self.curr_offset,
+                                             self.list_sorting_space, *bufs, *feats, ranges, bg_color, out)
         if fused is not None:
             num = fused()
             self._es_last_M = num
@@ -331,8 +344,7 @@ class Rasterizer:
         elif variant.startswith("preranges") or variant.startswith("reordered"):
             ops.render_16x16_preranges(num, W, H, xy, rgbd, con, vals, rb, bg, out)
         else:
-            from ._lib import RENDER_DEFAULT
-            ops._render(RENDER_DEFAULT, num, W, H, xy, rgbd, con, ks, vals, None, bg, out, bx, by)
+            ops._render(R.RENDER_DEFAULT, num, W, H, xy, rgbd, con, ks, vals, None, bg, out, bx, by)
 
     @staticmethod
     def _stats(requested, variant, bx, by, num, pre, srt, ren, used_es):
