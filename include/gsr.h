@@ -65,10 +65,11 @@ typedef enum {
  * buffers then hold quad keys, not the reference's per-tile keys. */
 #define GSR_QUAD_KEYS 0x100
 
-/* Or-ed into the variant of gsr_forward: it may sort quad keys and expand them
- * to per-tile lists before the render.  The sorted arrays, ranges, key count
- * and image are those of the call without the flag (pairs of equal key in any
- * order, as there); the unsorted arrays are scratch.  It does so for 16x16
+/* Or-ed into the variant of gsr_forward or gsr_forward_depth_first: the call
+ * may sort quad keys and expand them to per-tile lists before the render.  The
+ * sorted arrays, ranges, key count and image are those of the call without the
+ * flag (gsr_forward: pairs of equal key in any order, as there); the unsorted
+ * arrays are scratch.  It does so for 16x16
  * tiles, P below 2^28 and a key buffer that holds a few words per tile, and
  * ignores the flag otherwise.  It pays where Gaussians span several tiles:
  * polysplat_gb300/rasterizer.py has the measured line. */

@@ -406,6 +406,37 @@ gsr_status gsr_render(int variant, int num, const int32_t* d_num, int width, int
                        out_color, workspace, (cudaStream_t)stream);
 }
 
+// Whether a frame can sort quad keys and expand them: the shapes quad keys
+// take, and an unsorted key buffer that holds the expansion's arrays.
+static bool expand_fits(int variant, int P, int width, int height, int block_x, int block_y, int64_t key_capacity,
+                        size_t key_bytes)
+{
+    return block_x == 16 && block_y == 16 && variant >= 0 && variant < GSR_RENDER_SPLIT && P > 0 &&
+           P <= (int)kQuadGidMask && key_capacity > 0 && key_capacity < (1LL << 30) &&
+           (size_t)key_capacity * key_bytes >= expand_scratch_bytes(div_up(width, 16), div_up(height, 16));
+}
+
+static ExpandArgs expand_args(size_t key_bytes, const void* keys, const uint32_t* vals, WorkspaceHeader* h,
+                              int64_t key_capacity, int gx, int gy, void* unsorted, void* out_keys, uint32_t* out_vals,
+                              int32_t* ranges, int32_t* curr_offset)
+{
+    ExpandArgs x;
+    x.key_bytes = (int)key_bytes;
+    x.keys = keys;
+    x.vals = vals;
+    x.count = &h->pair_count;
+    x.cap = key_capacity;
+    x.gx = gx;
+    x.gy = gy;
+    x.scratch = unsorted;
+    x.scratch_bytes = (size_t)key_capacity * key_bytes;
+    x.out_keys = out_keys;
+    x.out_vals = out_vals;
+    x.ranges = reinterpret_cast<int2*>(ranges);
+    x.total = curr_offset;
+    return x;
+}
+
 gsr_status gsr_forward(int variant, int P, const float* pos, const void* shs, int shs_half, const float* opacity,
                        const float* cov3d, int width, int height, int block_x, int block_y, const float* cam_pos,
                        const float* cam_rot, float focal_x, float focal_y, float z_far, float z_near,
@@ -431,13 +462,10 @@ gsr_status gsr_forward(int variant, int P, const float* pos, const void* shs, in
     if (e != cudaSuccess) return from_cuda(e);
     profile_mark(s);
     const int tiles16 = width > 0 && height > 0 ? tiles_of(width, height, 16, 16) : 0;
-    const bool expand = may_expand && tiles16 > 0 && block_x == 16 && block_y == 16 && variant >= 0 &&
-                        variant < GSR_RENDER_SPLIT && P > 0 && P <= (int)kQuadGidMask && key_capacity < (1LL << 30) &&
-                        (ranges || tiles16 <= kWorkspaceRangeTiles) && keys_unsorted && values_unsorted &&
-                        keys_sorted && values_sorted && keys_unsorted != keys_sorted &&
+    const bool expand = may_expand && tiles16 > 0 && (ranges || tiles16 <= kWorkspaceRangeTiles) && keys_unsorted &&
+                        values_unsorted && keys_sorted && values_sorted && keys_unsorted != keys_sorted &&
                         values_unsorted != values_sorted &&
-                        (size_t)key_capacity * sizeof(uint64_t) >=
-                            expand_scratch_bytes(div_up(width, 16), div_up(height, 16));
+                        expand_fits(variant, P, width, height, block_x, block_y, key_capacity, sizeof(uint64_t));
     if (expand) {
         WorkspaceHeader* h = reinterpret_cast<WorkspaceHeader*>(workspace);
         gsr_status st = preprocess_impl(P, pos, shs, shs_half, opacity, cov3d, width, height, 16, 16, cam_pos, cam_rot,
@@ -465,19 +493,8 @@ gsr_status gsr_forward(int variant, int P, const float* pos, const void* shs, in
         // a recorded frame has one stage per digit pass of the per-tile order
         for (int p = passes; p < (32 + (int)bits_for((uint32_t)tiles16) + 7) / 8; p++) profile_mark(s);
         if (!ranges) ranges = reinterpret_cast<int32_t*>(workspace_ranges(workspace, key_capacity));
-        ExpandArgs x;
-        x.keys = quad_keys;
-        x.vals = quad_vals;
-        x.count = &h->pair_count;
-        x.cap = key_capacity;
-        x.gx = gx;
-        x.gy = gy;
-        x.scratch = keys_unsorted;
-        x.scratch_bytes = (size_t)key_capacity * sizeof(uint64_t);
-        x.out_keys = keys_sorted;
-        x.out_vals = values_sorted;
-        x.ranges = reinterpret_cast<int2*>(ranges);
-        x.total = curr_offset;
+        const ExpandArgs x = expand_args(sizeof(uint64_t), quad_keys, quad_vals, h, key_capacity, gx, gy, keys_unsorted,
+                                         keys_sorted, values_sorted, ranges, curr_offset);
         if ((e = launch_quad_expand(x, s)) != cudaSuccess) return from_cuda(e);
         profile_mark(s);
         st = render_impl(variant, 0, curr_offset, key_capacity, width, height, 16, 16, P, points_xy, rgb_depth,
@@ -528,7 +545,9 @@ gsr_status gsr_forward_depth_first(int variant, int P, const float* pos, const v
     cudaStream_t s = (cudaStream_t)stream;
     // GSR_QUAD_KEYS: the pairs name 2x2 groups of 16x16 tiles, same image
     const bool quad = (variant & GSR_QUAD_KEYS) != 0;
-    variant &= ~GSR_QUAD_KEYS;
+    // GSR_EXPAND_QUADS: quad pairs sorted, per-tile lists out (expand.cu)
+    const bool may_expand = (variant & GSR_EXPAND_QUADS) != 0 && !quad;
+    variant &= ~(GSR_QUAD_KEYS | GSR_EXPAND_QUADS);
     if (!workspace || !curr_offset || !scene_scratch || !valid_tile_shape(block_x, block_y)) return GSR_INVALID_ARG;
     if (variant < 0 || variant > GSR_RENDER_SPLIT) return GSR_INVALID_ARG;
     if (quad && (block_x != 16 || block_y != 16 || variant == GSR_RENDER_SPLIT || P > (int)kQuadGidMask))
@@ -541,6 +560,8 @@ gsr_status gsr_forward_depth_first(int variant, int P, const float* pos, const v
     // pair tile ids: tiles, or quads
     const int tiles = quad ? quad_cols(div_up(width, 16)) * quad_cols(div_up(height, 16))
                            : tiles_of(width, height, block_x, block_y);
+    const bool expand = may_expand && width > 0 && height > 0 &&
+                        expand_fits(variant, P, width, height, block_x, block_y, key_capacity, sizeof(uint32_t));
     if (!ranges) {
         if (tiles > kWorkspaceRangeTiles) return GSR_INVALID_ARG;
         ranges = reinterpret_cast<int32_t*>(workspace_ranges(workspace, key_capacity));
@@ -552,16 +573,33 @@ gsr_status gsr_forward_depth_first(int variant, int P, const float* pos, const v
                                       reinterpret_cast<uint64_t*>(tiles_unsorted), values_unsorted, key_capacity,
                                       curr_offset, workspace, workspace_bytes);
     if (st != GSR_OK) return st;
-    p.quad = quad ? 1 : 0;
+    p.quad = quad || expand ? 1 : 0;
     profile_frame_begin();
     cudaError_t e = cudaMemsetAsync(workspace, 0, sizeof(uint32_t), s);  // status word
     if (e == cudaSuccess) e = cudaMemsetAsync(curr_offset, 0, sizeof(int32_t), s);
     if (e != cudaSuccess) return from_cuda(e);
     profile_mark(s);
-    e = launch_depth_first(p, shs_half != 0, scene_scratch, scene_scratch_bytes,
-                           reinterpret_cast<WorkspaceHeader*>(workspace), workspace_sort_scratch(workspace, key_capacity),
-                           tiles, tiles_unsorted, values_unsorted, tiles_sorted, values_sorted,
-                           reinterpret_cast<int2*>(ranges), s);
+    WorkspaceHeader* h = reinterpret_cast<WorkspaceHeader*>(workspace);
+    SortScratch sc = workspace_sort_scratch(workspace, key_capacity);
+    if (expand) {
+        // the quad count goes to the low half of pair_count, the hit tiles of
+        // the counting pass to its high half; the sort ends in the workspace
+        const int gx = div_up(width, 16), gy = div_up(height, 16);
+        uint32_t *quad_ids = reinterpret_cast<uint32_t*>(sc.alt_keys), *quad_vals = sc.alt_vals;
+        sc.alt_keys = tiles_sorted;
+        sc.alt_vals = values_sorted;
+        p.pair_count = &h->pair_count;
+        p.counter = reinterpret_cast<int*>(&h->pair_count);
+        const ExpandArgs x = expand_args(sizeof(uint32_t), quad_ids, quad_vals, h, key_capacity, gx, gy, tiles_unsorted,
+                                         tiles_sorted, values_sorted, ranges, curr_offset);
+        e = launch_depth_first(p, shs_half != 0, scene_scratch, scene_scratch_bytes, h, sc,
+                               quad_cols(gx) * quad_cols(gy), tiles_unsorted, values_unsorted, quad_ids, quad_vals,
+                               nullptr, &x, s);
+    } else {
+        e = launch_depth_first(p, shs_half != 0, scene_scratch, scene_scratch_bytes, h, sc, tiles, tiles_unsorted,
+                               values_unsorted, tiles_sorted, values_sorted, reinterpret_cast<int2*>(ranges), nullptr,
+                               s);
+    }
     if (e != cudaSuccess) return from_cuda(e);
     st = render_impl(variant, 0, curr_offset, key_capacity, width, height, block_x, block_y, P, points_xy, rgb_depth,
                      conic_opacity, nullptr, values_sorted, ranges, bg_color, out_color, workspace, s, quad);

@@ -19,6 +19,8 @@
 //      (preprocess.cu, with the counting pass's tile test);
 //   6. stable radix sort of the 32-bit tile ids (2 passes at 1080p instead of
 //      5 over 12-byte pairs), then tile ranges from the sorted ids.
+// With GSR_EXPAND_QUADS steps 1 and 5 handle 2x2 groups of tiles, step 6 sorts
+// their ids, and expand.cu writes the per-tile pairs and ranges in that order.
 // Pairs with the same tile and the same depth bits come out in Gaussian
 // index order (the reference's order there depends on its atomics).
 #include <algorithm>
@@ -270,7 +272,7 @@ static DfLayout df_layout(void* scratch, int P)
 cudaError_t launch_depth_first(const PreprocessParams& p0, bool half_sh, void* scratch, size_t scratch_bytes,
                                WorkspaceHeader* hdr, const SortScratch& tile_sort, int tiles, uint32_t* tile_keys_in,
                                uint32_t* vals_in, uint32_t* tile_keys_out, uint32_t* vals_out, int2* ranges,
-                               cudaStream_t stream)
+                               const ExpandArgs* expand, cudaStream_t stream)
 {
     if (scratch_bytes < df_scratch_bytes(p0.P)) return cudaErrorInvalidValue;
     const DfLayout L = df_layout(scratch, p0.P);
@@ -336,6 +338,13 @@ cudaError_t launch_depth_first(const PreprocessParams& p0, bool half_sh, void* s
     e = launch_sort32(0, p.counter, p.cap, ot, (tb + 7) / 8, tile_keys_in, vals_in, tile_keys_out, vals_out, tile_sort,
                       stream);
     if (e != cudaSuccess) return e;
+    if (expand) {
+        // a recorded frame has one stage per digit pass of the per-tile order
+        for (int k = (tb + 7) / 8; k < (bits_for((uint32_t)(expand->gx * expand->gy)) + 7) / 8; k++) profile_mark(stream);
+        if ((e = launch_quad_expand(*expand, stream)) != cudaSuccess) return e;
+        profile_mark(stream);
+        return cudaSuccess;
+    }
     e = launch_tile_ranges32(p.counter, p.cap, tiles, tile_keys_out, ranges, stream);
     if (e != cudaSuccess) return e;
     profile_mark(stream);

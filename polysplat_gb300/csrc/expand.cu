@@ -47,14 +47,17 @@ struct QuadSeg {
     uint4* totals;    // [spans]
 };
 
+// K: 64-bit keys (quad << 32 | depth bits), or the depth-first pipeline's
+// 32-bit quad ids.
+template <typename K>
 struct ExpandJob {
-    const uint64_t* keys;
+    const K* keys;
     const uint32_t* vals;
     const unsigned long long* count;
     long long cap;
     int gx, gy, quads, spans;
     QuadSeg seg;
-    uint64_t* out_keys;
+    K* out_keys;
     uint32_t* out_vals;
     int2* ranges;
     int32_t* total;
@@ -62,7 +65,8 @@ struct ExpandJob {
 
 __host__ __device__ inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
-__device__ __forceinline__ int key_count(const ExpandJob& a)
+template <typename K>
+__device__ __forceinline__ int key_count(const ExpandJob<K>& a)
 {
     const long long n = (int)(uint32_t)*a.count;  // as the sort counts
     return (int)(n < 0 ? 0 : n > a.cap ? a.cap : n);
@@ -139,7 +143,8 @@ __device__ __forceinline__ uint4 step_counts(uint32_t val, uint4& at)
 
 // Bound by the latency of its loads.  Counting every step instead of those with
 // an end of a quad took 81 us for 50 (21 M keys): 1 step in 20 has one there.
-__global__ __launch_bounds__(kExpThreads, kExpCtas) void k_quad_starts(const __grid_constant__ ExpandJob a)
+template <typename K>
+__global__ __launch_bounds__(kExpThreads, kExpCtas) void k_quad_starts(const __grid_constant__ ExpandJob<K> a)
 {
     __shared__ uint2 s_sum[2][kExpWarps];
     const unsigned lane = threadIdx.x & 31u;
@@ -148,20 +153,21 @@ __global__ __launch_bounds__(kExpThreads, kExpCtas) void k_quad_starts(const __g
     const int len = span_length(n, a.spans);
     const long long first = (long long)blockIdx.x * len;
     const int lo = (int)min((long long)n, first), end = (int)min((long long)n, first + len);
-    const uint32_t* hi = reinterpret_cast<const uint32_t*>(a.keys) + 1;  // quads: the keys' high words
+    constexpr int kWords = sizeof(K) / 4;  // the quad is a key's last word
+    const uint32_t* hi = reinterpret_cast<const uint32_t*>(a.keys) + (kWords - 1);
     uint4 run = make_uint4(0, 0, 0, 0);
     int flip = 0;
     for (int c0 = lo; c0 < end; c0 += kExpChunk, flip ^= 1) {
         const int i0 = c0 + warp * kExpShare + (int)lane, left = end - i0;  // keys 32 k with 32 k < left
-        const uint32_t* hp = hi + 2 * (size_t)i0;
+        const uint32_t* hp = hi + kWords * (size_t)i0;
         const uint32_t* vp = a.vals + i0;
         uint32_t quad[kExpSteps], val[kExpSteps];
 #pragma unroll
         for (int k = 0; k < kExpSteps; k++) {
-            quad[k] = 32 * k < left ? __ldg(hp + 64 * k) : 0u;
+            quad[k] = 32 * k < left ? __ldg(hp + 32 * kWords * k) : 0u;
             val[k] = 32 * k < left ? __ldg(vp + 32 * k) : 0u;
         }
-        uint32_t before = lane == 0 && i0 > 0 && left > 0 ? __ldg(hp - 2) : 0u;
+        uint32_t before = lane == 0 && i0 > 0 && left > 0 ? __ldg(hp - kWords) : 0u;
         const uint4 at = warp_base(val, run, s_sum[flip], lane, warp);
         // counts are needed only in the steps in which a quad ends or begins
         uint32_t bytes = 0;  // this lane's tiles of the steps before
@@ -223,7 +229,8 @@ __device__ __forceinline__ uint32_t comp(const uint4* p, uint32_t i, int b)
 // A thread per tile.  Every CTA sums the list lengths of the tiles before its
 // own, quads at a time, instead of waiting for the CTAs that hold them (8 CTAs
 // and 7 us at 1080p, 127 and 22 us at 8K: latency).
-__global__ __launch_bounds__(kTileThreads) void k_quad_tiles(const __grid_constant__ ExpandJob a)
+template <typename K>
+__global__ __launch_bounds__(kTileThreads) void k_quad_tiles(const __grid_constant__ ExpandJob<K> a)
 {
     __shared__ uint32_t s_pre[4][kMaxSpans];  // P before each span
     __shared__ uint32_t s_all[kMaxSpans];     // sum of the four
@@ -274,7 +281,8 @@ __global__ __launch_bounds__(kTileThreads) void k_quad_tiles(const __grid_consta
     if (t == 0) *a.total = (int)(uint32_t)(*a.count >> 32);
 }
 
-__global__ __launch_bounds__(kExpThreads, kExpCtas) void k_quad_expand(const __grid_constant__ ExpandJob a)
+template <typename K>
+__global__ __launch_bounds__(kExpThreads, kExpCtas) void k_quad_expand(const __grid_constant__ ExpandJob<K> a)
 {
     __shared__ uint2 s_sum[2][kExpWarps];
     __shared__ uint4 s_run[kExpWarps];
@@ -298,26 +306,27 @@ __global__ __launch_bounds__(kExpThreads, kExpCtas) void k_quad_expand(const __g
     int flip = 0;
     for (int c0 = lo; c0 < end; c0 += kExpChunk, flip ^= 1) {
         const int i0 = c0 + warp * kExpShare + (int)lane, left = end - i0;
-        const uint64_t* kp = a.keys + i0;
+        const K* kp = a.keys + i0;
         const uint32_t* vp = a.vals + i0;
-        uint64_t key[kExpSteps];
+        K key[kExpSteps];
         uint32_t val[kExpSteps];
 #pragma unroll
         for (int k = 0; k < kExpSteps; k++) {
-            key[k] = 32 * k < left ? __ldg(kp + 32 * k) : 0ull;
+            key[k] = 32 * k < left ? __ldg(kp + 32 * k) : K(0);
             val[k] = 32 * k < left ? __ldg(vp + 32 * k) : 0u;
         }
         uint4 at = warp_base(val, run, s_sum[flip], lane, warp);
 #pragma unroll
         for (int k = 0; k < kExpSteps; k++) {
             const uint4 p = step_counts(val[k], at);
-            const uint32_t m = val[k], gid = m & kQuadGidMask, q = (uint32_t)(key[k] >> 32), depth = (uint32_t)key[k];
+            const uint32_t m = val[k], gid = m & kQuadGidMask;
+            const uint32_t q = (uint32_t)(key[k] >> 32 * (sizeof(K) / 4 - 1)), depth = (uint32_t)key[k];
             if (m >> kQuadShift != 0u && q < (uint32_t)a.quads) {
                 const uint4 base = *reinterpret_cast<const uint4*>(a.seg.base + 4 * (size_t)q);
                 const uint32_t t0 = a.seg.tile[q];
                 auto put = [&](uint32_t tile, uint32_t pos) {
                     if (pos < cap) {
-                        a.out_keys[pos] = (uint64_t)tile << 32 | depth;
+                        a.out_keys[pos] = sizeof(K) == 8 ? (K)((uint64_t)tile << 32 | depth) : (K)tile;
                         a.out_vals[pos] = gid;
                     }
                 };
@@ -340,10 +349,11 @@ size_t expand_scratch_bytes(int gx, int gy)
     return 256 + 3 * align256(quads * 16) + 3 * align256(quads * 4) + (size_t)kMaxSpans * 16;
 }
 
-cudaError_t launch_quad_expand(const ExpandArgs& e, cudaStream_t stream)
+template <typename K>
+static cudaError_t expand(const ExpandArgs& e, cudaStream_t stream)
 {
-    ExpandJob a;
-    a.keys = e.keys;
+    ExpandJob<K> a;
+    a.keys = static_cast<const K*>(e.keys);
     a.vals = e.vals;
     a.count = e.count;
     a.cap = e.cap;
@@ -351,7 +361,6 @@ cudaError_t launch_quad_expand(const ExpandArgs& e, cudaStream_t stream)
     a.gy = e.gy;
     a.quads = quad_cols(e.gx) * quad_cols(e.gy);
     a.spans = expand_spans();
-    if (e.scratch_bytes < expand_scratch_bytes(e.gx, e.gy) || e.cap >= (1LL << 30)) return cudaErrorInvalidValue;
     char* p = reinterpret_cast<char*>(align256(reinterpret_cast<size_t>(e.scratch)));
     const size_t q16 = align256((size_t)a.quads * 16), q4 = align256((size_t)a.quads * 4);
     a.seg.first = reinterpret_cast<uint4*>(p);
@@ -362,16 +371,22 @@ cudaError_t launch_quad_expand(const ExpandArgs& e, cudaStream_t stream)
     a.seg.base = reinterpret_cast<uint32_t*>(p + cleared);
     a.seg.tile = reinterpret_cast<uint32_t*>(p + cleared + q16);
     a.seg.totals = reinterpret_cast<uint4*>(p + cleared + q16 + q4);
-    a.out_keys = e.out_keys;
+    a.out_keys = static_cast<K*>(e.out_keys);
     a.out_vals = e.out_vals;
     a.ranges = e.ranges;
     a.total = e.total;
     cudaError_t err = cudaMemsetAsync(p, 0, cleared, stream);
     if (err != cudaSuccess) return err;
-    k_quad_starts<<<a.spans, kExpThreads, 0, stream>>>(a);
-    k_quad_tiles<<<div_up(e.gx * e.gy, kTileThreads), kTileThreads, 0, stream>>>(a);
-    k_quad_expand<<<a.spans, kExpThreads, 0, stream>>>(a);
+    k_quad_starts<K><<<a.spans, kExpThreads, 0, stream>>>(a);
+    k_quad_tiles<K><<<div_up(e.gx * e.gy, kTileThreads), kTileThreads, 0, stream>>>(a);
+    k_quad_expand<K><<<a.spans, kExpThreads, 0, stream>>>(a);
     return cudaGetLastError();
+}
+
+cudaError_t launch_quad_expand(const ExpandArgs& e, cudaStream_t stream)
+{
+    if (e.scratch_bytes < expand_scratch_bytes(e.gx, e.gy) || e.cap >= (1LL << 30)) return cudaErrorInvalidValue;
+    return e.key_bytes == 4 ? expand<uint32_t>(e, stream) : expand<uint64_t>(e, stream);
 }
 
 }  // namespace gsr

@@ -257,14 +257,15 @@ cudaError_t launch_gather(int num, const int32_t* d_num, const uint32_t* values,
 // keys (expand.cu).  `count` is PreprocessParams::pair_count's word; its high
 // half goes to `total`.
 struct ExpandArgs {
-    const uint64_t* keys;
+    int key_bytes;  // 8: quad << 32 | depth bits, 4: quad ids
+    const void* keys;
     const uint32_t* vals;
     const unsigned long long* count;
     long long cap;  // of both key buffers
     int gx, gy;
     void* scratch;
     size_t scratch_bytes;
-    uint64_t* out_keys;
+    void* out_keys;
     uint32_t* out_vals;
     int2* ranges;
     int32_t* total;
@@ -348,12 +349,13 @@ cudaError_t launch_render_views(const RenderArgs& a, const RenderView* views_dev
 
 // Depth-first forward (depthfirst.cu): scratch of P-sized arrays, and the
 // pipeline from the counting pass to the tile ranges.  The emitted pair count
-// goes to p.counter; tile ids and values land in tile_keys_out / vals_out.
+// goes to p.counter; tile ids and values land in tile_keys_out / vals_out.  With
+// `expand` (quad pairs) those are expanded instead, and `ranges` is not written.
 size_t df_scratch_bytes(int P);
 cudaError_t launch_depth_first(const PreprocessParams& p, bool half_sh, void* scratch, size_t scratch_bytes,
                                WorkspaceHeader* hdr, const SortScratch& tile_sort, int tiles, uint32_t* tile_keys_in,
                                uint32_t* vals_in, uint32_t* tile_keys_out, uint32_t* vals_out, int2* ranges,
-                               cudaStream_t stream);
+                               const ExpandArgs* expand, cudaStream_t stream);
 
 int device_sm_count();
 // Per-device host caches (occupancy, attribute set-up) hold kMaxDevices

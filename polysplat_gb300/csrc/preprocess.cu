@@ -186,7 +186,8 @@ constexpr int kWarps = 8;
 constexpr int kThreads = kWarps * 32;
 constexpr int kStage = 256;
 
-// HITS (quad keys of one view): the tiles the keys name are counted too.
+// HITS (quad keys of one view): the tiles the keys name are counted too; the
+// counting pass keeps only that count here.
 template <bool HITS>
 struct Stage {
     uint64_t* k;
@@ -289,6 +290,15 @@ __device__ __forceinline__ void block_reserve(const Stage<HITS>& st, const EmitO
         base = __shfl_sync(GSR_FULL_MASK, base, 0);
         if (lane < kWarps) s_base[lane] = base + incl - f;
     }
+}
+
+// The counting pass's hit tiles of a CTA's warps.
+__device__ __forceinline__ void add_hits(unsigned long long* pairs, const int* s_hits)
+{
+    uint32_t h = 0;
+#pragma unroll
+    for (int w = 0; w < kWarps; w++) h += (uint32_t)s_hits[w];
+    if (h) atomicAdd(pairs, (unsigned long long)h << 32);
 }
 
 template <bool HITS>
@@ -413,7 +423,10 @@ __global__ __launch_bounds__(kThreads, VIEWS ? 6 : 5) void k_preprocess(const __
     {
         bool v = single && tile_hit(rect_min.x, rect_min.y, a.bx, a.by, point_xy, conic, power);
         if (COUNT) {
-            if (v) s_cnt[warp][lane] = 1u;
+            if (v) {
+                s_cnt[warp][lane] = 1u;
+                st.hits++;
+            }
         } else if (QUAD) {
             const uint32_t qt = (uint32_t)(a.tile_base + (rect_min.y >> 1) * qgx + (rect_min.x >> 1));
             const uint32_t bit = 1u << ((rect_min.x & 1) | ((rect_min.y & 1) << 1));
@@ -498,6 +511,7 @@ __global__ __launch_bounds__(kThreads, VIEWS ? 6 : 5) void k_preprocess(const __
                     if (COUNT) {
                         const unsigned mm = __ballot_sync(GSR_FULL_MASK, m != 0u);
                         if (lane == 0) s_cnt[warp][i] += __popc(mm);
+                        st.hits += __popc(m);
                     } else {
                         const uint64_t key = ((uint64_t)(uint32_t)(a.tile_base + qy * qgx + qx) << 32) | db;
                         stage_emit(st, out, m != 0u, key, gid | (m << kQuadShift), lane);
@@ -587,6 +601,7 @@ __global__ __launch_bounds__(kThreads, VIEWS ? 6 : 5) void k_preprocess(const __
             }
             if (COUNT) {
                 if (v) atomicAdd(&s_cnt[warp][owner], 1u);
+                if (QUAD) st.hits += __popc(qm);
             } else if (QUAD) {
                 const uint64_t key = ((uint64_t)(uint32_t)(a.tile_base + y * qgx + x) << 32) | db;
                 stage_emit(st, out, v, key, (uint32_t)(a.gid_base + warp_first + owner) | (qm << kQuadShift), lane);
@@ -650,6 +665,12 @@ __global__ __launch_bounds__(kThreads, VIEWS ? 6 : 5) void k_preprocess(const __
                                                (int)((uint32_t)rect_min.y | ((uint32_t)rect_max.y << 16) |
                                                      (queued ? 0x80000000u : 0u)));
             }
+        }
+        if (QUAD && a.pair_count) {
+            const uint32_t h = __reduce_add_sync(GSR_FULL_MASK, st.hits);
+            if (lane == 0) s_fill[warp] = (int)h;
+            __syncthreads();
+            if (threadIdx.x == 0) add_hits(a.pair_count, s_fill);
         }
     } else {
         // (4) the staged keys, to the place reserved before the features
@@ -987,6 +1008,7 @@ __global__ __launch_bounds__(kThreads, 4) void k_emit_massive(const __grid_const
                         const unsigned mm = __ballot_sync(GSR_FULL_MASK, m != 0u);
                         if (MODE == kMassiveCount) {
                             hits += __popc(mm);
+                            if (QUAD) st.hits += __popc(m);
                         } else if (mm) {  // the next of the Gaussian's own slots
                             uint32_t p = 0;
                             if (lane == 0) p = atomicAdd(&s_pos[w], (uint32_t)__popc(mm));
@@ -1045,8 +1067,10 @@ __global__ __launch_bounds__(kThreads, 4) void k_emit_massive(const __grid_const
         } else if (MODE == kMassiveCount) {
             uint32_t cnt = 0;
             if (QUAD)
-                sweep_warp_quad(me, eb, a, lane,
-                                [&](bool v, int, int, uint32_t) { cnt += __popc(__ballot_sync(GSR_FULL_MASK, v)); });
+                sweep_warp_quad(me, eb, a, lane, [&](bool v, int, int, uint32_t m) {
+                    cnt += __popc(__ballot_sync(GSR_FULL_MASK, v));
+                    if (v) st.hits += __popc(m);
+                });
             else
                 sweep_warp(me, eb, a, lane,
                            [&](bool v, int, int) { cnt += __popc(__ballot_sync(GSR_FULL_MASK, v)); });
@@ -1083,6 +1107,11 @@ __global__ __launch_bounds__(kThreads, 4) void k_emit_massive(const __grid_const
     if (MODE == kMassiveEmit64) {
         block_reserve(st, out, s_fill, s_base, lane, warp);
         block_copy(st, out, s_base, lane, warp);
+    } else if (MODE == kMassiveCount && QUAD && a.pair_count) {
+        const uint32_t h = __reduce_add_sync(GSR_FULL_MASK, st.hits);
+        if (lane == 0) s_fill[warp] = (int)h;
+        __syncthreads();
+        if (threadIdx.x == 0) add_hits(a.pair_count, s_fill);
     }
 }
 

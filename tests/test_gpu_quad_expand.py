@@ -79,3 +79,36 @@ def test_empty_view_and_small_buffers(scene):
             _fused(scene, Rasterizer(scene, cap, 1 << 16), cam, R.RENDER_PERSISTENT_FUSED, None)
         assert ei.value.status == R.GSR_OVERFLOW and ei.value.num == n
     assert _fused(scene, Rasterizer(scene, n, 1 << 16), cam, R.RENDER_PERSISTENT_FUSED, None)[1] == n
+
+
+def _depth_first(scene, cam, cap, dev, flag):
+    r = Rasterizer(scene, cap, 1 << 16)
+    r._expand_quads = lambda _: bool(flag)
+    img, st = r.forward(scene, cam, BG, render_variant="preranges_smem_persistent_lite", use_es=True,
+                        return_stats=True)
+    assert st["used_es"]
+    return r, img, st["num_rendered"]
+
+
+@pytest.mark.parametrize("w,h", [(16, 16), (33, 17), (250, 131), (641, 359), (1920, 1080), (3839, 2161)])
+def test_depth_first_expanded_lists_are_the_same(cuda_device, scene, w, h):
+    """The depth-first order of equal keys is the Gaussians' index order, so the
+    arrays and the image are equal, not only alike."""
+    cam, cap, tiles = _camera(w, h), 6_000_000, -(-w // 16) * -(-h // 16)
+    a, ia, na = _depth_first(scene, cam, cap, cuda_device, True)
+    b, ib, nb = _depth_first(scene, cam, cap, cuda_device, False)
+    assert na == nb and torch.equal(ia, ib)
+    for x, y in ((a.gaussian_keys_sorted.view(torch.int32)[:na], b.gaussian_keys_sorted.view(torch.int32)[:na]),
+                 (a.gaussian_values_sorted[:na], b.gaussian_values_sorted[:na]),
+                 (a.tile_ranges_buf[:tiles], b.tile_ranges_buf[:tiles])):
+        assert torch.equal(x, y)
+
+
+def test_depth_first_expansion_reports_the_per_tile_count(cuda_device, scene):
+    cam = _camera(1920, 1080)
+    n = _depth_first(scene, cam, 6_000_000, cuda_device, False)[2]
+    for cap in (n - 1, n // 2, n // 8):
+        with pytest.raises(GsrError) as ei:
+            _depth_first(scene, cam, cap, cuda_device, True)
+        assert ei.value.status == R.GSR_OVERFLOW and ei.value.num == n
+    assert _depth_first(scene, cam, n, cuda_device, True)[2] == n
