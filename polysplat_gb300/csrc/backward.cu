@@ -256,14 +256,16 @@ gsr_status gsr_train_forward(int P, const float* means, const float* log_scales,
     if (workspace_bytes < sort_workspace_bytes(key_capacity) || key_capacity >= (1LL << 30)) return GSR_INVALID_ARG;
     const int tiles = div_up(width, 16) * div_up(height, 16);
     cudaError_t e = launch_scene_prepare(P, log_scales, quats, logits, opacity, cov3d, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(workspace, 0, sizeof(uint32_t), s);
+    if (e == cudaSuccess) e = clear_header(workspace, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(curr_offset, 0, sizeof(int32_t), s);
     if (e != cudaSuccess) return GSR_CUDA_ERROR;
-    gsr_status st = gsr_preprocess(P, means, shs, 0, opacity, cov3d, width, height, 16, 16, cam_pos, cam_rot,
-                                   focal_x, focal_y, z_far, z_near, points_xy, rgb_depth, conic_opacity,
-                                   keys_unsorted, values_unsorted, key_capacity, curr_offset, workspace,
-                                   workspace_bytes, stream);
+    PreprocessParams p;
+    gsr_status st = preprocess_params(p, P, means, shs, opacity, cov3d, width, height, 16, 16, cam_pos, cam_rot, focal_x,
+                                      focal_y, z_far, z_near, points_xy, rgb_depth, conic_opacity, keys_unsorted,
+                                      values_unsorted, key_capacity, curr_offset, workspace, workspace_bytes);
     if (st != GSR_OK) return st;
+    p.header_clear = 1;
+    if (launch_preprocess(p, false, s) != cudaSuccess) return GSR_CUDA_ERROR;
     SortArgs sa;
     sa.num = 0;
     sa.d_num = curr_offset;
@@ -276,6 +278,7 @@ gsr_status gsr_train_forward(int P, const float* means, const float* log_scales,
     sa.vals_out = values_sorted;
     sa.ws = workspace;
     sa.ws_bytes = workspace_bytes;
+    sa.header_clear = true;
     if ((e = launch_sort(sa, s)) != cudaSuccess) return GSR_CUDA_ERROR;
     if ((e = launch_tile_ranges(0, curr_offset, key_capacity, tiles, keys_sorted, ranges, false, s)) != cudaSuccess)
         return GSR_CUDA_ERROR;
@@ -393,7 +396,7 @@ gsr_status gsr_train_forward_views(int P, const float* means, const float* log_s
     if ((long long)P * n_views >= (1LL << 31) || (long long)tiles * n_views >= (1LL << 30)) return GSR_INVALID_ARG;
     const int kt = quad ? quad_cols(div_up(width, 16)) * quad_cols(div_up(height, 16)) : tiles;
     cudaError_t e = launch_scene_prepare(P, log_scales, quats, logits, opacity, cov3d, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(workspace, 0, sizeof(uint32_t), s);
+    if (e == cudaSuccess) e = clear_header(workspace, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(curr_offset, 0, sizeof(int32_t), s);
     if (e != cudaSuccess) return GSR_CUDA_ERROR;
     // every view's parameter block, as the single-view preprocess fills it,
@@ -421,6 +424,7 @@ gsr_status gsr_train_forward_views(int P, const float* means, const float* log_s
     } else {
         PreprocessParams base = hp[0];
         base.n_views = n_views;
+        base.header_clear = 1;
         base.interleave = 1;  // every view has the scene's P
         // a pageable source is staged before the call returns
         e = cudaMemcpyAsync(d_params, hp.data(), sizeof(PreprocessParams) * (size_t)n_views, cudaMemcpyHostToDevice, s);
@@ -438,6 +442,7 @@ gsr_status gsr_train_forward_views(int P, const float* means, const float* log_s
         sa.vals_out = values_sorted;
         sa.ws = workspace;
         sa.ws_bytes = workspace_bytes;
+        sa.header_clear = true;
         if ((e = launch_sort(sa, s)) != cudaSuccess) return GSR_CUDA_ERROR;
         e = launch_tile_ranges(0, curr_offset, key_capacity, kt * n_views, keys_sorted, ranges, false, s);
     }

@@ -155,7 +155,7 @@ void pack_view(PreprocessParams& p, const gsr_scene_ref& sc, const gsr_view& v, 
 cudaError_t enqueue(gsr_batcher* b, const Shape& s, cudaStream_t st)
 {
     WorkspaceHeader* h = reinterpret_cast<WorkspaceHeader*>(b->ws);
-    cudaError_t e = cudaMemsetAsync(&h->status, 0, sizeof(uint32_t), st);
+    cudaError_t e = clear_header(h, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(b->counter, 0, sizeof(int32_t), st);
     if (e != cudaSuccess) return e;
     PreprocessParams base;
@@ -175,6 +175,7 @@ cudaError_t enqueue(gsr_batcher* b, const Shape& s, cudaStream_t st)
     base.bx = s.bx;
     base.by = s.by;
     base.quad = s.quad;
+    base.header_clear = 1;
     e = launch_preprocess_views(base, s.n_views, s.blocks, s.half != 0, st);
     if (e != cudaSuccess) return e;
     SortArgs sa;
@@ -189,6 +190,7 @@ cudaError_t enqueue(gsr_batcher* b, const Shape& s, cudaStream_t st)
     sa.vals_out = b->vs;
     sa.ws = b->ws;
     sa.ws_bytes = b->ws_bytes;
+    sa.header_clear = true;
     if ((e = launch_sort(sa, st)) != cudaSuccess) return e;
     e = launch_tile_ranges(0, b->counter, b->cap, s.tiles, b->ks, reinterpret_cast<int32_t*>(b->ranges), false, st);
     if (e != cudaSuccess) return e;

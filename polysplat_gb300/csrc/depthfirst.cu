@@ -312,7 +312,8 @@ cudaError_t launch_depth_first(const PreprocessParams& p0, bool half_sh, void* s
         profile_mark(stream);
 
         // depth sort of the V emitting Gaussians (count read on the device)
-        const SortScratch ds = carve_sort_scratch(hdr, L.sort_mem, p.P, 4);
+        SortScratch ds = carve_sort_scratch(hdr, L.sort_mem, p.P, 4);
+        ds.header_clear = p.header_clear != 0;
         OrderMap od{kOrderDepth32, 32};
         e = launch_sort32(0, reinterpret_cast<const int32_t*>(&L.misc[0]), p.P, od, 4, L.ckeys, L.cgids, L.skeys,
                           L.sgids, ds, stream);

@@ -89,6 +89,8 @@ struct PreprocessParams {
     // Quad keys that are expanded to per-tile lists after the sort: counts the
     // keys (low half) and the hit tiles (high half) in place of `counter`.
     unsigned long long* pair_count = nullptr;
+    // the caller has cleared the whole workspace header (clear_header)
+    int header_clear = 0;
 };
 // Quad keys: bit (x & 1) | (y & 1) << 1 of value >> kQuadShift is set when
 // the Gaussian hits tile (x, y) of the quad, by the same exact tile test the
@@ -157,6 +159,12 @@ constexpr size_t kPreprocessRegionOffset = 2 * sizeof(uint32_t);
 constexpr size_t kPreprocessRegionBytes = 10 * sizeof(uint32_t);
 constexpr size_t kSortRegionOffset = 16 * sizeof(uint32_t);
 constexpr size_t kHeaderBytes = 16384;
+// One fill for a frame's preprocess and first sort in place of one for each
+// region (about 2 us of a small frame's stream time apiece).
+inline cudaError_t clear_header(void* workspace, cudaStream_t stream)
+{
+    return cudaMemsetAsync(workspace, 0, sizeof(WorkspaceHeader), stream);
+}
 static_assert(sizeof(WorkspaceHeader) <= kHeaderBytes, "header too large");
 static_assert(offsetof(WorkspaceHeader, mq_count) == kPreprocessRegionOffset &&
                   offsetof(WorkspaceHeader, pad) == kPreprocessRegionOffset + kPreprocessRegionBytes &&
@@ -209,6 +217,7 @@ struct SortArgs {
     uint32_t* vals_out;
     void* ws;
     size_t ws_bytes;
+    bool header_clear = false;  // the header's sort region is clear
 };
 cudaError_t launch_sort(const SortArgs& a, cudaStream_t stream);
 
@@ -233,6 +242,7 @@ struct SortScratch {
     uint32_t* alt_vals;
     uint32_t* look[2];
     long long tiles_cap;
+    bool header_clear = false;  // the sort region of hdr is clear
 };
 size_t sort_scratch_bytes(long long cap, int key_bytes);
 SortScratch carve_sort_scratch(WorkspaceHeader* hdr, void* mem, long long cap, int key_bytes);

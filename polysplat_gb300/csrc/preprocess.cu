@@ -1344,7 +1344,7 @@ static int emit_grid(Kern kern)
 static cudaError_t preprocess_common(const PreprocessParams& p, bool half_sh, bool count, cudaStream_t stream)
 {
     if (p.P <= 0) return cudaSuccess;
-    if (p.mq.capacity > 0) {
+    if (p.mq.capacity > 0 && !p.header_clear) {
         // queue counters, heads of both passes and depth_hi: the preprocess
         // region of the workspace header, which starts at the count words
         cudaError_t e = cudaMemsetAsync(p.mq.count, 0, kPreprocessRegionBytes, stream);
@@ -1385,7 +1385,7 @@ cudaError_t launch_preprocess_views(const PreprocessParams& base, int n_views, i
     if (n_views <= 0 || blocks <= 0) return cudaSuccess;
     if (n_views > 32767 || !base.views || base.mq.capacity <= 0) return cudaErrorInvalidValue;
     if (base.quad && (base.bx != 16 || base.by != 16)) return cudaErrorInvalidValue;
-    cudaError_t e = cudaMemsetAsync(base.mq.count, 0, kPreprocessRegionBytes, stream);
+    cudaError_t e = base.header_clear ? cudaSuccess : cudaMemsetAsync(base.mq.count, 0, kPreprocessRegionBytes, stream);
     if (e != cudaSuccess) return e;
     const dim3 grid(blocks);
     const DfEmit none{nullptr, nullptr, nullptr, nullptr, 0};

@@ -602,8 +602,10 @@ cudaError_t run_sort(const SortJob<K>& job, int max_passes, cudaStream_t stream)
     SortJob<K> a = job;
     a.spin_limit = sort_wait_limit();
     // clear the sort region of the header (pass counters and histograms)
-    cudaError_t e = cudaMemsetAsync(reinterpret_cast<char*>(a.s.hdr) + kSortRegionOffset, 0,
-                                    sizeof(WorkspaceHeader) - kSortRegionOffset, stream);
+    cudaError_t e = cudaSuccess;
+    if (!a.s.header_clear)
+        e = cudaMemsetAsync(reinterpret_cast<char*>(a.s.hdr) + kSortRegionOffset, 0,
+                            sizeof(WorkspaceHeader) - kSortRegionOffset, stream);
     if (e != cudaSuccess) return e;
     // failure-detection hook: the first pass starts at tile 1, so tile 0 never
     // publishes and the look-back of the tiles after it runs out
@@ -719,6 +721,7 @@ cudaError_t launch_sort(const SortArgs& a, cudaStream_t stream)
     j.keys_out = a.keys_out;
     j.vals_out = a.vals_out;
     j.s = workspace_sort_scratch(a.ws, a.cap);
+    j.s.header_clear = a.header_clear;
     j.spin_limit = kSpinLimit;
     return run_sort(j, (a.end_bit + 7) / 8, stream);
 }

@@ -38,6 +38,27 @@ def _p(t: torch.Tensor):
     return ctypes.c_void_p(t.data_ptr())
 
 
+def _slab(dev, nbytes):
+    """One allocation for parts of `nbytes` each (an allocation of its own takes
+    the host 2 to 3 us)."""
+    return torch.empty(sum((int(n) + 255) & ~255 for n in nbytes), dtype=torch.uint8, device=dev)
+
+
+def _parts(slab, nbytes):
+    """The addresses of a slab's parts, each on 256 bytes."""
+    at, out = slab.data_ptr(), []
+    for n in nbytes:
+        out.append(ctypes.c_void_p(at))
+        at += (int(n) + 255) & ~255
+    return out
+
+
+def _kept_bytes(cap, rows, tiles, pixels):
+    """What a backward reads: count, sorted values, features (xy, colour and
+    depth, conic and opacity), ranges, blended counts, transmittance."""
+    return 4, 4 * cap, 8 * rows, 16 * rows, 16 * rows, 8 * tiles, 4 * tiles, 4 * pixels
+
+
 def _cam_args(cam: Camera):
     pos = (ctypes.c_float * 3)(*[float(v) for v in cam.position.reshape(-1).tolist()])
     rot = (ctypes.c_float * 9)(*[float(v) for v in cam.rotation.reshape(-1).tolist()])
@@ -57,52 +78,48 @@ class _RenderFn(torch.autograd.Function):
         stream = ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
         cap = int(key_capacity)
         while True:
-            b = dict(
-                opacity=torch.empty(P, device=dev), cov3d=torch.empty((P, 6), device=dev),
-                count=torch.zeros(1, dtype=torch.int32, device=dev),
-                ws=torch.empty(get_sort_buffer_size(cap), dtype=torch.int8, device=dev),
-                ku=torch.empty(cap, dtype=torch.int64, device=dev), vu=torch.empty(cap, dtype=torch.int32, device=dev),
-                ks=torch.empty(cap, dtype=torch.int64, device=dev), vs=torch.empty(cap, dtype=torch.int32, device=dev),
-                xy=torch.empty((P, 2), device=dev), rgbd=torch.empty((P, 4), device=dev),
-                con=torch.empty((P, 4), device=dev), ranges=torch.empty((tiles, 2), dtype=torch.int32, device=dev),
-                n_tile=torch.empty(tiles, dtype=torch.int32, device=dev), T=torch.empty((H, W), device=dev),
-                image=torch.empty((H, W, 3), device=dev))
+            wsb = get_sort_buffer_size(cap)
+            work_bytes = (4 * P, 24 * P, wsb, 8 * cap, 4 * cap, 8 * cap)
+            kept_bytes = _kept_bytes(cap, P, tiles, H * W)
+            work, kept = _slab(dev, work_bytes), _slab(dev, kept_bytes)
+            op, cov, ws, ku, vu, ks = _parts(work, work_bytes)
+            count, vs, xy, rgbd, con, ranges, n_tile, T = _parts(kept, kept_bytes)
+            image = torch.empty((H, W, 3), device=dev)
             check(lib().gsr_train_forward(
                 P, *[_p(t) for t in params], W, H, pos, rot, cam.focal_x, cam.focal_y, cam.zFar, cam.zNear, bgc,
-                _p(b["opacity"]), _p(b["cov3d"]), _p(b["count"]), _p(b["ws"]), b["ws"].numel(), _p(b["ku"]),
-                _p(b["vu"]), _p(b["ks"]), _p(b["vs"]), cap, _p(b["xy"]), _p(b["rgbd"]), _p(b["con"]),
-                _p(b["ranges"]), _p(b["n_tile"]), _p(b["T"]), _p(b["image"]), stream), "train_forward")
+                op, cov, count, ws, wsb, ku, vu, ks, vs, cap, xy, rgbd, con, ranges, n_tile, T, _p(image), stream),
+                "train_forward")
             n = ctypes.c_int32(0)
-            st = lib().gsr_read_status(_p(b["ws"]), _p(b["count"]), cap, ctypes.byref(n), stream)
+            st = lib().gsr_read_status(ws, count, cap, ctypes.byref(n), stream)
             if st == R.GSR_OVERFLOW:
                 cap = max(2 * cap, int(n.value * 1.25))
                 continue
             check(st, "train_forward", n.value)
             break
-        for k in ("ku", "ks", "ws", "opacity", "cov3d"):
-            del b[k]
-        ctx.b, ctx.cam, ctx.bg, ctx.cap, ctx.P = b, cam, [float(v) for v in bg], cap, P
+        ctx.b, ctx.cam, ctx.bg, ctx.cap, ctx.P = (kept, kept_bytes), cam, [float(v) for v in bg], cap, P
         ctx.save_for_backward(*params)
         ctx.num_rendered = n.value
-        return b["image"]
+        return image
 
     @staticmethod
     def backward(ctx, grad_image):
         means, log_scales, quats, logits, shs = ctx.saved_tensors
-        b, cam, P = ctx.b, ctx.cam, ctx.P
+        kept, kept_bytes = ctx.b
+        cam, P = ctx.cam, ctx.P
+        count, vs, xy, rgbd, con, ranges, n_tile, T = _parts(kept, kept_bytes)
         dev = means.device
         g = grad_image.contiguous().float()
         pos, rot = _cam_args(cam)
         bgc = (ctypes.c_float * 3)(*ctx.bg)
-        gxy, gcon, grgb = (torch.empty((P, 2), device=dev), torch.empty((P, 4), device=dev),
-                           torch.empty((P, 3), device=dev))
+        grad_bytes = (8 * P, 16 * P, 12 * P)
+        grads = _slab(dev, grad_bytes)
+        gxy, gcon, grgb = _parts(grads, grad_bytes)
         outs = [torch.empty_like(t) for t in (means, log_scales, quats, logits, shs)]
         stream = ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
         check(lib().gsr_train_backward(
             P, _p(means), _p(log_scales), _p(quats), _p(logits), _p(shs), cam.width, cam.height, pos, rot,
-            cam.focal_x, cam.focal_y, cam.zFar, cam.zNear, bgc, _p(b["count"]), ctx.cap, _p(b["vs"]),
-            _p(b["ranges"]), _p(b["n_tile"]), _p(b["T"]), _p(b["xy"]), _p(b["rgbd"]), _p(b["con"]), _p(g), _p(gxy),
-            _p(gcon), _p(grgb), *[_p(t) for t in outs], 0, stream), "train_backward")
+            cam.focal_x, cam.focal_y, cam.zFar, cam.zNear, bgc, count, ctx.cap, vs, ranges, n_tile, T, xy, rgbd, con,
+            _p(g), gxy, gcon, grgb, *[_p(t) for t in outs], 0, stream), "train_backward")
         ctx.b = None
         gm, gls, gq, glg, gsh = outs
         return gm, gls, gq, glg, gsh, None, None, None
@@ -140,26 +157,21 @@ class _RenderViewsFn(torch.autograd.Function):
         bgc = (ctypes.c_float * 3)(*[float(v) for v in bg])
         params = [t.detach().contiguous().float() for t in (means, log_scales, quats, logits, shs.reshape(P, 48))]
         stream = ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
-        scratch = torch.empty(lib().gsr_train_views_scratch_bytes(V), dtype=torch.int8, device=dev)
+        scb = lib().gsr_train_views_scratch_bytes(V)
         cap = int(key_capacity)
         while True:
-            b = dict(
-                opacity=torch.empty(P, device=dev), cov3d=torch.empty((P, 6), device=dev),
-                count=torch.zeros(1, dtype=torch.int32, device=dev),
-                ws=torch.empty(get_sort_buffer_size(cap), dtype=torch.int8, device=dev),
-                ku=torch.empty(cap, dtype=torch.int64, device=dev), vu=torch.empty(cap, dtype=torch.int32, device=dev),
-                ks=torch.empty(cap, dtype=torch.int64, device=dev), vs=torch.empty(cap, dtype=torch.int32, device=dev),
-                xy=torch.empty((V * P, 2), device=dev), rgbd=torch.empty((V * P, 4), device=dev),
-                con=torch.empty((V * P, 4), device=dev), ranges=torch.empty((V * tiles, 2), dtype=torch.int32, device=dev),
-                n_tile=torch.empty(V * tiles, dtype=torch.int32, device=dev), T=torch.empty((V, H, W), device=dev),
-                image=torch.empty((V, H, W, 3), device=dev))
+            wsb = get_sort_buffer_size(cap)
+            work_bytes = (4 * P, 24 * P, scb, wsb, 8 * cap, 4 * cap, 8 * cap)
+            kept_bytes = _kept_bytes(cap, V * P, V * tiles, V * H * W)
+            work, kept = _slab(dev, work_bytes), _slab(dev, kept_bytes)
+            op, cov, scratch, ws, ku, vu, ks = _parts(work, work_bytes)
+            count, vs, xy, rgbd, con, ranges, n_tile, T = _parts(kept, kept_bytes)
+            image = torch.empty((V, H, W, 3), device=dev)
             check(lib().gsr_train_forward_views(
-                P, *[_p(t) for t in params], V, W, H, pos, rot, intr, bgc, _p(b["opacity"]), _p(b["cov3d"]),
-                _p(scratch), scratch.numel(), _p(b["count"]), _p(b["ws"]), b["ws"].numel(), _p(b["ku"]), _p(b["vu"]),
-                _p(b["ks"]), _p(b["vs"]), cap, _p(b["xy"]), _p(b["rgbd"]), _p(b["con"]), _p(b["ranges"]),
-                _p(b["n_tile"]), _p(b["T"]), _p(b["image"]), flags, stream), "train_forward_views")
+                P, *[_p(t) for t in params], V, W, H, pos, rot, intr, bgc, op, cov, scratch, scb, count, ws, wsb, ku,
+                vu, ks, vs, cap, xy, rgbd, con, ranges, n_tile, T, _p(image), flags, stream), "train_forward_views")
             n = ctypes.c_int32(0)
-            st = lib().gsr_read_status(_p(b["ws"]), _p(b["count"]), cap, ctypes.byref(n), stream)
+            st = lib().gsr_read_status(ws, count, cap, ctypes.byref(n), stream)
             if st == R.GSR_OVERFLOW:
                 cap = max(2 * cap, int(n.value * 1.25))
                 if cap >= 1 << 30:
@@ -167,17 +179,17 @@ class _RenderViewsFn(torch.autograd.Function):
                 continue
             check(st, "train_forward_views", n.value)
             break
-        for k in ("ku", "ks", "ws", "opacity", "cov3d"):
-            del b[k]
-        ctx.b, ctx.cams, ctx.bg, ctx.cap, ctx.flags = b, list(cams), [float(v) for v in bg], cap, flags
+        ctx.b, ctx.cams, ctx.bg, ctx.cap, ctx.flags = (kept, kept_bytes), list(cams), [float(v) for v in bg], cap, flags
         ctx.save_for_backward(*params)
         ctx.num_rendered = n.value
-        return b["image"]
+        return image
 
     @staticmethod
     def backward(ctx, grad_image):
         means, log_scales, quats, logits, shs = ctx.saved_tensors
-        b, cams = ctx.b, ctx.cams
+        kept, kept_bytes = ctx.b
+        cams = ctx.cams
+        count, vs, xy, rgbd, con, ranges, n_tile, T = _parts(kept, kept_bytes)
         dev = means.device
         P, V = means.shape[0], len(cams)
         g = grad_image.contiguous().float()
@@ -188,8 +200,7 @@ class _RenderViewsFn(torch.autograd.Function):
         stream = ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
         check(lib().gsr_train_backward_views(
             P, _p(means), _p(log_scales), _p(quats), _p(logits), _p(shs), V, cams[0].width, cams[0].height, pos, rot,
-            intr, bgc, _p(b["count"]), ctx.cap, _p(b["vs"]), _p(b["ranges"]), _p(b["n_tile"]), _p(b["T"]),
-            _p(b["xy"]), _p(b["rgbd"]), _p(b["con"]), _p(g), _p(gfeat), *[_p(t) for t in outs], 0, ctx.flags,
+            intr, bgc, count, ctx.cap, vs, ranges, n_tile, T, xy, rgbd, con, _p(g), _p(gfeat), *[_p(t) for t in outs], 0, ctx.flags,
             stream), "train_backward_views")
         ctx.b = None
         gm, gls, gq, glg, gsh = outs

@@ -68,8 +68,12 @@ def _dev(t: torch.Tensor, what: str, dtype=None) -> torch.Tensor:
 
 
 def _host_floats(t, n: int, what: str):
-    """Camera position/rotation and background are read on the host."""
+    """Camera position/rotation and background are read on the host.  A float32
+    host tensor is read in place (1 us instead of 10): the caller holds it
+    through the call."""
     if isinstance(t, torch.Tensor):
+        if t.dtype == torch.float32 and t.device.type == "cpu" and t.numel() >= n and t.is_contiguous():
+            return ctypes.c_void_p(t.data_ptr())
         vals = t.detach().to("cpu", torch.float32).reshape(-1).tolist()
     else:
         vals = [float(v) for v in np.asarray(t, dtype=np.float32).reshape(-1)]
