@@ -200,6 +200,7 @@ cudaError_t enqueue(gsr_batcher* b, const Shape& s, cudaStream_t st)
     ra.num = 0;
     ra.d_num = b->counter;
     ra.cap = b->cap;
+    ra.queue_clear = 1;
     ra.W = ra.H = 1;
     ra.bx = s.bx;
     ra.by = s.by;

@@ -274,6 +274,7 @@ struct StatusWords {
 
 __global__ void k_read_status(const uint32_t* status, const int32_t* num, volatile uint32_t* out)
 {
+    chain_wait();
     out[0] = status ? *status : 0u;
     out[1] = num ? (uint32_t)*num : 0u;
 }
@@ -303,8 +304,9 @@ gsr_status gsr_read_status(const void* workspace, const int32_t* d_num, int64_t 
     int32_t num = 0;
     static thread_local StatusWords words;
     if (word_on_device(workspace) && word_on_device(d_num) && words.ready()) {
-        k_read_status<<<1, 1, 0, s>>>(static_cast<const uint32_t*>(workspace), d_num, words.device);
-        if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(s) != cudaSuccess) return GSR_CUDA_ERROR;
+        if (launch_chained(k_read_status, 1, 1, 0, s, static_cast<const uint32_t*>(workspace), d_num, words.device) !=
+                cudaSuccess ||
+            cudaStreamSynchronize(s) != cudaSuccess) return GSR_CUDA_ERROR;
         status = words.host[0];
         num = (int32_t)words.host[1];
     } else {
@@ -436,7 +438,7 @@ static gsr_status render_impl(int variant, int num, const int32_t* d_num, long l
                               int block_x, int block_y, int P, const float* points_xy, const float* rgb_depth,
                               const float* conic_opacity, const uint64_t* keys_sorted, const uint32_t* values_sorted,
                               const int32_t* ranges, const float* bg_color, uint8_t* out_color, void* workspace,
-                              cudaStream_t s, bool quad = false)
+                              cudaStream_t s, bool quad = false, bool queue_clear = false)
 {
     if (!workspace || !out_color || !bg_color || width <= 0 || height <= 0 || !valid_tile_shape(block_x, block_y))
         return GSR_INVALID_ARG;
@@ -465,6 +467,7 @@ static gsr_status render_impl(int variant, int num, const int32_t* d_num, long l
     a.out = out_color;
     a.ws = reinterpret_cast<WorkspaceHeader*>(workspace);
     a.quad = quad ? 1 : 0;
+    a.queue_clear = queue_clear ? 1 : 0;
     return from_cuda(launch_render(a, s));
 }
 
@@ -572,7 +575,7 @@ gsr_status gsr_forward(int variant, int P, const float* pos, const void* shs, in
         if ((e = launch_quad_expand(x, s)) != cudaSuccess) return from_cuda(e);
         profile_mark(s);
         st = render_impl(variant, 0, curr_offset, key_capacity, width, height, 16, 16, P, points_xy, rgb_depth,
-                         conic_opacity, keys_sorted, values_sorted, ranges, bg_color, out_color, workspace, s);
+                         conic_opacity, keys_sorted, values_sorted, ranges, bg_color, out_color, workspace, s, false, true);
         if (st == GSR_OK) profile_mark(s);
         return st;
     }
@@ -599,7 +602,7 @@ gsr_status gsr_forward(int variant, int P, const float* pos, const void* shs, in
         profile_mark(s);
     }
     st = render_impl(variant, 0, curr_offset, key_capacity, width, height, block_x, block_y, P, points_xy, rgb_depth,
-                     conic_opacity, keys_sorted, values_sorted, ranges, bg_color, out_color, workspace, s, quad);
+                     conic_opacity, keys_sorted, values_sorted, ranges, bg_color, out_color, workspace, s, quad, true);
     if (st == GSR_OK) profile_mark(s);
     return st;
 }
@@ -677,7 +680,7 @@ gsr_status gsr_forward_depth_first(int variant, int P, const float* pos, const v
     }
     if (e != cudaSuccess) return from_cuda(e);
     st = render_impl(variant, 0, curr_offset, key_capacity, width, height, block_x, block_y, P, points_xy, rgb_depth,
-                     conic_opacity, nullptr, values_sorted, ranges, bg_color, out_color, workspace, s, quad);
+                     conic_opacity, nullptr, values_sorted, ranges, bg_color, out_color, workspace, s, quad, true);
     if (st == GSR_OK) profile_mark(s);
     return st;
 }

@@ -149,6 +149,8 @@ __global__ __launch_bounds__(kExpThreads, kExpCtas) void k_quad_starts(const __g
     __shared__ uint2 s_sum[2][kExpWarps];
     const unsigned lane = threadIdx.x & 31u;
     const int warp = threadIdx.x >> 5;
+    chain_wait();
+    chain_ready();
     const int n = key_count(a);
     const int len = span_length(n, a.spans);
     const long long first = (long long)blockIdx.x * len;
@@ -236,6 +238,8 @@ __global__ __launch_bounds__(kTileThreads) void k_quad_tiles(const __grid_consta
     __shared__ uint32_t s_all[kMaxSpans];     // sum of the four
     __shared__ uint32_t s_warp[kTileThreads / 32];
     const int tid = threadIdx.x;
+    chain_wait();
+    chain_ready();
     {
         const uint4 t = tid < a.spans ? a.seg.totals[tid] : make_uint4(0, 0, 0, 0);
         uint32_t sum;
@@ -288,6 +292,8 @@ __global__ __launch_bounds__(kExpThreads, kExpCtas) void k_quad_expand(const __g
     __shared__ uint4 s_run[kExpWarps];
     const unsigned lane = threadIdx.x & 31u;
     const int warp = threadIdx.x >> 5;
+    chain_wait();
+    chain_ready();
     const int n = key_count(a);
     const int len = span_length(n, a.spans);
     const long long first = (long long)blockIdx.x * len;
@@ -377,10 +383,10 @@ static cudaError_t expand(const ExpandArgs& e, cudaStream_t stream)
     a.total = e.total;
     cudaError_t err = cudaMemsetAsync(p, 0, cleared, stream);
     if (err != cudaSuccess) return err;
-    k_quad_starts<K><<<a.spans, kExpThreads, 0, stream>>>(a);
-    k_quad_tiles<K><<<div_up(e.gx * e.gy, kTileThreads), kTileThreads, 0, stream>>>(a);
-    k_quad_expand<K><<<a.spans, kExpThreads, 0, stream>>>(a);
-    return cudaGetLastError();
+    if ((err = launch_chained(k_quad_starts<K>, a.spans, kExpThreads, 0, stream, a)) != cudaSuccess) return err;
+    err = launch_chained(k_quad_tiles<K>, div_up(e.gx * e.gy, kTileThreads), kTileThreads, 0, stream, a);
+    if (err != cudaSuccess) return err;
+    return launch_chained(k_quad_expand<K>, a.spans, kExpThreads, 0, stream, a);
 }
 
 cudaError_t launch_quad_expand(const ExpandArgs& e, cudaStream_t stream)

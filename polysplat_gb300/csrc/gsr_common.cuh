@@ -163,6 +163,30 @@ __device__ __forceinline__ float rsqrt_approx(float x)
     return y;
 }
 
+// A frame is a chain of short kernels.  One launched by launch_chained may be
+// resident before the kernel in front of it has ended: it begins with
+// chain_wait, which returns when that kernel is complete and its writes are
+// visible, and chain_ready lets the next one in once every CTA has started.
+// Every kernel of the chain waits in every CTA, so completion carries over.
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_ready() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... P, typename... A>
+inline cudaError_t launch_chained(void (*kern)(P...), dim3 grid, int block, size_t smem, cudaStream_t stream, A&&... args)
+{
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = grid;
+    c.blockDim = dim3(block);
+    c.dynamicSmemBytes = smem;
+    c.stream = stream;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kern, static_cast<P>(args)...);
+}
+
 __host__ __device__ __forceinline__ int div_up(int a, int b) { return (a + b - 1) / b; }
 
 // Number of bits needed to hold n (n < 2^bits); the key-width trim rule.

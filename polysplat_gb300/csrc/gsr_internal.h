@@ -300,6 +300,7 @@ struct RenderArgs {
     uint8_t* out;
     WorkspaceHeader* ws;
     int quad = 0;  // keys and ranges per 2x2 group of 16x16 tiles (PreprocessParams::quad)
+    int queue_clear = 0;  // the header's tile queue is clear (clear_header)
 };
 cudaError_t launch_render(const RenderArgs& a, cudaStream_t stream);
 

@@ -329,6 +329,7 @@ __device__ __forceinline__ void block_copy(Stage<HITS>& st, const EmitOut& out, 
 template <bool HALF, bool COUNT, bool VIEWS, bool QUAD = false>
 __global__ __launch_bounds__(kThreads, VIEWS ? 6 : 5) void k_preprocess(const __grid_constant__ PreprocessParams a0)
 {
+    chain_ready();
     // VIEWS: the views' blocks follow one another along the grid (parameter
     // blocks in device memory); a block past the last view has no work
     int vi = 0, lblock = (int)blockIdx.x;
@@ -879,6 +880,8 @@ __global__ __launch_bounds__(kThreads, 4) void k_emit_massive(const __grid_const
     __shared__ int s_rows[kWarps];                 // rows listed
     const unsigned lane = threadIdx.x & 31u;
     const int warp = threadIdx.x >> 5;
+    chain_wait();
+    chain_ready();
     Stage<QUAD && !VIEWS> st{s_keys[MODE == kMassiveEmit64 ? warp : 0], s_vals[MODE == kMassiveEmit64 ? warp : 0], 0};
     const EmitOut out{a.keys, a.vals, a.cap, a.counter, a.pair_count};
     uint32_t* head = a.mq.head + (MODE == kMassiveEmitDf ? 2 : 0);
@@ -1341,6 +1344,13 @@ static int emit_grid(Kern kern)
     return device_sm_count() * b;
 }
 
+template <int MODE, bool VIEWS, bool QUAD>
+static cudaError_t launch_massive(const PreprocessParams& a, const DfEmit& df, cudaStream_t stream)
+{
+    auto kern = k_emit_massive<MODE, VIEWS, QUAD>;
+    return launch_chained(kern, emit_grid(kern), kThreads, 0, stream, a, df);
+}
+
 static cudaError_t preprocess_common(const PreprocessParams& p, bool half_sh, bool count, cudaStream_t stream)
 {
     if (p.P <= 0) return cudaSuccess;
@@ -1368,15 +1378,10 @@ static cudaError_t preprocess_common(const PreprocessParams& p, bool half_sh, bo
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess || p.mq.capacity <= 0) return e;
     const DfEmit none{nullptr, nullptr, nullptr, nullptr, 0};
-    if (count && p.quad)
-        k_emit_massive<kMassiveCount, false, true>
-            <<<emit_grid(k_emit_massive<kMassiveCount, false, true>), kThreads, 0, stream>>>(p, none);
-    else if (count) k_emit_massive<kMassiveCount, false><<<emit_grid(k_emit_massive<kMassiveCount, false>), kThreads, 0, stream>>>(p, none);
-    else if (p.quad)
-        k_emit_massive<kMassiveEmit64, false, true>
-            <<<emit_grid(k_emit_massive<kMassiveEmit64, false, true>), kThreads, 0, stream>>>(p, none);
-    else k_emit_massive<kMassiveEmit64, false><<<emit_grid(k_emit_massive<kMassiveEmit64, false>), kThreads, 0, stream>>>(p, none);
-    return cudaGetLastError();
+    if (count && p.quad) return launch_massive<kMassiveCount, false, true>(p, none, stream);
+    if (count) return launch_massive<kMassiveCount, false, false>(p, none, stream);
+    if (p.quad) return launch_massive<kMassiveEmit64, false, true>(p, none, stream);
+    return launch_massive<kMassiveEmit64, false, false>(p, none, stream);
 }
 
 cudaError_t launch_preprocess_views(const PreprocessParams& base, int n_views, int blocks, bool half_sh,
@@ -1394,15 +1399,12 @@ cudaError_t launch_preprocess_views(const PreprocessParams& base, int n_views, i
         if (half_sh) k_preprocess<true, false, true, true><<<grid, kThreads, 0, stream>>>(base);
         else k_preprocess<false, false, true, true><<<grid, kThreads, 0, stream>>>(base);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
-        k_emit_massive<kMassiveEmit64, true, true>
-            <<<emit_grid(k_emit_massive<kMassiveEmit64, true, true>), kThreads, 0, stream>>>(base, none);
-        return cudaGetLastError();
+        return launch_massive<kMassiveEmit64, true, true>(base, none, stream);
     }
     if (half_sh) k_preprocess<true, false, true><<<grid, kThreads, 0, stream>>>(base);
     else k_preprocess<false, false, true><<<grid, kThreads, 0, stream>>>(base);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    k_emit_massive<kMassiveEmit64, true><<<emit_grid(k_emit_massive<kMassiveEmit64, true>), kThreads, 0, stream>>>(base, none);
-    return cudaGetLastError();
+    return launch_massive<kMassiveEmit64, true, false>(base, none, stream);
 }
 
 cudaError_t launch_preprocess(const PreprocessParams& p, bool half_sh, cudaStream_t stream)
@@ -1422,13 +1424,8 @@ cudaError_t launch_df_emit_massive(const PreprocessParams& p, const uint32_t* of
     // takes the queue again through the second pair of heads (cleared with
     // the rest of the preprocess region before the counting pass)
     const DfEmit df{offsets, rank, tiles, vals, cap};
-    if (p.quad)
-        k_emit_massive<kMassiveEmitDf, false, true>
-            <<<emit_grid(k_emit_massive<kMassiveEmitDf, false, true>), kThreads, 0, stream>>>(p, df);
-    else
-        k_emit_massive<kMassiveEmitDf, false>
-            <<<emit_grid(k_emit_massive<kMassiveEmitDf, false>), kThreads, 0, stream>>>(p, df);
-    return cudaGetLastError();
+    if (p.quad) return launch_massive<kMassiveEmitDf, false, true>(p, df, stream);
+    return launch_massive<kMassiveEmitDf, false, false>(p, df, stream);
 }
 
 // The reference's ES pass B (preprocess.cu:993-1248): every Gaussian in

@@ -28,6 +28,8 @@ template <typename K>
 __global__ void k_ranges_exact(int num, const int32_t* __restrict__ d_num, long long cap, int tiles,
                                const K* __restrict__ keys, int2* __restrict__ ranges)
 {
+    chain_wait();
+    chain_ready();
     const int n = clamp_count(num, d_num, cap);
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i <= n; i += stride) {
@@ -102,7 +104,7 @@ cudaError_t launch_tile_ranges(int num, const int32_t* d_num, long long cap, int
         k_zero_ranges<<<min(sms * 4, div_up(tiles, 256)), 256, 0, stream>>>(tiles, r);
         k_ranges_scan<<<grid, 256, 0, stream>>>(num, d_num, cap, tiles, keys, r);
     } else {
-        k_ranges_exact<uint64_t><<<grid, 256, 0, stream>>>(num, d_num, cap, tiles, keys, r);
+        return launch_chained(k_ranges_exact<uint64_t>, grid, 256, 0, stream, num, d_num, cap, tiles, keys, r);
     }
     return cudaGetLastError();
 }
@@ -113,8 +115,7 @@ cudaError_t launch_tile_ranges32(const int32_t* d_num, long long cap, int tiles,
     if (tiles <= 0) return cudaSuccess;
     const int sms = device_sm_count();
     const int grid = (int)max(1LL, min((long long)sms * 8, (cap + 256) / 256));
-    k_ranges_exact<uint32_t><<<grid, 256, 0, stream>>>(0, d_num, cap, tiles, tile_ids, ranges);
-    return cudaGetLastError();
+    return launch_chained(k_ranges_exact<uint32_t>, grid, 256, 0, stream, 0, d_num, cap, tiles, tile_ids, ranges);
 }
 
 cudaError_t launch_gather(int num, const int32_t* d_num, const uint32_t* values, const float2* sxy,

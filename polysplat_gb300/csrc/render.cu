@@ -749,6 +749,8 @@ __global__ __launch_bounds__(kRenderWarps * 32, BX * BY == 256 ? 4 : 1) void k_b
     const unsigned lane = threadIdx.x & 31u;
     const int warp = threadIdx.x >> 5;
     BlendRing<SPLIT == 1>& R = rings[warp];
+    chain_wait();
+    chain_ready();
     const long long nl = p.d_num ? (long long)*p.d_num : (long long)p.n_host;
     const int n = (int)max(0LL, min(nl, p.cap));
     const int cb = (int)(lane & 7u) * TX;
@@ -820,9 +822,8 @@ cudaError_t launch_blend(const RenderParams& p, cudaStream_t stream)
 {
     if constexpr (BX == 16 && BY == 16) {
         if (split_tiles(p.items)) {
-            k_blend<BX, BY, CADENCE, RANGE_MODE, BATCH, QUAD, kRenderWarps>
-                <<<p.items, kRenderWarps * 32, 0, stream>>>(p);
-            return cudaGetLastError();
+            return launch_chained(k_blend<BX, BY, CADENCE, RANGE_MODE, BATCH, QUAD, kRenderWarps>, p.items,
+                                  kRenderWarps * 32, 0, stream, p);
         }
     }
     auto kern = k_blend<BX, BY, CADENCE, RANGE_MODE, BATCH, QUAD, 1>;
@@ -838,8 +839,7 @@ cudaError_t launch_blend(const RenderParams& p, cudaStream_t stream)
         per_sm_cache[dev].store(per_sm, std::memory_order_relaxed);
     }
     const int grid = max(1, min(device_sm_count() * per_sm, div_up(p.items, kRenderWarps)));
-    kern<<<grid, kRenderWarps * 32, 0, stream>>>(p);
-    return cudaGetLastError();
+    return launch_chained(kern, grid, kRenderWarps * 32, 0, stream, p);
 }
 
 template <int BX, int BY, int CADENCE, int SHADER, bool DT, int RANGE_MODE, bool TMA, bool BATCH = false,
@@ -1325,7 +1325,7 @@ cudaError_t launch_render_views(const RenderArgs& a, const RenderView* views_dev
 static cudaError_t launch_prepared(const RenderArgs& a, RenderParams& p, cudaStream_t stream)
 {
     if (p.tiles <= 0) return cudaSuccess;
-    cudaError_t e = cudaMemsetAsync(p.queue, 0, sizeof(uint32_t), stream);
+    cudaError_t e = a.queue_clear ? cudaSuccess : cudaMemsetAsync(p.queue, 0, sizeof(uint32_t), stream);
     if (e != cudaSuccess) return e;
     // TMA bulk copies need 16-byte aligned feature arrays; GSR_RENDER_TMA=0
     // stages batches with per-thread cp.async copies instead.

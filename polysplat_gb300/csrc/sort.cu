@@ -154,6 +154,8 @@ __global__ __launch_bounds__(256) void k_upsweep(SortJob<K> a)
     __shared__ uint32_t s_hist[256];
     s_hist[threadIdx.x] = 0u;
     __syncthreads();
+    chain_wait();
+    chain_ready();
     const int n = sort_count(a);
     const int tiles = (n + kSortTile - 1) / kSortTile;
     const KeyMap km = key_map(a.order, a.s.hdr);
@@ -523,6 +525,8 @@ __global__ __launch_bounds__(kSortThreads, kSortCtas) void k_pass(SortJob<K> a, 
     static_assert(kSortThreads == 256, "thread d owns digit d");
     const unsigned lane = threadIdx.x & 31u;
     const int warp = threadIdx.x >> 5, tid = threadIdx.x;
+    chain_wait();
+    chain_ready();
     const KeyMap km = key_map(a.order, a.s.hdr);
     const int passes = passes_of(km);
     if (pass >= passes) return;  // nothing left to order in this digit
@@ -613,8 +617,7 @@ cudaError_t run_sort(const SortJob<K>& job, int max_passes, cudaStream_t stream)
         return e;
     const int sms = device_sm_count();
     int up_grid = (int)std::min<long long>((long long)sms * 4, std::max<long long>(1, (a.cap + 2047) / 2048));
-    k_upsweep<K><<<up_grid, 256, 0, stream>>>(a);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if ((e = launch_chained(k_upsweep<K>, up_grid, 256, 0, stream, a)) != cudaSuccess) return e;
     profile_mark(stream);
 
     const int mode = sort_rank_mode();
@@ -637,8 +640,7 @@ cudaError_t run_sort(const SortJob<K>& job, int max_passes, cudaStream_t stream)
     }
     const int grid = (int)std::min<long long>((long long)sms * per_sm, std::max<long long>(1, a.s.tiles_cap));
     for (int p = 0; p < max_passes; p++) {
-        kern<<<grid, kSortThreads, smem, stream>>>(a, p);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        if ((e = launch_chained(kern, grid, kSortThreads, smem, stream, a, p)) != cudaSuccess) return e;
         profile_mark(stream);
     }
     return cudaSuccess;
