@@ -118,7 +118,7 @@ gsr_status gsr_scene_prepare(int P, const float* log_scales, const float* quats,
  * key_capacity are dropped but counted.  shs_half != 0 selects FP16 SH.
  * `workspace` (at least gsr_render_workspace_size() bytes, or NULL) holds
  * the queue of Gaussians with large tile rectangles, which a second kernel
- * spreads over whole CTAs; without it those are emitted by their own warp
+ * spreads over the chip; without it those are emitted by their own warp
  * (same keys, slower).  Replaces preprocess / preprocess_half_sh
  * (csrc/ops.h:42-48, 104-111; csrc/cuda_rasterizer/preprocess.cu:1252-1330;
  * csrc/pybind.cpp:122-181). */
@@ -181,8 +181,9 @@ gsr_status gsr_gather(int num, const int32_t* d_num, const uint32_t* values, con
                       float* dst_conic, gsr_stream_t stream);
 
 /* ---- render ------------------------------------------------------------- */
-/* Persistent tile-queue blend: one warp per tile, 32-Gaussian batches staged
- * into shared memory by TMA bulk copies under mbarrier double-buffering,
+/* Persistent tile-queue blend: one warp per tile (four where the frame has few
+ * tiles), 32-Gaussian batches staged into shared memory by double-buffered
+ * asynchronous copies (GSR_RENDER_TMA=1: TMA bulk copies on an mbarrier),
  * whole-tile early exit by warp vote, truncating uint8 encode.
  * `ranges` is required for the *_RANGES/DT variants, `keys_sorted` for the
  * FUSED/DEFAULT variants.  P is the length of the feature arrays (bounds).
@@ -354,8 +355,9 @@ const int32_t* gsr_batcher_counter(const gsr_batcher* b);
 const uint32_t* gsr_batcher_status(const gsr_batcher* b);
 /* Dispatch thresholds of the tile-key emission, in tiles of a Gaussian's
  * rectangle: from massive_area (default 32) on, a rectangle is queued for the
- * large-Gaussian kernel; from huge_area (default 2048) on, a whole CTA sweeps
- * it.  They change which scheme tests the tiles, never the keys. */
+ * large-Gaussian kernel; from huge_area (default 2048) on, a CTA takes it with
+ * seven others.  A massive_area above 128 acts as 128.  They change which
+ * scheme tests the tiles, never the keys. */
 gsr_status gsr_batcher_set_thresholds(gsr_batcher* b, int massive_area, int huge_area);
 
 /* ---- differentiable render -------------------------------------------------- */
