@@ -190,10 +190,10 @@ class Rasterizer:
         digit passes move fewer pairs, three more kernels write all M.
 
         The line, frame times sorting per tile and expanding (us):
-          M 9.5 M = 3.2 P   754 / 612      M 5.2 M = 1.7 P   556 / 512
-          M 2.0 M = 2.0 P   353 / 332      M 1.5 M = 3.1 P   314 / 310
-          M 3.7 M = 1.2 P   489 / 477      M 26 M = 1.3 P   4267 / 4328
-          M 2.6 M = 1.3 P   719 / 750      M 0.3 M = 3.3 P   259 / 278
+          M 9.5 M = 3.2 P   680 / 539      M 5.2 M = 1.7 P   484 / 439
+          M 2.0 M = 2.0 P   281 / 262      M 1.5 M = 3.1 P   242 / 236
+          M 3.7 M = 1.2 P   417 / 401      M 26 M = 1.3 P   4228 / 4283
+          M 2.6 M = 1.3 P   653 / 683      M 0.3 M = 3.3 P   182 / 197
         Below 1.5 P most Gaussians hit one tile of a quad.  Depth-first, 6 M
         Gaussians at 1440p (M over 5 P): 1803 / 1603."""
         M = self._es_last_M
