@@ -166,10 +166,10 @@ __global__ __launch_bounds__(kExpThreads, kExpCtas) void k_quad_starts(const __g
         uint32_t quad[kExpSteps], val[kExpSteps];
 #pragma unroll
         for (int k = 0; k < kExpSteps; k++) {
-            quad[k] = 32 * k < left ? __ldg(hp + 32 * kWords * k) : 0u;
-            val[k] = 32 * k < left ? __ldg(vp + 32 * k) : 0u;
+            quad[k] = 32 * k < left ? hp[32 * kWords * k] : 0u;
+            val[k] = 32 * k < left ? vp[32 * k] : 0u;
         }
-        uint32_t before = lane == 0 && i0 > 0 && left > 0 ? __ldg(hp - kWords) : 0u;
+        uint32_t before = lane == 0 && i0 > 0 && left > 0 ? *(hp - kWords) : 0u;
         const uint4 at = warp_base(val, run, s_sum[flip], lane, warp);
         // counts are needed only in the steps in which a quad ends or begins
         uint32_t bytes = 0;  // this lane's tiles of the steps before
@@ -225,7 +225,7 @@ __device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t (&s_warp)[kT
 
 __device__ __forceinline__ uint32_t comp(const uint4* p, uint32_t i, int b)
 {
-    return __ldg(reinterpret_cast<const uint32_t*>(p + i) + b);
+    return reinterpret_cast<const uint32_t*>(p + i)[b];
 }
 
 // A thread per tile.  Every CTA sums the list lengths of the tiles before its
@@ -318,8 +318,8 @@ __global__ __launch_bounds__(kExpThreads, kExpCtas) void k_quad_expand(const __g
         uint32_t val[kExpSteps];
 #pragma unroll
         for (int k = 0; k < kExpSteps; k++) {
-            key[k] = 32 * k < left ? __ldg(kp + 32 * k) : K(0);
-            val[k] = 32 * k < left ? __ldg(vp + 32 * k) : 0u;
+            key[k] = 32 * k < left ? kp[32 * k] : K(0);
+            val[k] = 32 * k < left ? vp[32 * k] : 0u;
         }
         uint4 at = warp_base(val, run, s_sum[flip], lane, warp);
 #pragma unroll

@@ -25,8 +25,7 @@ __device__ __forceinline__ uint32_t tile_of(uint64_t k) { return (uint32_t)(k >>
 __device__ __forceinline__ uint32_t tile_of(uint32_t k) { return k; }
 
 template <typename K>
-__global__ void k_ranges_exact(int num, const int32_t* __restrict__ d_num, long long cap, int tiles,
-                               const K* __restrict__ keys, int2* __restrict__ ranges)
+__global__ void k_ranges_exact(int num, const int32_t* d_num, long long cap, int tiles, const K* keys, int2* ranges)
 {
     chain_wait();
     chain_ready();
@@ -34,8 +33,8 @@ __global__ void k_ranges_exact(int num, const int32_t* __restrict__ d_num, long 
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i <= n; i += stride) {
         int a = -1, b = tiles;  // tile(i-1), tile(i); virtual -1 and T at the ends
-        if (i > 0) a = (int)min((uint32_t)tiles, tile_of(__ldg(keys + i - 1)));
-        if (i < n) b = (int)min((uint32_t)tiles, tile_of(__ldg(keys + i)));
+        if (i > 0) a = (int)min((uint32_t)tiles, tile_of(keys[i - 1]));
+        if (i < n) b = (int)min((uint32_t)tiles, tile_of(keys[i]));
         if (a == b) continue;
         // start = i for tiles a+1 .. b (capped at T-1); end = i for tiles max(a,0) .. b-1
         const int lo = max(a, 0), hi = min(b, tiles - 1);

@@ -83,14 +83,14 @@ __device__ __forceinline__ uchar3 encode_px(const float (&c)[3], float t, bool a
 // First index in keys[lo, hi) whose tile id is > t (UPPER) or >= t (!UPPER);
 // warp-cooperative 32-way search, log32(n) rounds.
 template <bool UPPER>
-__device__ __forceinline__ int warp_bound(const uint64_t* __restrict__ keys, int lo, int hi, uint32_t t, unsigned lane)
+__device__ __forceinline__ int warp_bound(const uint64_t* keys, int lo, int hi, uint32_t t, unsigned lane)
 {
     while (hi - lo > 32) {
         const int step = (hi - lo + 31) >> 5;
         const int p = lo + ((int)lane + 1) * step - 1;
         bool pred = false;
         if (p < hi) {
-            const uint32_t kt = (uint32_t)(__ldg(keys + p) >> 32);
+            const uint32_t kt = (uint32_t)(keys[p] >> 32);
             pred = UPPER ? (kt <= t) : (kt < t);
         }
         const int c = __popc(__ballot_sync(GSR_FULL_MASK, pred));
@@ -102,7 +102,7 @@ __device__ __forceinline__ int warp_bound(const uint64_t* __restrict__ keys, int
     const int p = lo + (int)lane;
     bool pred = false;
     if (p < hi) {
-        const uint32_t kt = (uint32_t)(__ldg(keys + p) >> 32);
+        const uint32_t kt = (uint32_t)(keys[p] >> 32);
         pred = UPPER ? (kt <= t) : (kt < t);
     }
     return lo + __popc(__ballot_sync(GSR_FULL_MASK, pred));
@@ -555,7 +555,7 @@ struct Feed {
         end = REV ? start : stop;
         head = tail = 0;
         sub_bit = bit;
-        ahead = (int)lane < left() ? __ldg(f.vals + mine(lane)) : 0u;
+        ahead = (int)lane < left() ? f.vals[mine(lane)] : 0u;
     }
 
     __device__ __forceinline__ void fetch(BlendRing<DUP>& R, const Features& f, unsigned lane, bool& bad)
@@ -572,7 +572,7 @@ struct Feed {
                 }
                 tail += __popc(m);
                 pos += REV ? -kBatch : kBatch;
-                ahead = (int)lane < left() ? __ldg(f.vals + mine(lane)) : 0u;
+                ahead = (int)lane < left() ? f.vals[mine(lane)] : 0u;
             }
             __syncwarp();
             n = min(kBatch, tail - head);
@@ -588,14 +588,14 @@ struct Feed {
             v = ahead;
             where = mine(lane);
             pos += REV ? -n : n;
-            ahead = (int)lane < left() ? __ldg(f.vals + mine(lane)) : 0u;
+            ahead = (int)lane < left() ? f.vals[mine(lane)] : 0u;
         }
         if ((int)lane < n) {
             if (v < f.P) {
                 gid = v;
-                xy = __ldg(f.xy + v);
-                con = __ldg(f.con + v);
-                rgbd = __ldg(f.rgbd + v);
+                xy = f.xy[v];
+                con = f.con[v];
+                rgbd = f.rgbd[v];
             } else {  // index outside the feature arrays: a transparent stand-in
                 bad = true;
                 gid = 0xFFFFFFFFu;
@@ -770,7 +770,7 @@ __global__ __launch_bounds__(kRenderWarps * 32, BX * BY == 256 ? 4 : 1) void k_b
             int lo = 0, hi = p.n_views - 1;
             while (lo < hi) {
                 const int mid = (lo + hi + 1) >> 1;
-                if (__ldg(&p.views[mid].tile_base) <= tile) lo = mid;
+                if (p.views[mid].tile_base <= tile) lo = mid;
                 else hi = mid - 1;
             }
             const RenderView& v = p.views[lo];
@@ -786,7 +786,7 @@ __global__ __launch_bounds__(kRenderWarps * 32, BX * BY == 256 ? 4 : 1) void k_b
         if (!QUAD || (ox < W && oy < H)) {  // a quad's tile beyond the image edge has no pixels
             int start, end;
             if (RANGE_MODE == 0) {
-                const int2 r = __ldg(p.ranges + tile);
+                const int2 r = p.ranges[tile];
                 // ranges come from the caller: keep them inside [0, n]
                 start = min(max(r.x, 0), n);
                 end = min(max(r.y, start), n);
@@ -1001,7 +1001,7 @@ struct TrainTile {
         oy = ty * 16;
         cb = (int)(lane & 7u) * 2;
         rb = (SPLIT > 1 ? warp * (16 / SPLIT) : 0) + (int)(lane >> 3) * (4 / SPLIT);
-        const int2 rg = __ldg(a.ranges + train_list<QUAD>(view, tile, tx, ty, gx, gy, qbit));
+        const int2 rg = a.ranges[train_list<QUAD>(view, tile, tx, ty, gx, gy, qbit)];
         start = min(max(rg.x, 0), n);
         stop = min(max(rg.y, start), n);
         return true;

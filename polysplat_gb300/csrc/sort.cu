@@ -130,7 +130,7 @@ __device__ __forceinline__ void load8(const K* src, long long b, int cnt, K (&k)
         const uint4* v = reinterpret_cast<const uint4*>(src + b);
 #pragma unroll
         for (int q = 0; q < 8 / kPer; q++) {
-            const uint4 w = __ldg(v + q);
+            const uint4 w = v[q];
             const K* e = reinterpret_cast<const K*>(&w);
 #pragma unroll
             for (int j = 0; j < kPer; j++) k[q * kPer + j] = e[j];
@@ -138,7 +138,7 @@ __device__ __forceinline__ void load8(const K* src, long long b, int cnt, K (&k)
         return;
     }
 #pragma unroll
-    for (int j = 0; j < 8; j++) k[j] = j < cnt ? __ldg(src + b + j) : K(0);
+    for (int j = 0; j < 8; j++) k[j] = j < cnt ? src[b + j] : K(0);
 }
 
 // ---------------------------------------------------------------------------
