@@ -261,12 +261,16 @@ __device__ __forceinline__ int small_div(int a, int b) { return (int)__fdividef(
 
 constexpr int kPoolArea = 128;
 
-// Block-wide final flush of every warp's staged keys with one atomic per CTA:
-// the reservation, whose round trip the preprocess hides behind its colours,
-// and the copy.
+// Block-wide final flush of every warp's staged keys with one atomic per CTA.
+//
+// Pairs of equal (tile, depth) keys stay in the order of these reservations to
+// the blend, so the preprocess flushes last, behind its colours.  Reserving in
+// front of them gains nothing (1.00x over all of the timed cases) and orders
+// CTAs by their tile tests alone: of 250 small training steps it moved pixels
+// in 222 tiles where the order of flushing last moves 169, a second run 86.
 template <bool HITS>
-__device__ __forceinline__ void block_reserve(const Stage<HITS>& st, const EmitOut& out, int* s_fill,
-                                              long long* s_base, unsigned lane, int warp)
+__device__ __forceinline__ void block_flush(Stage<HITS>& st, const EmitOut& out, int* s_fill, long long* s_base,
+                                            unsigned lane, int warp)
 {
     if (HITS && out.pairs) {
         const uint32_t h = __reduce_add_sync(GSR_FULL_MASK, st.hits);
@@ -290,21 +294,6 @@ __device__ __forceinline__ void block_reserve(const Stage<HITS>& st, const EmitO
         base = __shfl_sync(GSR_FULL_MASK, base, 0);
         if (lane < kWarps) s_base[lane] = base + incl - f;
     }
-}
-
-// The counting pass's hit tiles of a CTA's warps.
-__device__ __forceinline__ void add_hits(unsigned long long* pairs, const int* s_hits)
-{
-    uint32_t h = 0;
-#pragma unroll
-    for (int w = 0; w < kWarps; w++) h += (uint32_t)s_hits[w];
-    if (h) atomicAdd(pairs, (unsigned long long)h << 32);
-}
-
-template <bool HITS>
-__device__ __forceinline__ void block_copy(Stage<HITS>& st, const EmitOut& out, const long long* s_base, unsigned lane,
-                                           int warp)
-{
     __syncthreads();
     const long long wb = s_base[warp];
     for (int i = lane; i < st.fill; i += 32) {
@@ -315,6 +304,15 @@ __device__ __forceinline__ void block_copy(Stage<HITS>& st, const EmitOut& out, 
         }
     }
     st.fill = 0;
+}
+
+// The counting pass's hit tiles of a CTA's warps.
+__device__ __forceinline__ void add_hits(unsigned long long* pairs, const int* s_hits)
+{
+    uint32_t h = 0;
+#pragma unroll
+    for (int w = 0; w < kWarps; w++) h += (uint32_t)s_hits[w];
+    if (h) atomicAdd(pairs, (unsigned long long)h << 32);
 }
 
 // COUNT = false: emit (tile | depth, index) keys (the reference's single-pass
@@ -614,8 +612,6 @@ __global__ __launch_bounds__(kThreads, VIEWS ? 6 : 5) void k_preprocess(const __
         }
     }
     __syncwarp();
-    if (!COUNT) block_reserve(st, out, s_fill, s_base, lane, warp);
-
     // (3) render features for every Gaussian that emitted at least one key.
     const bool emitted = (s_hit[warp] >> lane) & 1u;
     if (a.mq.depth_hi) {
@@ -674,8 +670,7 @@ __global__ __launch_bounds__(kThreads, VIEWS ? 6 : 5) void k_preprocess(const __
             if (threadIdx.x == 0) add_hits(a.pair_count, s_fill);
         }
     } else {
-        // (4) the staged keys, to the place reserved before the features
-        block_copy(st, out, s_base, lane, warp);
+        block_flush(st, out, s_fill, s_base, lane, warp);
     }
 }
 
@@ -1108,8 +1103,7 @@ __global__ __launch_bounds__(kThreads, 4) void k_emit_massive(const __grid_const
         }
     }
     if (MODE == kMassiveEmit64) {
-        block_reserve(st, out, s_fill, s_base, lane, warp);
-        block_copy(st, out, s_base, lane, warp);
+        block_flush(st, out, s_fill, s_base, lane, warp);
     } else if (MODE == kMassiveCount && QUAD && a.pair_count) {
         const uint32_t h = __reduce_add_sync(GSR_FULL_MASK, st.hits);
         if (lane == 0) s_fill[warp] = (int)h;
