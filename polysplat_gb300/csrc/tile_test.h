@@ -13,11 +13,16 @@
 #define GSR_TT_MUL(a, b) __fmul_rn(a, b)
 #define GSR_TT_SUB(a, b) __fsub_rn(a, b)
 #define GSR_TT_FMA(a, b, c) __fmaf_rn(a, b, c)
+// fast math: within 2 ulp of the quotient, which a host check can stand in for
+#define GSR_TT_DIV(a, b) ((a) / (b))
 #else
 #define GSR_TT_FN inline
 #define GSR_TT_MUL(a, b) ((a) * (b))
 #define GSR_TT_SUB(a, b) ((a) - (b))
 #define GSR_TT_FMA(a, b, c) std::fma(a, b, c)
+#ifndef GSR_TT_DIV
+#define GSR_TT_DIV(a, b) ((a) / (b))
+#endif
 struct int2 { int x, y; };
 struct float2 { float x, y; };
 struct float3 { float x, y, z; };
@@ -183,15 +188,15 @@ GSR_TT_FN Band make_band(float3 q, float power, float2 c, int x_lo, int x_hi, in
     const float u = 5.9604645e-8f;
     const float bb = B * B;
     const float det = GSR_TT_FMA(A, C, -bb) + GSR_TT_FMA(-B, B, bb);
-    const float kappa = 2.0f * (A * C) / det;
+    const float kappa = GSR_TT_DIV(2.0f * (A * C), det);
     const float wb = w * (1.0f + 64.0f * u * (1.0f + kappa));  // inflated for the test's rounding
     b.B = B;
-    b.inv_a = 1.0f / A;
-    b.inv_c = 1.0f / C;
+    b.inv_a = GSR_TT_DIV(1.0f, A);
+    b.inv_c = GSR_TT_DIV(1.0f, C);
     b.det = det;
-    b.dymax = sqrtf(wb * A / det);
-    b.dxmax = sqrtf(wb * C / det);
-    b.dyr = -B * sqrtf(wb / (C * det));  // dy where the ellipse reaches its largest x
+    b.dymax = sqrtf(GSR_TT_DIV(wb * A, det));
+    b.dxmax = sqrtf(GSR_TT_DIV(wb * C, det));
+    b.dyr = -B * sqrtf(GSR_TT_DIV(wb, C * det));  // dy where the ellipse reaches its largest x
     b.cx = c.x;
     b.cy = c.y;
     b.m = 0.5f + 1e-5f * fmaxf(b.dxmax, b.dymax);
@@ -240,8 +245,10 @@ GSR_TT_FN bool band_columns(const Band& e, int ty, int by, int bx, int x_lo, int
         hi = e.cx + xr + e.m;
     } else {
         const bool row_of_centre = e.cy >= l && e.cy <= r;
-        lo = row_of_centre ? e.cx : 3e38f;
-        hi = row_of_centre ? e.cx : -3e38f;
+        // a pixel on either side, as everywhere: the quotient by a width that is
+        // no power of two may fall below a whole number
+        lo = row_of_centre ? e.cx - 1.0f : 3e38f;
+        hi = row_of_centre ? e.cx + 1.0f : -3e38f;
         if (e.kind == kBandNeedle) {
             const float u = 5.9604645e-8f;
             // horizontal edge: the test's dy, its middle and half-width
@@ -262,7 +269,7 @@ GSR_TT_FN bool band_columns(const Band& e, int ty, int by, int bx, int x_lo, int
                     hi = 3e38f;
                 }
             } else {
-                const float d0 = v0 / slope, d1 = v1 / slope;  // dx range, in either order
+                const float d0 = GSR_TT_DIV(v0, slope), d1 = GSR_TT_DIV(v1, slope);  // dx range, in either order
                 const float dmin = fminf(d0, d1), dmax = fmaxf(d0, d1);
                 const float mv = 1.0f + 1e-5f * (fabsf(e.cx) + fmaxf(fabsf(dmin), fabsf(dmax)));
                 // the edge ex = cx - dx is the tile's first or last column
@@ -275,8 +282,8 @@ GSR_TT_FN bool band_columns(const Band& e, int ty, int by, int bx, int x_lo, int
         lo = -3e38f;
         hi = 3e38f;
     }
-    c_lo = (int)fmaxf((float)x_lo, fminf(floorf(lo / (float)bx), (float)x_hi));
-    c_hi = (int)fminf((float)(x_hi - 1), fmaxf(floorf(hi / (float)bx), -1.0f));
+    c_lo = (int)fmaxf((float)x_lo, fminf(floorf(GSR_TT_DIV(lo, (float)bx)), (float)x_hi));
+    c_hi = (int)fminf((float)(x_hi - 1), fmaxf(floorf(GSR_TT_DIV(hi, (float)bx)), -1.0f));
     return c_lo <= c_hi;
 }
 
