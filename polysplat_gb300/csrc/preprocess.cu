@@ -495,7 +495,7 @@ __global__ __launch_bounds__(kThreads, VIEWS ? 6 : 5) void k_preprocess(const __
         const uint32_t db = __shfl_sync(GSR_FULL_MASK, depth_bits, i);
         const float pw = __shfl_sync(GSR_FULL_MASK, power, i);
         const uint32_t gid = (uint32_t)(a.gid_base + warp_first + i);
-        bool hit = a.mq.capacity > 0;  // features are written for Gaussians that belong to a queue
+        bool hit = !a.df.ref_layout;  // the ES layout has features where a tile is hit; elsewhere as for a queued one
         if (QUAD) {
             const int qx_lo = quad_lo(x_lo), qx_hi = quad_hi(x_hi), qy_lo = quad_lo(y_lo), qy_hi = quad_hi(y_hi);
             for (int y0 = qy_lo; y0 < qy_hi; y0 += 4) {
