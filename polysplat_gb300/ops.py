@@ -72,7 +72,8 @@ def _host_floats(t, n: int, what: str):
     host tensor is read in place (1 us instead of 10): the caller holds it
     through the call."""
     if isinstance(t, torch.Tensor):
-        if t.dtype == torch.float32 and t.device.type == "cpu" and t.numel() >= n and t.is_contiguous():
+        if (t.dtype == torch.float32 and t.device.type == "cpu" and t.numel() >= n and t.is_contiguous()
+                and not t.is_neg()):  # a lazily negated view's memory holds the other sign
             return ctypes.c_void_p(t.data_ptr())
         vals = t.detach().to("cpu", torch.float32).reshape(-1).tolist()
     else:
