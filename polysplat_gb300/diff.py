@@ -45,10 +45,11 @@ def _slab(dev, nbytes):
 
 
 def _parts(slab, nbytes):
-    """The addresses of a slab's parts, each on 256 bytes."""
+    """The addresses of a slab's parts, each on 256 bytes; null for an empty one,
+    as an empty tensor's is (a scene without Gaussians is refused by it)."""
     at, out = slab.data_ptr(), []
     for n in nbytes:
-        out.append(ctypes.c_void_p(at))
+        out.append(ctypes.c_void_p(at if n else 0))
         at += (int(n) + 255) & ~255
     return out
 
