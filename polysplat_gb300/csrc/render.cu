@@ -739,8 +739,18 @@ static bool split_tiles(long long tiles) { return tiles <= 16LL * device_sm_coun
 
 // Persistent render, a tile per warp; with SPLIT = 4 a tile per CTA and no
 // queue.
+//
+// 32x16 tiles need three CTAs per SM (162 to 168 registers): left to itself the
+// compiler takes 196, two CTAs fit, and where tiles are many the kernel falls
+// behind k_render (four CTAs); at four CTAs it spills.  Render alone, k_render /
+// two / three / four CTAs: 20 M Gaussians at 7680x4320 3964 / 4290 / 3799 / 4109
+// us, 3 M at 3840x2160 127 / 137 / 111 / 123, 500 k at 1271x717 144 / 162 / 128 /
+// 146, 100 k at 800x600 174 / 146 / 127 / 183.  32x32 tiles (255 registers, two
+// CTAs, some bytes spilled) beat k_render throughout: 8325 / 6333, 156 / 124 (at
+// 3840x2160), 709 / 365 (at 800x600).
 template <int BX, int BY, int CADENCE, int RANGE_MODE, bool BATCH, bool QUAD, int SPLIT>
-__global__ __launch_bounds__(kRenderWarps * 32, BX * BY == 256 ? 4 : 1) void k_blend(const RenderParams p)
+__global__ __launch_bounds__(kRenderWarps * 32, BX * BY == 256 ? 4 : BX * BY == 512 ? 3 : 1)
+void k_blend(const RenderParams p)
 {
     static_assert(!QUAD || (BX == 16 && BY == 16), "quad renders: 16x16 tiles");
     static_assert(SPLIT == 1 || (SPLIT == kRenderWarps && BY == 16), "a tile per warp, or per CTA");
@@ -866,8 +876,9 @@ cudaError_t launch_variant(const RenderParams& p, cudaStream_t stream)
 }
 
 // TMA staging, the distance-thresholded and the split renders, the general
-// shader (SH 1) and 24-wide tiles take the scalar kernel; the rest take the
-// paired one.
+// shader (SH 1) and 24-wide tiles (three columns a lane) take the scalar kernel;
+// the rest take the paired one, the faster of the two at every size measured (see
+// k_blend).
 template <int BX, int BY, int CADENCE, int SHADER, int RANGE_MODE>
 cudaError_t launch_whole(bool tma, const RenderParams& p, cudaStream_t stream)
 {
