@@ -17,6 +17,12 @@
 // large Gaussians.  26 M pairs of 21 M at 8K: 50 + 22 + 148 us, which the passes do
 // not give back.  The expansion reads 12 bytes a key and writes 12 a pair at 4.5
 // TB/s; spans of 4, 5 or 6 CTAs per SM and 4 keys a thread measure alike.
+//
+// Step 2 needs the lists before a CTA's own tiles.  Adding them up in every CTA
+// saves a launch but is quadratic in the tiles, so above kDirectTiles a kernel of
+// its own (k_quad_sums) leaves the CTAs' totals.  Frames with the totals / adding
+// up: 8160 tiles 522 / 516 us, 14400 360 / 355, 32400 555 / 557, 129600 919 / 929,
+// 291600 4856 / 4890, 518400 1916 / 1982 and 2758 / 2822.
 #include <algorithm>
 #include <cstdint>
 
@@ -35,6 +41,7 @@ constexpr int kExpChunk = kExpWarps * kExpShare;
 constexpr int kExpCtas = 4;  // spans per SM
 constexpr int kTileThreads = 1024;
 constexpr int kMaxSpans = 1024;
+constexpr int kDirectTiles = 32768;
 
 // Arrays of one expansion, in the unsorted key buffer (the sort has read it).
 struct QuadSeg {
@@ -45,6 +52,7 @@ struct QuadSeg {
     uint32_t* base;   // [quads][4] place of the tile's first key - P there
     uint32_t* tile;   // [quads] the quad's first tile
     uint4* totals;    // [spans]
+    uint32_t* sums;   // [CTAs of k_quad_tiles] their tiles' list lengths, or nullptr
 };
 
 // K: 64-bit keys (quad << 32 | depth bits), or the depth-first pipeline's
@@ -228,53 +236,89 @@ __device__ __forceinline__ uint32_t comp(const uint4* p, uint32_t i, int b)
     return reinterpret_cast<const uint32_t*>(p + i)[b];
 }
 
-// A thread per tile.  Every CTA sums the list lengths of the tiles before its
-// own, quads at a time, instead of waiting for the CTAs that hold them (8 CTAs
-// and 7 us at 1080p, 127 and 22 us at 8K: latency).
+// P before each span, one of the four counts at a time, and the sum of the four.
+struct SpanPrefix {
+    uint32_t pre[4][kMaxSpans];
+    uint32_t all[kMaxSpans];
+};
+
+template <typename K>
+__device__ __forceinline__ void span_prefix(const ExpandJob<K>& a, SpanPrefix& s, uint32_t (&s_warp)[kTileThreads / 32])
+{
+    const int tid = threadIdx.x;
+    const uint4 t = tid < a.spans ? a.seg.totals[tid] : make_uint4(0, 0, 0, 0);
+    uint32_t sum;
+    s.pre[0][tid] = block_scan(t.x, s_warp, sum);
+    s.pre[1][tid] = block_scan(t.y, s_warp, sum);
+    s.pre[2][tid] = block_scan(t.z, s_warp, sum);
+    s.pre[3][tid] = block_scan(t.w, s_warp, sum);
+    s.all[tid] = s.pre[0][tid] + s.pre[1][tid] + s.pre[2][tid] + s.pre[3][tid];
+    __syncthreads();
+}
+
+// Length of tile t's list; q, b: its quad and number there, p: P at its start.
+template <typename K>
+__device__ __forceinline__ uint32_t list_length(const ExpandJob<K>& a, const SpanPrefix& s, int t, uint32_t& q, int& b,
+                                                uint32_t& p)
+{
+    const int y = t / a.gx, x = t - y * a.gx;
+    q = (uint32_t)((y >> 1) * quad_cols(a.gx) + (x >> 1));
+    b = (x & 1) | (y & 1) << 1;
+    p = s.pre[b][a.seg.first_span[q]] + comp(a.seg.first, q, b);
+    return s.pre[b][a.seg.last_span[q]] + comp(a.seg.last, q, b) - p;
+}
+
+// Sum of the list lengths of each CTA's tiles, for grids in which adding up all
+// earlier quads in every CTA of k_quad_tiles costs more than this launch.
+template <typename K>
+__global__ __launch_bounds__(kTileThreads) void k_quad_sums(const __grid_constant__ ExpandJob<K> a)
+{
+    __shared__ SpanPrefix s;
+    __shared__ uint32_t s_warp[kTileThreads / 32];
+    chain_wait();
+    chain_ready();
+    span_prefix(a, s, s_warp);
+    const int t = blockIdx.x * kTileThreads + (int)threadIdx.x;
+    uint32_t q, p, sum;
+    int b;
+    block_scan(t < a.gx * a.gy ? list_length(a, s, t, q, b, p) : 0u, s_warp, sum);
+    if (threadIdx.x == 0) a.seg.sums[blockIdx.x] = sum;
+}
+
+// A thread per tile.  In grids of up to kDirectTiles every CTA sums the list
+// lengths of the tiles before its own, quads at a time, instead of waiting for
+// the CTAs that hold them (8 CTAs and 7 us at 1080p: latency); in larger ones it
+// sums k_quad_sums' totals.
 template <typename K>
 __global__ __launch_bounds__(kTileThreads) void k_quad_tiles(const __grid_constant__ ExpandJob<K> a)
 {
-    __shared__ uint32_t s_pre[4][kMaxSpans];  // P before each span
-    __shared__ uint32_t s_all[kMaxSpans];     // sum of the four
+    __shared__ SpanPrefix s;
     __shared__ uint32_t s_warp[kTileThreads / 32];
     const int tid = threadIdx.x;
     chain_wait();
     chain_ready();
-    {
-        const uint4 t = tid < a.spans ? a.seg.totals[tid] : make_uint4(0, 0, 0, 0);
-        uint32_t sum;
-        s_pre[0][tid] = block_scan(t.x, s_warp, sum);
-        s_pre[1][tid] = block_scan(t.y, s_warp, sum);
-        s_pre[2][tid] = block_scan(t.z, s_warp, sum);
-        s_pre[3][tid] = block_scan(t.w, s_warp, sum);
-        s_all[tid] = s_pre[0][tid] + s_pre[1][tid] + s_pre[2][tid] + s_pre[3][tid];
-    }
-    __syncthreads();
+    span_prefix(a, s, s_warp);
     const int tiles = a.gx * a.gy, qgx = quad_cols(a.gx);
-    // length of a tile's list; q, b: its quad and number there, p: P at its start
-    auto length = [&](int t, uint32_t& q, int& b, uint32_t& p) {
-        const int y = t / a.gx, x = t - y * a.gx;
-        q = (uint32_t)((y >> 1) * qgx + (x >> 1));
-        b = (x & 1) | (y & 1) << 1;
-        p = s_pre[b][a.seg.first_span[q]] + comp(a.seg.first, q, b);
-        return s_pre[b][a.seg.last_span[q]] + comp(a.seg.last, q, b) - p;
-    };
     const int t0 = blockIdx.x * kTileThreads;
     uint32_t q = 0, p = 0, before = 0, sum;
     int b = 0;
-    // whole rows of quads before the CTA's first tile, then the tiles between
-    const int rows = t0 / a.gx >> 1;
+    if (a.seg.sums) {
+        for (int k = tid; k < (int)blockIdx.x; k += kTileThreads) before += a.seg.sums[k];
+    } else {
+        // whole rows of quads before the CTA's first tile, then the tiles between
+        const int rows = t0 / a.gx >> 1;
 #pragma unroll 4
-    for (int k = tid; k < rows * qgx; k += kTileThreads) {
-        const uint4 f = a.seg.first[k], l = a.seg.last[k];
-        const int fs = a.seg.first_span[k], ls = a.seg.last_span[k];
-        before += (l.x - f.x) + (l.y - f.y) + (l.z - f.z) + (l.w - f.w) + s_all[ls] - s_all[fs];
+        for (int k = tid; k < rows * qgx; k += kTileThreads) {
+            const uint4 f = a.seg.first[k], l = a.seg.last[k];
+            const int fs = a.seg.first_span[k], ls = a.seg.last_span[k];
+            before += (l.x - f.x) + (l.y - f.y) + (l.z - f.z) + (l.w - f.w) + s.all[ls] - s.all[fs];
+        }
+        for (int t = 2 * rows * a.gx + tid; t < t0; t += kTileThreads) before += list_length(a, s, t, q, b, p);
     }
-    for (int t = 2 * rows * a.gx + tid; t < t0; t += kTileThreads) before += length(t, q, b, p);
     block_scan(before, s_warp, sum);
     const uint32_t earlier = sum;
     const int t = t0 + tid;
-    const uint32_t n = t < tiles ? length(t, q, b, p) : 0u;
+    const uint32_t n = t < tiles ? list_length(a, s, t, q, b, p) : 0u;
     const uint32_t start = earlier + block_scan(n, s_warp, sum);
     if (t < tiles) {
         const uint32_t cap = (uint32_t)a.cap;
@@ -352,7 +396,8 @@ int expand_spans() { return std::min(kMaxSpans, device_sm_count() * kExpCtas); }
 size_t expand_scratch_bytes(int gx, int gy)
 {
     const size_t quads = (size_t)quad_cols(gx) * quad_cols(gy);
-    return 256 + 3 * align256(quads * 16) + 3 * align256(quads * 4) + (size_t)kMaxSpans * 16;
+    const size_t ctas = ((size_t)gx * gy + kTileThreads - 1) / kTileThreads;
+    return 256 + 3 * align256(quads * 16) + 3 * align256(quads * 4) + (size_t)kMaxSpans * 16 + align256(ctas * 4);
 }
 
 template <typename K>
@@ -377,6 +422,8 @@ static cudaError_t expand(const ExpandArgs& e, cudaStream_t stream)
     a.seg.base = reinterpret_cast<uint32_t*>(p + cleared);
     a.seg.tile = reinterpret_cast<uint32_t*>(p + cleared + q16);
     a.seg.totals = reinterpret_cast<uint4*>(p + cleared + q16 + q4);
+    const int tiles = e.gx * e.gy, ctas = div_up(tiles, kTileThreads);
+    a.seg.sums = tiles > kDirectTiles ? reinterpret_cast<uint32_t*>(a.seg.totals + kMaxSpans) : nullptr;
     a.out_keys = static_cast<K*>(e.out_keys);
     a.out_vals = e.out_vals;
     a.ranges = e.ranges;
@@ -384,7 +431,8 @@ static cudaError_t expand(const ExpandArgs& e, cudaStream_t stream)
     cudaError_t err = cudaMemsetAsync(p, 0, cleared, stream);
     if (err != cudaSuccess) return err;
     if ((err = launch_chained(k_quad_starts<K>, a.spans, kExpThreads, 0, stream, a)) != cudaSuccess) return err;
-    err = launch_chained(k_quad_tiles<K>, div_up(e.gx * e.gy, kTileThreads), kTileThreads, 0, stream, a);
+    if (a.seg.sums && (err = launch_chained(k_quad_sums<K>, ctas, kTileThreads, 0, stream, a)) != cudaSuccess) return err;
+    err = launch_chained(k_quad_tiles<K>, ctas, kTileThreads, 0, stream, a);
     if (err != cudaSuccess) return err;
     return launch_chained(k_quad_expand<K>, a.spans, kExpThreads, 0, stream, a);
 }
