@@ -126,6 +126,7 @@ class Rasterizer:
         self._out_color = None
         self._auto_render_choice = None
         self._es_last_M = None
+        self._frame_tiles = 0
 
     # -- buffers ------------------------------------------------------------------
     def _get_out_color(self, height, width, device):
@@ -146,6 +147,7 @@ class Rasterizer:
         t = ((camera.width + bx - 1) // bx) * ((camera.height + by - 1) // by)
         if t > self.MAX_NUM_TILES:
             raise ValueError("image needs %d tiles, MAX_NUM_TILES is %d" % (t, self.MAX_NUM_TILES))
+        self._frame_tiles = t
 
     # -- autotune of the tile shape (example.py:199-231) ----------------------------
     def _autotune_render_config(self, scene, camera, bg_color, measure_runs=2):
@@ -195,9 +197,15 @@ class Rasterizer:
           M 3.7 M = 1.2 P   417 / 401      M 26 M = 1.3 P   4228 / 4283
           M 2.6 M = 1.3 P   653 / 683      M 0.3 M = 3.3 P   182 / 197
         Below 1.5 P most Gaussians hit one tile of a quad.  Depth-first, 6 M
-        Gaussians at 1440p (M over 5 P): 1803 / 1603."""
+        Gaussians at 1440p (M over 5 P): 1803 / 1603.  What is above 1.5 P also
+        pays for the kernels that go over the frame's T tiles (us):
+          M 8.9 M = 1.5 P + 2.6 T   1898 / 1916    M 35 M = 1.5 P + 10 T   5602 / 5563
+          M 7.6 M = 1.5 P + 0.4 T   1537 / 1562    M 7.4 M = 74 P = 56 T   1079 / 919
+
+        The unsorted key and value buffers hold the quad keys of such a frame,
+        overwritten in part, and not its per-tile pairs."""
         M = self._es_last_M
-        return M is not None and M >= 1_500_000 and M >= 1.5 * scene.num_vertex
+        return M is not None and M >= 1_500_000 and M >= 1.5 * scene.num_vertex + 5 * self._frame_tiles
 
     @staticmethod
     def _df_variant(render_variant):
