@@ -208,8 +208,8 @@ GSR_HD void forward(const T m[3], const T ls[3], const T q[4], T logit, const T*
 }
 
 // The colour's share of the adjoint on its own: adds its part of dL/dmean to
-// g_m and gives the colour gradient behind the clamp, with which the SH
-// gradient is B[k] g[ch] (B: sh_basis of the view direction).
+// g_m and gives the colour gradient behind the clamp, of which add_sh_gradient
+// makes the SH gradient B[k] g[ch] (B: sh_basis of the view direction).
 template <typename T>
 GSR_HD void color_adjoint(const T m[3], const T campos[3], const T* sh, const T g_rgb[3], T g_m[3], T g[3])
 {
@@ -233,8 +233,21 @@ GSR_HD void color_adjoint(const T m[3], const T campos[3], const T* sh, const T 
     for (int i = 0; i < 3; i++) g_m[i] += (g_dir[i] - dir[i] * dd) / vlen;
 }
 
+// Adds the SH gradient of one view to g_sh, from color_adjoint's g.
+template <typename T>
+GSR_HD void add_sh_gradient(const T m[3], const T campos[3], const T g[3], T* g_sh)
+{
+    T d[3] = {m[0] - campos[0], m[1] - campos[1], m[2] - campos[2]};
+    const T len = t_sqrt(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
+    T B[16], dB[16][3];
+    sh_basis(d[0] / len, d[1] / len, d[2] / len, B, dB);
+    for (int k = 0; k < 16; k++)
+        for (int ch = 0; ch < 3; ch++) g_sh[3 * k + ch] += B[k] * g[ch];
+}
+
 // Gradients of the raw parameters from those of xy, con and rgb.  COLOR =
-// false leaves the colour's part (and g_sh) out.
+// false leaves the colour's part (and g_sh) to the caller's color_adjoint and
+// add_sh_gradient, of which the other form is made.
 template <typename T, bool COLOR = true>
 GSR_HD void backward(const T m[3], const T* sh, const Cam<T>& cam, const Tape<T>& tp, const T g_xy[2], const T g_con[4],
                      const T g_rgb[3], T g_m[3], T g_ls[3], T g_q[4], T& g_logit, T* g_sh)
@@ -331,17 +344,10 @@ GSR_HD void backward(const T m[3], const T* sh, const Cam<T>& cam, const Tape<T>
     for (int col = 0; col < 3; col++)
         for (int r4 = 0; r4 < 4; r4++) g_m[col] += P[4 * col + r4] * g_ph[r4];
     if (!COLOR) return;
-    // colour
-    T g_dir[3] = {0, 0, 0};
-    for (int ch = 0; ch < 3; ch++) {
-        const T g = tp.clamp_rgb[ch] ? (T)0 : g_rgb[ch];
-        for (int k = 0; k < 16; k++) {
-            g_sh[3 * k + ch] = tp.B[k] * g;
-            for (int d = 0; d < 3; d++) g_dir[d] += tp.dB[k][d] * sh[3 * k + ch] * g;
-        }
-    }
-    const T dd = g_dir[0] * tp.dir[0] + g_dir[1] * tp.dir[1] + g_dir[2] * tp.dir[2];
-    for (int i = 0; i < 3; i++) g_m[i] += (g_dir[i] - tp.dir[i] * dd) / tp.vlen;
+    T g[3];
+    color_adjoint(m, cam.campos, sh, g_rgb, g_m, g);
+    for (int k = 0; k < 48; k++) g_sh[k] = 0;
+    add_sh_gradient(m, cam.campos, g, g_sh);
 }
 
 }  // namespace gsr_adj

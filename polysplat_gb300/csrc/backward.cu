@@ -189,13 +189,7 @@ __global__ __launch_bounds__(kAdjThreads) void k_preprocess_backward(const __gri
             for (int k = first; k < first + n; k++) {
                 const float* o = s_out[k - begin];
                 for (int c = 0; c < 11; c++) sum[c] += o[c];
-                const float* campos = a.cam[s_pair[k] >> 8].campos;
-                float d[3] = {m[0] - campos[0], m[1] - campos[1], m[2] - campos[2]};
-                const float len = sqrtf(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
-                float B[16], dB[16][3];
-                gsr_adj::sh_basis(d[0] / len, d[1] / len, d[2] / len, B, dB);
-                for (int c = 0; c < 16; c++)
-                    for (int ch = 0; ch < 3; ch++) sh[3 * c + ch] += B[c] * o[11 + ch];
+                gsr_adj::add_sh_gradient(m, a.cam[s_pair[k] >> 8].campos, o + 11, sh);
             }
             auto put = [&](float* dst, size_t off, float v) { dst[off] = a.accumulate ? dst[off] + v : v; };
             for (int k = 0; k < 3; k++) {
