@@ -545,6 +545,7 @@ struct Feed {
     uint32_t gid;     // feature row, ~0 outside the feature arrays
     float2 xy;
     float4 con, rgbd;
+    float3 mid;       // REV: taken off the stored colours (centre())
 
     __device__ __forceinline__ int left() const { return REV ? pos - end : end - pos; }
     __device__ __forceinline__ int mine(unsigned lane) const { return REV ? pos - 1 - (int)lane : pos + (int)lane; }
@@ -606,19 +607,32 @@ struct Feed {
         }
     }
 
+    // The backward's colours relative to that of the first batch's first
+    // Gaussian, the farthest one blended (0 if that is not finite).
+    __device__ __forceinline__ void centre()
+    {
+        auto of_lane0 = [](float v) {
+            v = __shfl_sync(GSR_FULL_MASK, v, 0);
+            return fabsf(v) < 1e30f ? v : 0.0f;
+        };
+        mid = n > 0 ? make_float3(of_lane0(rgbd.x), of_lane0(rgbd.y), of_lane0(rgbd.z)) : make_float3(0.f, 0.f, 0.f);
+    }
+
     __device__ __forceinline__ void store(BlendRing<DUP>& R, unsigned lane) const
     {
         if ((int)lane < n) {
+            const float r = REV ? rgbd.x - mid.x : rgbd.x, g = REV ? rgbd.y - mid.y : rgbd.y,
+                        b = REV ? rgbd.z - mid.z : rgbd.z;
             if (DUP) {
                 R.xyab[2 * lane] = make_float4(xy.x, xy.x, xy.y, xy.y);
                 R.xyab[2 * lane + 1] = make_float4(con.x, con.x, con.y, con.y);
                 R.cwrg[2 * lane] = make_float4(con.z, con.z, con.w, con.w);
-                R.cwrg[2 * lane + 1] = make_float4(rgbd.x, rgbd.x, rgbd.y, rgbd.y);
+                R.cwrg[2 * lane + 1] = make_float4(r, r, g, g);
             } else {
                 R.xyab[lane] = make_float4(xy.x, xy.y, con.x, con.y);
-                R.cwrg[lane] = make_float4(con.z, con.w, rgbd.x, rgbd.y);
+                R.cwrg[lane] = make_float4(con.z, con.w, r, g);
             }
-            R.bl[lane] = make_float2(rgbd.z, rgbd.z);
+            R.bl[lane] = make_float2(b, b);
             if (REV) R.gid[lane] = gid;  // the backward's gradient row
         }
     }
@@ -1088,7 +1102,10 @@ __device__ __forceinline__ float warp_sum2_spread(float a, float b, unsigned lan
 
 // A lane's TY x 2 pixels of the reverse walk, columns in pairs.  R . G is
 // carried as one number per pixel: the walk only needs the colour behind a
-// Gaussian through its product with the pixel's gradient.
+// Gaussian through its product with the pixel's gradient.  All colours, R's
+// too, are relative to the list's farthest one (Feed::centre): (c - R) . G is
+// then a difference of products as small as the colours' differences, and does
+// not cancel where neighbours along a ray have nearly one colour.
 template <int TY>
 struct BackPixels {
     f32x2 T[TY], RG[TY], G[TY][3];
@@ -1180,11 +1197,16 @@ __global__ __launch_bounds__(kTrainWarps * 32, 4) void k_render_backward(const T
     TrainTile<QUAD, SPLIT> t;
     if (!t.open(a, lane, warp)) return;
     const int count = min(max(__ldg(a.n_tile + t.tile), 0), t.stop - t.start);
+    const Features f{a.xy, a.con, a.rgbd, a.vals, (uint32_t)a.P};
+    bool bad = false;
+    Feed<QUAD, true, SPLIT == 1> feed;
+    feed.open(f, t.start, t.start + count, t.qbit, lane);
+    // the pixels' loads travel with the list's
     BackPixels<TY> px;
     px.ncol = pair(-(float)(t.ox + t.cb), -(float)(t.ox + t.cb + 1));
 #pragma unroll
     for (int i = 0; i < TY; i++) {
-        float T[2], rg[2], g[2][3];
+        float T[2], g[2][3];
         const int y = t.oy + t.rb + i;
         px.nrow[i] = pair(-(float)y, -(float)y);
 #pragma unroll
@@ -1195,23 +1217,28 @@ __global__ __launch_bounds__(kTrainWarps * 32, 4) void k_render_backward(const T
             T[j] = in ? __ldg(a.T_final + o) : 1.0f;
 #pragma unroll
             for (int ch = 0; ch < 3; ch++) g[j][ch] = in ? __ldg(a.grad_image + 3 * o + ch) : 0.0f;
-            rg[j] = T[j] < 0.0001f ? 0.0f : a.bg[0] * g[j][0] + a.bg[1] * g[j][1] + a.bg[2] * g[j][2];
         }
         px.T[i] = pair(T[0], T[1]);
-        px.RG[i] = pair(rg[0], rg[1]);
 #pragma unroll
         for (int ch = 0; ch < 3; ch++) px.G[i][ch] = pair(g[0][ch], g[1][ch]);
+    }
+    feed.fetch(R, f, lane, bad);
+    feed.centre();
+    // R . G behind everything: the background's, or 0 where the forward dropped it
+    const float3 m = feed.mid, bg = make_float3(a.bg[0] - m.x, a.bg[1] - m.y, a.bg[2] - m.z);
+#pragma unroll
+    for (int i = 0; i < TY; i++) {
+        auto behind = [&](float T, float g0, float g1, float g2) {
+            return T < 0.0001f ? -(m.x * g0 + m.y * g1 + m.z * g2) : bg.x * g0 + bg.y * g1 + bg.z * g2;
+        };
+        px.RG[i] = pair(behind(lo_of(px.T[i]), lo_of(px.G[i][0]), lo_of(px.G[i][1]), lo_of(px.G[i][2])),
+                        behind(hi_of(px.T[i]), hi_of(px.G[i][0]), hi_of(px.G[i][1]), hi_of(px.G[i][2])));
     }
     // where a lane's total goes: lane l has value (l >> 1) & 7 of the first
     // (l < 16) or second Gaussian; lanes 0 and 16 add the blue sums as well
     const int slot = (int)(lane >> 1) & 7;
     const bool first = lane < 16u;
     const float unit = slot < 6 ? 0.69314718055994531f : 1.0f;  // the ln 2 of d power
-    const Features f{a.xy, a.con, a.rgbd, a.vals, (uint32_t)a.P};
-    bool bad = false;
-    Feed<QUAD, true, SPLIT == 1> feed;
-    feed.open(f, t.start, t.start + count, t.qbit, lane);
-    feed.fetch(R, f, lane, bad);
     while (feed.n > 0) {
         const int n = feed.n;
         __syncwarp();
