@@ -182,9 +182,11 @@ gsr_status gsr_gather(int num, const int32_t* d_num, const uint32_t* values, con
 
 /* ---- render ------------------------------------------------------------- */
 /* Persistent tile-queue blend: one warp per tile (four where the frame has few
- * tiles), 32-Gaussian batches staged into shared memory by double-buffered
- * asynchronous copies (GSR_RENDER_TMA=1: TMA bulk copies on an mbarrier),
- * whole-tile early exit by warp vote, truncating uint8 encode.
+ * tiles), 32-Gaussian batches loaded into registers one batch ahead and blended
+ * from shared memory (the distance-thresholded, split and 24-wide renders and
+ * the general shader: double-buffered asynchronous copies; GSR_RENDER_TMA=1: TMA
+ * bulk copies on an mbarrier), whole-tile early exit by warp vote, truncating
+ * uint8 encode.
  * `ranges` is required for the *_RANGES/DT variants, `keys_sorted` for the
  * FUSED/DEFAULT variants.  P is the length of the feature arrays (bounds).
  * block_x/block_y select the tile shape (16x16, 24x16, 32x16, 32x32).

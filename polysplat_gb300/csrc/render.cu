@@ -927,7 +927,8 @@ cudaError_t dispatch_shape(int variant, bool tma, const RenderParams& p, cudaStr
     }
 }
 
-// Quad renders (16x16 tiles, keys per 2x2 group of tiles; cp.async staging).
+// Quad renders (16x16 tiles, keys per 2x2 group of tiles): the paired kernel, but
+// for the distance-thresholded render.
 template <bool BATCH>
 cudaError_t dispatch_quad(int variant, const RenderParams& p, cudaStream_t stream)
 {
@@ -946,7 +947,7 @@ cudaError_t dispatch_quad(int variant, const RenderParams& p, cudaStream_t strea
     }
 }
 
-// Batched renders: ranges always precomputed, cp.async staging, 16x16,
+// Batched renders: ranges always precomputed, never staged by TMA, 16x16,
 // 32x16 and 32x32 tiles.
 template <int BX, int BY>
 cudaError_t dispatch_batch(int variant, const RenderParams& p, cudaStream_t stream)
@@ -970,9 +971,10 @@ static cudaError_t launch_prepared(const RenderArgs& a, RenderParams& p, cudaStr
 
 static bool use_render_tma()
 {
-    // per-thread cp.async staging measured faster than per-lane 16-byte bulk
-    // copies (28 vs 48 us at 1080p, 2.5 vs 3.6 ms at 8K): bulk copies only on
-    // request (read once, thread-safe initialisation)
+    // in the scalar kernel per-thread cp.async staging measured faster than
+    // per-lane 16-byte bulk copies (28 vs 48 us at 1080p, 2.5 vs 3.6 ms at 8K), and
+    // k_blend stages neither way: bulk copies only on request (read once,
+    // thread-safe initialisation)
     static const bool tma = [] {
         const char* e = getenv("GSR_RENDER_TMA");
         return e && strcmp(e, "1") == 0;
@@ -1365,8 +1367,7 @@ static cudaError_t launch_prepared(const RenderArgs& a, RenderParams& p, cudaStr
     if (p.tiles <= 0) return cudaSuccess;
     cudaError_t e = a.queue_clear ? cudaSuccess : cudaMemsetAsync(p.queue, 0, sizeof(uint32_t), stream);
     if (e != cudaSuccess) return e;
-    // TMA bulk copies need 16-byte aligned feature arrays; GSR_RENDER_TMA=0
-    // stages batches with per-thread cp.async copies instead.
+    // TMA bulk copies, where asked for, need 16-byte aligned feature arrays
     const bool tma = use_render_tma() && ((reinterpret_cast<uintptr_t>(a.xy) | reinterpret_cast<uintptr_t>(a.rgbd) |
                                            reinterpret_cast<uintptr_t>(a.con)) & 15u) == 0;
     if (p.views) {
