@@ -170,8 +170,8 @@ __device__ __forceinline__ float rsqrt_approx(float x)
 // Every kernel of the chain waits in every CTA, so completion carries over.
 // Such a kernel reads what the kernels in front of it write by plain loads:
 // __ldg and const __restrict__ are for memory that nobody writes while the
-// kernel is resident, and the wait does not order the read-only path.  Plain
-// loads cost nothing here (frame times within the noise, both ways).
+// kernel is resident, and the wait does not order the read-only path.  Frames
+// take the time they took with __ldg, within the noise.
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_ready() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -264,10 +264,11 @@ constexpr int kPoolArea = 128;
 // Block-wide final flush of every warp's staged keys with one atomic per CTA.
 //
 // Pairs of equal (tile, depth) keys stay in the order of these reservations to
-// the blend, so the preprocess flushes last, behind its colours.  Reserving in
-// front of them gains nothing (1.00x over all of the timed cases) and orders
-// CTAs by their tile tests alone: of 250 small training steps it moved pixels
-// in 222 tiles where the order of flushing last moves 169, a second run 86.
+// the blend, so the preprocess flushes last, behind its colours, and CTAs come in
+// the order in which they end.  Reserving in front of the colours orders them by
+// their tile tests alone, which gives tiles with such pairs other pixels, and
+// gains nothing: 1.00x over all of the timed cases, and 568 against 541 us for
+// the preprocess of eight training views, whose registers it holds longer.
 template <bool HITS>
 __device__ __forceinline__ void block_flush(Stage<HITS>& st, const EmitOut& out, int* s_fill, long long* s_base,
                                             unsigned lane, int warp)
